@@ -247,8 +247,12 @@ int mfista_plan_profile(mfista_plan plan, int kernel, int reps, double *ms_per_l
                         double *bytes_per_launch);
 int mfista_plan_kernel_launches(mfista_plan plan);   /* kernels per solve, last run */
 /* Launch shapes of the plan's operator kernels, as int[4]:
- *   [0] interpolation points per warp (shared geometry; 1..32),
- *   [1] spreading CTAs per tile cluster (shared geometry; 1..16),
+ *   [0] interpolation points per warp (shared geometry; 1..32): how the
+ *       tap-by-tap interpolation and the residual from kept models divide
+ *       the points,
+ *   [1] spreading CTAs per tile cluster (shared geometry; 1..16) of the
+ *       tap-by-tap spreading; kept, but without effect on the spreading by
+ *       matrix products,
  *   [2] image rows per CTA of the row FFT passes,
  *   [3] grid columns per CTA of the column FFT passes;
  * 0 = not used by this plan's operator (get) or keep the current value

@@ -1,0 +1,503 @@
+// NUFFT interpolation and spreading (NUFFT2d2 / NUFFT2d1 of
+// c/mfista_nufft_lib.c:123-243) on the FP64 matrix instruction
+// (mma.sync m8n8k4.f64), for one problem, batches that share their points and
+// batches with points of their own.
+//
+// Both are separable tap sums: a point's 576 weights are wx[24] x wy[24].
+// Tap by tap they are bound by gathers and by address arithmetic (an FP64
+// batch ran at 3 % of the FP64 rate).  Here a warp takes 16 points of one tile
+// (interpolation) or 8 x 8 cells (spreading) through matrix products whose
+// operands come from shared memory and registers, on "virtual" coordinates:
+// grid rows and columns before the reference's row wrap and Hermitian fold,
+// so that every point sees plain consecutive taps.
+//
+// FP64 products and sums throughout, also for the FP32 operators (whose grids
+// and residuals stay FP32): m8n8k4.f64 runs at the rate of the FP64 pipe
+// (37 TFLOP/s measured, with one shared-memory operand per 512 operations).
+//
+// Measured on B200, FP64, microseconds per launch, tap by tap -> here:
+//   grid, points, problems          interpolation    spreading
+//   64 x 64, 2016, 1                 40.1 -> 12.4     37.0 -> 10.6
+//   128 x 128, 8100, 1               39.7 -> 12.4     60.6 -> 14.5
+//   128 x 128, 8100, 64               489 -> 187       581 -> 199
+//   256 x 256, 19998, 64             1130 -> 486      1710 -> 508
+//   128 x 128, 102070 over 16 frames  163 -> 54        605 -> 123
+// The products alone would take 87 us and 80 us at 128 x 128 with 64 problems.
+#pragma once
+#include "nufft_ops.cuh"
+
+namespace mf {
+
+__device__ __forceinline__ void dmma_884(double (&d)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+               : "+d"(d[0]), "+d"(d[1])
+               : "d"(a), "d"(b));
+}
+
+// asynchronous copy of one complex grid cell; valid = false writes zero
+template <typename T>
+__device__ __forceinline__ void cp_async_cell(cplx<T>* dst, const cplx<T>* src, bool valid) {
+  const unsigned int d = (unsigned int)__cvta_generic_to_shared(dst);
+  const unsigned int n = valid ? (unsigned int)sizeof(cplx<T>) : 0u;
+  if (sizeof(cplx<T>) == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+}
+
+// ---------------------------------------------------------------------------
+// Interpolation.  The points are binned by their first tap (mx - 11, my - 11)
+// into kImTile x kImTile tiles of virtual positions; all taps of a tile's
+// points lie in a 39 x 39 window (kImWin = 40 staged).  A CTA takes up to 128
+// points of a tile and a chunk of PB problems.  Per problem it stages the
+// window (cp.async, the next problem's window in flight behind the products;
+// dropped taps are staged as zeros), and each warp forms, for 16 points and 4
+// window rows at a time,
+//   T[p][row, re/im] = sum_c wy_p[c] G[row, c][re/im]      (K = columns)
+//   y_p += sum_row wx_p[row] T[p][row]
+// as m8n8k4 products: A = wy (in registers for all problems), B = the window's
+// cells (one 8-byte shared load per lane serves both blocks of 8 points), so
+// nothing of a matrix tile is idle for a single problem.  Only the rows and
+// columns that the 16 points reach are walked.  A CTA with few points splits
+// its window rows over the warps.
+// Signs: the reference negates the imaginary part of direct taps (NU_SIGN) and
+// keeps that of mirrored ones; a tap is direct or mirrored by its column alone,
+// so the imaginary parts of mirrored columns are flipped at the fragment and
+// the sum is negated once.
+// A problem's sums depend neither on the chunk nor on its slot in it.
+// ---------------------------------------------------------------------------
+constexpr int kImTile = 16;
+constexpr int kImWin = kImTile + kTaps;  // 40: 39 used, a multiple of 4
+constexpr int kImPts = 128;              // points per CTA: 8 warps x 16
+constexpr int kImSteps = kImWin / 4;     // column steps of 4
+
+struct ImTileItem {
+  int row0, col0;    // window origin, virtual
+  int start, count;  // perm[start, start + count)
+  int prob;          // its problem (points of its own), or -1 (shared points)
+  int slot;          // chi^2 slot
+  int ntiles;        // CTAs (= chi^2 slots written) of this problem
+  int pad;
+};
+
+// row stride of the staged window: the four rows of a B fragment hit all banks
+template <typename T> struct ImWindow {
+  static constexpr int kLd = sizeof(T) == 8 ? 44 : 52;
+  static constexpr size_t kBytes = sizeof(cplx<T>) * (size_t)kImWin * kLd;
+};
+constexpr size_t im_red_bytes(int pb) { return sizeof(double2) * (size_t)pb * 8 * 16; }
+template <typename T, int PB> constexpr size_t im_smem() {
+  return (PB > 1 ? 2 : 1) * ImWindow<T>::kBytes + im_red_bytes(PB);
+}
+
+template <typename T, int PB>
+__global__ void __launch_bounds__(256, 2)
+    k_nufft_interp_mma(NufftGeom<T> geo, const double* __restrict__ wxd, const double* __restrict__ wyd,
+                       const ImTileItem* __restrict__ tiles, const int2* __restrict__ perm,
+                       const cplx<T>* __restrict__ gall, long gstride, int nx, int ny, double inv_mm,
+                       const ProbState* __restrict__ st, int gate, Partials part, int qchi, int nslots,
+                       cplx<T>* __restrict__ y2, int B, const double2* __restrict__ ax_base,
+                       double2* __restrict__ ax_out) {
+  constexpr int LD = ImWindow<T>::kLd;
+  constexpr int kCells = (kImWin * kImWin + 255) / 256;
+  extern __shared__ __align__(16) unsigned char im_smem_raw[];
+  cplx<T>* win = reinterpret_cast<cplx<T>*>(im_smem_raw);
+  double2* s_red = reinterpret_cast<double2*>(im_smem_raw + (PB > 1 ? 2 : 1) * ImWindow<T>::kBytes);
+  __shared__ int s_list[PB];
+  __shared__ int s_cnt[8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  const ImTileItem tl = tiles[blockIdx.x];
+  int nact;
+  if (PB > 1) {
+    nact = active_chunk<PB>(st, gate, B, blockIdx.y, s_list, s_cnt, geo.act_lists);
+  } else {
+    const int b = tl.prob >= 0 ? tl.prob : (int)blockIdx.y;
+    nact = gate_ok(st[b], gate) ? 1 : 0;
+    if (threadIdx.x == 0) s_list[0] = b;
+    __syncthreads();
+  }
+  if (nact == 0) return;
+  // stored cell of each window cell this thread copies (-1: dropped tap)
+  int cell[kCells];
+#pragma unroll
+  for (int i = 0; i < kCells; ++i) {
+    const int v = threadIdx.x + 256 * i;
+    cell[i] = -1;
+    if (v < kImWin * kImWin) {
+      const int vr = tl.row0 + v / kImWin, vc = tl.col0 + v % kImWin;
+      int col = half_col(vc, ny), row = -1;
+      if (col >= 0) {
+        row = wrap_row(vr, nx);
+      } else {
+        col = half_col(-vc, ny);
+        row = wrap_row(-vr, nx);
+      }
+      if (col >= 0 && row >= 0) cell[i] = row * (ny + 1) + col;
+    }
+  }
+  auto stage = [&](int slot, int buf) {
+    const cplx<T>* gr = gall + (size_t)s_list[slot] * gstride;
+    cplx<T>* w = win + (size_t)buf * kImWin * LD;
+#pragma unroll
+    for (int i = 0; i < kCells; ++i) {
+      const int v = threadIdx.x + 256 * i;
+      if (v < kImWin * kImWin)
+        cp_async_cell<T>(w + (v / kImWin) * LD + v % kImWin, gr + max(cell[i], 0), cell[i] >= 0);
+    }
+  };
+  stage(0, 0);
+  cp_async_commit();
+  // chi^2 slots beyond this problem's tiles: zero
+  if ((int)threadIdx.x < nact && qchi >= 0)
+    for (int sl = tl.slot + tl.ntiles; sl < nslots; sl += tl.ntiles) part.at(qchi, s_list[threadIdx.x])[sl] = 0.0;
+
+  // warps over (unit of 16 points, row group): nu units, ng groups of rows
+  const int nu = max(1, (tl.count + 15) >> 4), ng = 8 / nu;
+  const int unit = warp % nu, grp = warp / nu;
+  const bool on = grp < ng;
+  const int p0 = tl.start + unit * 16;
+  const int np = on ? min(16, tl.start + tl.count - p0) : 0;
+  int kq = 0, drq = 0, dcq = 0;
+  if (lane < np) {
+    const int2 pk = perm[p0 + lane];
+    kq = pk.x;
+    drq = pk.y & 0xff;
+    dcq = pk.y >> 8;
+  }
+  const unsigned int all = 0xffffffffu;
+  const int ka = __shfl_sync(all, kq, g), kb = __shfl_sync(all, kq, g + 8);
+  const int dra = __shfl_sync(all, drq, g), drb = __shfl_sync(all, drq, g + 8);
+  const int dca = __shfl_sync(all, dcq, g), dcb = __shfl_sync(all, dcq, g + 8);
+  const bool va = g < np, vb = g + 8 < np;
+  const bool two = np > 8;
+  // rows and columns of the window that the unit's points reach, in steps of 4
+  int rlo = __reduce_min_sync(all, lane < np ? drq : kImWin), rhi = __reduce_max_sync(all, lane < np ? drq + kTaps : 0);
+  int clo = __reduce_min_sync(all, lane < np ? dcq : kImWin), chi_ = __reduce_max_sync(all, lane < np ? dcq + kTaps : 0);
+  const int ns = (rhi - rlo + 3) >> 2, nk = (chi_ - clo + 3) >> 2;
+  rlo = min(rlo, kImWin - 4 * ns);
+  clo = min(clo, kImWin - 4 * nk);
+  double a0[kImSteps], a1[kImSteps];
+  unsigned int mir = 0;  // bit kk: column clo + 4 kk + t is mirrored (imaginary lanes only)
+#pragma unroll
+  for (int kk = 0; kk < kImSteps; ++kk) {
+    const int c = clo + 4 * kk + t;
+    const int ja = c - dca, jb = c - dcb;
+    a0[kk] = (va && kk < nk && ja >= 0 && ja < kTaps) ? wyd[(size_t)ka * kTaps + ja] : 0.0;
+    a1[kk] = (vb && kk < nk && jb >= 0 && jb < kTaps) ? wyd[(size_t)kb * kTaps + jb] : 0.0;
+    if ((g & 1) && half_col(tl.col0 + c, ny) < 0) mir |= 1u << kk;
+  }
+  const bool mixed = __any_sync(all, mir != 0);
+  const int per = (ns + ng - 1) / ng;
+  const int s0 = grp * per, s1 = on ? min(ns, s0 + per) : 0;
+  for (int i = 0; i < nact; ++i) {
+    if (PB > 1 && i + 1 < nact) stage(i + 1, (i + 1) & 1);
+    if (PB > 1) cp_async_commit();
+    if (PB > 1) cp_async_wait<1>();
+    else cp_async_wait<0>();
+    __syncthreads();  // window i has landed for every thread
+    const T* w = reinterpret_cast<const T*>(win + (size_t)(PB > 1 ? (i & 1) : 0) * kImWin * LD);
+    double y0[2] = {0.0, 0.0}, y1[2] = {0.0, 0.0};
+    for (int s = s0; s < s1; ++s) {
+      const int r = rlo + 4 * s;
+      const int ja = r + t - dra, jb = r + t - drb;
+      const double wa = (va && ja >= 0 && ja < kTaps) ? wxd[(size_t)ka * kTaps + ja] : 0.0;
+      const double wb = (vb && jb >= 0 && jb < kTaps) ? wxd[(size_t)kb * kTaps + jb] : 0.0;
+      const T* brow = w + 2 * ((r + (g >> 1)) * LD + clo + t) + (g & 1);
+      double d0[2][2] = {{0.0, 0.0}, {0.0, 0.0}}, d1[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+#pragma unroll
+      for (int kk = 0; kk < kImSteps; ++kk) {
+        if (kk < nk) {
+          double b = (double)brow[8 * kk];
+          if (mixed && ((mir >> kk) & 1u)) b = -b;
+          dmma_884(d0[kk & 1], a0[kk], b);
+          if (two) dmma_884(d1[kk & 1], a1[kk], b);
+        }
+      }
+      y0[0] = fma(wa, d0[0][0] + d0[1][0], y0[0]);
+      y0[1] = fma(wa, d0[0][1] + d0[1][1], y0[1]);
+      y1[0] = fma(wb, d1[0][0] + d1[1][0], y1[0]);
+      y1[1] = fma(wb, d1[0][1] + d1[1][1], y1[1]);
+    }
+    // over the four rows of a step (lanes t)
+#pragma unroll
+    for (int o = 1; o <= 2; o <<= 1) {
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        y0[q] += __shfl_xor_sync(all, y0[q], o);
+        y1[q] += __shfl_xor_sync(all, y1[q], o);
+      }
+    }
+    if (on && t < 2) {
+      const double2 v = t == 0 ? make_double2(y0[0], y0[1]) : make_double2(y1[0], y1[1]);
+      s_red[(i * 8 + warp) * 16 + 8 * t + g] = v;
+    }
+    if (PB > 1) __syncthreads();  // the buffer just read is refilled by the copies issued next
+  }
+  if (PB == 1) __syncthreads();
+  // residual, chi^2 and models: a warp per problem, lanes over the points
+  for (int i = warp; i < nact; i += 8) {
+    const int b = s_list[i];
+    double chi = 0.0;
+    for (int j = lane; j < tl.count; j += 32) {
+      double fr = 0.0, fi = 0.0;
+      for (int q = 0; q < ng; ++q) {  // row groups in order
+        const double2 v = s_red[(i * 8 + (j >> 4) + q * nu) * 16 + (j & 15)];
+        fr += v.x;
+        fi += v.y;
+      }
+      const int k = perm[tl.start + j].x;
+      const size_t e = (size_t)b * geo.y2_bstride + k;
+      fr *= inv_mm;
+      fi *= -inv_mm;
+      if (ax_base) {
+        const double2 ab = ax_base[e];
+        fr += ab.x;
+        fi += ab.y;
+      }
+      if (ax_out) ax_out[e] = make_double2(fr, fi);
+      const double wgt = geo.weight[k];
+      const double rr = (geo.vis_r[k] - fr) * wgt, ri = (geo.vis_i[k] - fi) * wgt;
+      chi += rr * rr + ri * ri;
+      if (y2) y2[e] = mk<T>((T)(rr * wgt), (T)(ri * wgt));
+    }
+    chi = warp_sum(chi);
+    if (lane == 0 && qchi >= 0) part.at(qchi, b)[tl.slot] = chi;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Spreading, output-stationary: the stored half grid is cut into tiles of
+// 8 rows x 16 columns, each with the list of the virtual points that have a
+// tap on it (every uv point as itself, imaginary part negated, and mirrored,
+// both weight vectors reversed, each with half the residual).  A tile is four
+// 8 x 8 products over the list,
+//   D[(row, re/im)][col] = sum_p (wx_p[row] y_p[re/im]) wy_p[col],
+// four rows x {re, im} by eight columns, K = points, so a single problem fills
+// the matrix tile.  A CTA takes up to kSmSeg list entries and up to PB
+// problems: its warps go over (problem, block) and, with one problem, over the
+// even and odd steps of 4 points too.  Each block's sum is the even steps'
+// plus the odd steps' whatever the mapping, and longer lists are cut into
+// segments whose partial tiles the tile's last CTA adds in segment order, so
+// neither the batch nor the order of the CTAs changes a result.
+// The weights are read where they lie (48 values a point, shared by the tiles
+// around it): cached, with the taps outside [0, 24) as zeros.
+// ---------------------------------------------------------------------------
+constexpr int kSmRows = 8, kSmCols = 16;
+constexpr int kSmSeg = 256;  // list entries per CTA at most
+
+struct SmItem {
+  int tile;          // tile of the stored half grid, row-major
+  int start, count;  // list entries; count a multiple of 8
+  int seg, nseg;     // segment of the tile's list
+  int scratch;       // scratch slot of the tile's segment 0
+  int ticket;        // the tile's ticket
+  int prob;          // its problem, or -1 (shared points)
+};
+
+struct SmPoint {
+  unsigned int k24;  // first weight of the point
+  int x0, y0;  // first tap, virtual
+  int fl;      // mirrored
+};
+
+template <typename T, int PB> constexpr size_t sm_smem() {
+  return (size_t)kSmSeg * sizeof(SmPoint) + sizeof(double2) * (size_t)PB * kSmSeg + sizeof(double) * 4 * 64;
+}
+
+// the products of the warp's MB x NB blocks (from mb0, nb0) over its CH step
+// parities (from ch0)
+template <int MB, int NB, int CH>
+__device__ __forceinline__ void spread_products(const SmPoint* s_pt, const double* s_yp, int count, int mb0, int nb0,
+                                                int ch0, int row_base, int col_base, int nx, int ny, int lane,
+                                                const double* __restrict__ wxd, const double* __restrict__ wyd,
+                                                double (&acc)[CH][MB][NB][2]) {
+  const int g = lane >> 2, t = lane & 3;
+  constexpr int kOut = 1 << 28;  // no tap reaches it
+  int mr[MB], mc[NB];
+#pragma unroll
+  for (int m = 0; m < MB; ++m) {
+    const int row = row_base + 4 * (mb0 + m) + (g >> 1);
+    mr[m] = row < nx ? row : row < 2 * nx ? row - 2 * nx : kOut;
+  }
+#pragma unroll
+  for (int n = 0; n < NB; ++n) {
+    const int col = col_base + 8 * (nb0 + n) + g;
+    mc[n] = col < ny ? col : col == ny ? -ny : kOut;
+  }
+#pragma unroll
+  for (int c = 0; c < CH; ++c)
+#pragma unroll
+    for (int m = 0; m < MB; ++m)
+#pragma unroll
+      for (int n = 0; n < NB; ++n) acc[c][m][n][0] = acc[c][m][n][1] = 0.0;
+#pragma unroll 2
+  for (int e0 = 0; e0 < count; e0 += 8) {
+#pragma unroll
+    for (int c = 0; c < CH; ++c) {
+      const int e = e0 + 4 * (ch0 + c) + t;
+      const SmPoint p = s_pt[e];
+      const double y = s_yp[2 * e + (g & 1)];
+      double a[MB], b[NB];
+#pragma unroll
+      for (int m = 0; m < MB; ++m) {
+        const int j = mr[m] - p.x0;
+        a[m] = (unsigned)j < (unsigned)kTaps ? __ldg(wxd + p.k24 + (p.fl ? kTaps - 1 - j : j)) * y : 0.0;
+      }
+#pragma unroll
+      for (int n = 0; n < NB; ++n) {
+        const int j = mc[n] - p.y0;
+        b[n] = (unsigned)j < (unsigned)kTaps ? __ldg(wyd + p.k24 + (p.fl ? kTaps - 1 - j : j)) : 0.0;
+      }
+#pragma unroll
+      for (int m = 0; m < MB; ++m)
+#pragma unroll
+        for (int n = 0; n < NB; ++n) dmma_884(acc[c][m][n], a[m], b[n]);
+    }
+  }
+}
+
+template <typename T, int PB>
+__global__ void __launch_bounds__(256, 2)
+    k_nufft_spread_mma(NufftGeom<T> geo, const double* __restrict__ wxd, const double* __restrict__ wyd,
+                       const SmItem* __restrict__ items, const unsigned int* __restrict__ vlist,
+                       const cplx<T>* __restrict__ y2, cplx<T>* __restrict__ gall, long gstride, int nx, int ny,
+                       int ntcol, const ProbState* __restrict__ st, int gate, int B, double* __restrict__ scratch,
+                       unsigned int* __restrict__ tickets) {
+  extern __shared__ __align__(16) unsigned char sm_smem_raw[];
+  SmPoint* s_pt = reinterpret_cast<SmPoint*>(sm_smem_raw);
+  double2* s_y = reinterpret_cast<double2*>(sm_smem_raw + (size_t)kSmSeg * sizeof(SmPoint));  // [PB][kSmSeg]
+  double* s_ex = reinterpret_cast<double*>(s_y + (size_t)PB * kSmSeg);                        // [4 blocks][64]
+  __shared__ int s_list[PB];
+  __shared__ int s_cnt[8];
+  __shared__ unsigned int s_ticket;
+  const SmItem it = items[blockIdx.x];
+  int nact;
+  if (PB > 1) {
+    nact = active_chunk<PB>(st, gate, B, blockIdx.y, s_list, s_cnt, geo.act_lists);
+  } else {
+    const int b = it.prob >= 0 ? it.prob : (int)blockIdx.y;
+    nact = gate_ok(st[b], gate) ? 1 : 0;
+    if (threadIdx.x == 0) s_list[0] = b;
+    __syncthreads();
+  }
+  if (nact == 0) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int tr = it.tile / ntcol, tcl = it.tile - tr * ntcol;
+  const int row_base = tr * kSmRows, col_base = tcl * kSmCols;
+  for (int e = threadIdx.x; e < it.count * nact; e += blockDim.x) {
+    const int i = e / it.count, q = e - i * it.count;
+    const unsigned int code = vlist[it.start + q];
+    double2 y = make_double2(0.0, 0.0);
+    if (code != 0xffffffffu) {
+      const int k = (int)(code >> 1);
+      const cplx<T> r = y2[(size_t)s_list[i] * geo.y2_bstride + k];
+      y = make_double2(0.5 * (double)r.x, (code & 1u) ? 0.5 * (double)r.y : -0.5 * (double)r.y);
+    }
+    s_y[(size_t)i * kSmSeg + q] = y;
+    if (i == 0) {
+      SmPoint p{0, 1 << 29, 1 << 29, 0};  // an empty entry: no tap anywhere
+      if (code != 0xffffffffu) {
+        const int k = (int)(code >> 1), fl = (int)(code & 1u);
+        p.k24 = (unsigned int)k * kTaps;
+        p.x0 = fl ? -geo.mx[k] - kMSP : geo.mx[k] - (kMSP - 1);
+        p.y0 = fl ? -geo.my[k] - kMSP : geo.my[k] - (kMSP - 1);
+        p.fl = fl;
+      }
+      s_pt[q] = p;
+    }
+  }
+  __syncthreads();
+  // warps over (problem, block of the tile): the more warps a problem gets,
+  // the fewer blocks each takes
+  const int wpp = nact > 4 ? 1 : nact > 2 ? 2 : nact > 1 ? 4 : 8;  // warps per problem
+  const int prob = warp / wpp, sub = warp - prob * wpp;
+  const bool on = prob < nact;
+  const double* yp = reinterpret_cast<const double*>(s_y + (size_t)(on ? prob : 0) * kSmSeg);
+  const int count = on ? it.count : 0;
+  double d[4][2];  // blocks 2 mb + nb of the tile held by this warp: [blk0, blk0 + nblk)
+  int blk0 = 0, nblk = 0;
+  if (PB > 1 && wpp == 1) {
+    double acc[2][2][2][2];
+    spread_products<2, 2, 2>(s_pt, yp, count, 0, 0, 0, row_base, col_base, nx, ny, lane, wxd, wyd, acc);
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) d[q][h] = acc[0][q >> 1][q & 1][h] + acc[1][q >> 1][q & 1][h];
+    nblk = 4;
+  } else if (PB > 1 && wpp == 2) {
+    double acc[2][1][2][2];
+    spread_products<1, 2, 2>(s_pt, yp, count, sub, 0, 0, row_base, col_base, nx, ny, lane, wxd, wyd, acc);
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) d[q][h] = acc[0][0][q][h] + acc[1][0][q][h];
+    blk0 = 2 * sub;
+    nblk = 2;
+  } else if (PB > 1 && wpp == 4) {
+    double acc[2][1][1][2];
+    spread_products<1, 1, 2>(s_pt, yp, count, sub >> 1, sub & 1, 0, row_base, col_base, nx, ny, lane, wxd, wyd, acc);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) d[0][h] = acc[0][0][0][h] + acc[1][0][0][h];
+    blk0 = sub;
+    nblk = 1;
+  } else {
+    double acc[1][1][1][2];
+    const int blk = sub & 3;
+    spread_products<1, 1, 1>(s_pt, yp, count, blk >> 1, blk & 1, sub >> 2, row_base, col_base, nx, ny, lane, wxd, wyd,
+                             acc);
+    if (sub >> 2) {
+      s_ex[blk * 64 + 2 * lane] = acc[0][0][0][0];
+      s_ex[blk * 64 + 2 * lane + 1] = acc[0][0][0][1];
+    }
+    __syncthreads();  // (uniform: nact == 1)
+    blk0 = blk;
+    nblk = (sub >> 2) ? 0 : 1;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) d[0][h] = acc[0][0][0][h] + s_ex[blk * 64 + 2 * lane + h];
+  }
+  if (!on) nblk = 0;
+  constexpr int kPart = 4 * 64;  // doubles of one problem's tile
+  if (it.nseg > 1) {
+    const size_t cs = (size_t)gridDim.y * PB * kPart;
+    double* mine = scratch + (size_t)(it.scratch + it.seg) * cs + ((size_t)blockIdx.y * PB + prob) * kPart;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (q < nblk) *reinterpret_cast<double2*>(mine + (blk0 + q) * 64 + 2 * lane) = make_double2(d[q][0], d[q][1]);
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_ticket = atomicAdd(&tickets[(size_t)it.ticket * gridDim.y + blockIdx.y], 1u);
+    __syncthreads();
+    if (s_ticket != (unsigned int)(it.nseg - 1)) return;
+    __threadfence();
+#pragma unroll
+    for (int q = 0; q < 4; ++q) d[q][0] = d[q][1] = 0.0;
+    for (int sg = 0; sg < it.nseg; ++sg) {
+      const double* p = scratch + (size_t)(it.scratch + sg) * cs + ((size_t)blockIdx.y * PB + prob) * kPart;
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (q < nblk) {
+          const double2 v = __ldcg(reinterpret_cast<const double2*>(p + (blk0 + q) * 64 + 2 * lane));
+          d[q][0] += v.x;
+          d[q][1] += v.y;
+        }
+    }
+    if (threadIdx.x == 0) tickets[(size_t)it.ticket * gridDim.y + blockIdx.y] = 0u;  // for the next launch
+  }
+  if (nblk == 0) return;
+  // lane (g, t): row g >> 1, re or im (g & 1), columns 2t, 2t + 1; lanes g and
+  // g ^ 1 exchange so that each writes one complex cell
+  const int g = lane >> 2, t = lane & 3;
+  cplx<T>* gr = gall + (size_t)s_list[prob] * gstride;
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    if (q < nblk) {
+      const double other = __shfl_xor_sync(0xffffffffu, (g & 1) ? d[q][0] : d[q][1], 4);
+      const double re = (g & 1) ? other : d[q][0], im = (g & 1) ? d[q][1] : other;
+      const int blk = blk0 + q;
+      const int row = row_base + 4 * (blk >> 1) + (g >> 1), col = col_base + 8 * (blk & 1) + 2 * t + (g & 1);
+      if (row < 2 * nx && col <= ny) gr[(size_t)row * (ny + 1) + col] = mk<T>((T)re, (T)im);
+    }
+}
+
+}  // namespace mf

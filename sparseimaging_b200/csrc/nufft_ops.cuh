@@ -1668,8 +1668,8 @@ namespace mf {
 // and the f(z) inside Q agree to the bit and the backtracking test is not
 // decided by rounding.  Grid (cdiv(chi slots, 8), B) for shared geometry
 // (one warp per slot), (chi slots, B) otherwise; 256 threads.
-template <typename T> __device__ __forceinline__ int slots_of(const NufftGeom<T>& geo, int ppw) {
-  const int m = geo.pt_hi[0];
+template <typename T> __device__ __forceinline__ int slots_of(const NufftGeom<T>& geo, int b, int ppw) {
+  const int m = geo.pt_hi[b] - geo.pt_lo[b];
   return max(1, (m + 8 * ppw - 1) / (8 * ppw));
 }
 
@@ -1695,12 +1695,12 @@ __global__ void k_nufft_resid_model(NufftGeom<T> geo, const double2* __restrict_
     // interpolation's order (per warp w in q order, then over w)
     __shared__ double s_t[8][8 * 32];
     const int slot = blockIdx.x * 8 + warp;
-    if (slot >= slots_of(geo, ppw)) {  // a slot beyond the points (padding for another kernel's CTAs)
+    if (slot >= slots_of(geo, b, ppw)) {  // a slot beyond the points (padding for another kernel's CTAs)
       if (lane == 0 && qchi >= 0 && slot < nslots) part.at(qchi, b)[slot] = 0.0;
       return;
     }
-    const int mtot = geo.pt_hi[0];
-    const int n = 8 * ppw, k0 = slot * n;
+    const int mtot = geo.pt_hi[b];
+    const int n = 8 * ppw, k0 = geo.pt_lo[b] + slot * n;
     for (int l = lane; l < n; l += 32) s_t[warp][l] = (k0 + l < mtot) ? term(k0 + l) : 0.0;
     __syncwarp();
     if (lane == 0 && qchi >= 0) {

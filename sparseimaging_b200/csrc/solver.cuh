@@ -24,6 +24,7 @@
 #include "fftvar_ops.cuh"
 #include "fgp.cuh"
 #include "mfista_ops.cuh"
+#include "nufft_mma.cuh"
 #include "nufft_ops.cuh"
 
 #include "../../include/mfista_b200.h"
@@ -273,6 +274,12 @@ template <typename T> struct NufftOp : Op {
   bool spread_tc = false;
   DevMem d_sitems, d_svlist, d_sscratch, d_stickets, d_safrag, d_sbx;
   int nsitems = 0, stc_cols = 0;
+  // interpolation and spreading on the FP64 matrix instruction
+  // (k_nufft_interp_mma, k_nufft_spread_mma)
+  bool interp_mma = false, spread_mma = false;
+  DevMem d_im, d_imperm, d_smitems, d_smlist, d_smscratch, d_smtickets;
+  DevMem d_wxd, d_wyd;  // FP64 weights of an FP32 operator (wxd(), wyd())
+  int nim = 0, nsm = 0, sm_cols = 0;
   // chi^2 partial slots every interpolation kernel of this operator writes
   // (at least its own CTA count; the extra CTAs write zeros), so that the
   // CUDA-core, tensor-core and FP64 kernels fill the same slots
@@ -281,7 +288,8 @@ template <typename T> struct NufftOp : Op {
   long gstride = 0;
   double inv_mm = 0;
 
-  NufftOp(Ctx& ctx, const NufftInput& in, bool correct = false) : c(ctx) {
+  // forward_only: no adjoint (the FP64 operator of the anchors)
+  NufftOp(Ctx& ctx, const NufftInput& in, bool correct = false, bool forward_only = false) : c(ctx) {
     if (const char* f = getenv("MFISTA_INTERP_FLY")) interp_fly = f[0] == '1';
     if (const char* f = getenv("MFISTA_FFT_DYN")) fft_dyn = f[0] != '0';
     if (sizeof(T) == 4 && in.shared != 0 && in.M < kItcMaxPoints) {
@@ -290,11 +298,17 @@ template <typename T> struct NufftOp : Op {
       const char* f2 = getenv("MFISTA_SPREAD_TC");
       spread_tc = !(f2 && f2[0] == '0');
     }
+    auto off = [](const char* name) {
+      const char* e = getenv(name);
+      return e && e[0] == '0';
+    };
+    interp_mma = !interp_tc && !off("MFISTA_INTERP_TC");
+    spread_mma = !spread_tc && !off("MFISTA_SPREAD_TC");
     // with the tensor-core interpolation the points-per-warp knob only sets
     // the FP64 anchor interpolation's and the model residual's partition:
     // 8 points per warp (the autotuner's choice on the lambda grid) keeps
     // the chi^2 slot count at the tile count
-    if (interp_tc) ippw = 8;
+    if (interp_tc || interp_mma) ippw = 8;
     nx = in.Nx;
     ny = in.Ny;
     B = ctx.B;
@@ -343,30 +357,19 @@ template <typename T> struct NufftOp : Op {
     // spread tiles (16 x 16 for the shared-geometry kernels)
     if (shared) tile_r = tile_c = 16;
     ntiles = cdiv(2 * nx, tile_r) * cdiv(ny + 1, tile_c);
-    int ngeo = shared ? 1 : B;
-    std::vector<int> tptr;
-    std::vector<int> tpts;
-    tptr.reserve((size_t)ngeo * ntiles + 1);
-    tptr.push_back(0);
-    for (int g = 0; g < ngeo; ++g) {
-      std::vector<std::vector<int>> lists(ntiles);
-      bin_points(mx, my, lo[g], hi[g], nx, ny, tile_r, tile_c, lists);
-      for (int t = 0; t < ntiles; ++t) {
-        tpts.insert(tpts.end(), lists[t].begin(), lists[t].end());
-        tptr.push_back((int)tpts.size());
-      }
-    }
-    d_tptr.upload(tptr.data(), tptr.size());
-    d_tpts.upload(tpts.data(), std::max<size_t>(tpts.size(), 1));
-    if (shared) {  // spreading launch order: tiles by falling point count (ties by index)
-      std::vector<int> ord(ntiles);
-      for (int t = 0; t < ntiles; ++t) ord[t] = t;
-      std::stable_sort(ord.begin(), ord.end(),
-                       [&](int a, int b) { return tptr[a + 1] - tptr[a] > tptr[b + 1] - tptr[b]; });
-      d_tord.upload(ord.data(), ord.size());
-    }
+    if (!spread_mma && !spread_tc && !forward_only) build_tap_lists(mx, my, lo, hi);
     if (interp_tc) build_itc_tiles(mx, my);
     if (spread_tc) build_stc_items(mx, my);
+    if (interp_mma) build_im_tiles(mx, my, lo, hi);
+    if (spread_mma && !forward_only) build_sm_items(mx, my, lo, hi);
+    if (sizeof(T) == 4 && (interp_mma || spread_mma) && mtot > 0) {
+      d_wxd.alloc(sizeof(double) * (size_t)mtot * kTaps);
+      d_wyd.alloc(sizeof(double) * (size_t)mtot * kTaps);
+      k_nufft_prep_points<double><<<cdiv(mtot, 256), 256>>>(d_u.as<double>(), d_v.as<double>(), d_mx.as<int>(),
+                                                             d_my.as<int>(), mtot, nx, ny, d_wxd.as<double>(),
+                                                             d_wyd.as<double>());
+      MF_LAUNCH_CK();
+    }
     // FFTs: rows as complex length Ny, columns length 2Nx
     fh.init(ny);
     fcol.init(2 * nx);
@@ -389,9 +392,9 @@ template <typename T> struct NufftOp : Op {
     set_smem(k_nufft_spread_shared<T>, spread_smem());
     MF_CK(cudaFuncSetAttribute(k_nufft_spread_shared<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     if (correct && sizeof(T) == 4) {
-      exact.reset(new NufftOp<double>(ctx, in, false));
+      exact.reset(new NufftOp<double>(ctx, in, false, true));
       exact->ippw = ippw;  // its chi^2 partials land in the same slots as ours
-      exact->chi_pad = chi_pad;
+      exact->chi_pad = chi_pad = std::max(chi_pad, exact->chi_pad);
       d_axa.alloc(sizeof(double2) * (size_t)y2n);
       const char* nm = getenv("MFISTA_NO_MODEL_Z");  // direct forward at z instead (comparison runs)
       model = !(nm && nm[0] == '1');
@@ -421,7 +424,193 @@ template <typename T> struct NufftOp : Op {
     MF_CK(cudaDeviceSynchronize());
   }
 
-  int interp_blocks() const { return std::max({1, cdiv(mmax, shared ? 8 * ippw : 8), chi_pad}); }
+  // points per warp of the CUDA-core partition (also the model residual's)
+  int part_ppw() const { return shared || interp_mma ? ippw : 1; }
+  int interp_blocks() const { return std::max({1, cdiv(mmax, 8 * part_ppw()), chi_pad}); }
+
+  const double* wxd() const { return sizeof(T) == 8 ? d_wx.as<double>() : d_wxd.as<double>(); }
+  const double* wyd() const { return sizeof(T) == 8 ? d_wy.as<double>() : d_wyd.as<double>(); }
+
+  // the CUDA-core spreading's tile lists
+  void build_tap_lists(const std::vector<int>& mx, const std::vector<int>& my, const std::vector<int>& lo,
+                       const std::vector<int>& hi) {
+    int ngeo = shared ? 1 : B;
+    std::vector<int> tptr;
+    std::vector<int> tpts;
+    tptr.reserve((size_t)ngeo * ntiles + 1);
+    tptr.push_back(0);
+    for (int g = 0; g < ngeo; ++g) {
+      std::vector<std::vector<int>> lists(ntiles);
+      bin_points(mx, my, lo[g], hi[g], nx, ny, tile_r, tile_c, lists);
+      for (int t = 0; t < ntiles; ++t) {
+        tpts.insert(tpts.end(), lists[t].begin(), lists[t].end());
+        tptr.push_back((int)tpts.size());
+      }
+    }
+    d_tptr.upload(tptr.data(), tptr.size());
+    d_tpts.upload(tpts.data(), std::max<size_t>(tpts.size(), 1));
+    if (shared) {  // spreading launch order: tiles by falling point count (ties by index)
+      std::vector<int> ord(ntiles);
+      for (int t = 0; t < ntiles; ++t) ord[t] = t;
+      std::stable_sort(ord.begin(), ord.end(),
+                       [&](int a, int b) { return tptr[a + 1] - tptr[a] > tptr[b + 1] - tptr[b]; });
+      d_tord.upload(ord.data(), ord.size());
+    }
+  }
+
+  // k_nufft_interp_mma's tiles: each problem's points (once, when shared)
+  // binned by their first tap into kImTile x kImTile virtual tiles, ordered
+  // within a tile by 4 x 4 blocks so that 16 consecutive points lie close
+  // together, and cut into CTAs of at most kImPts.  A problem without points
+  // gets one empty tile (it writes the problem's chi^2).
+  void build_im_tiles(const std::vector<int>& mx, const std::vector<int>& my, const std::vector<int>& lo,
+                      const std::vector<int>& hi) {
+    struct Key {
+      long long tile;
+      int sub, k;
+    };
+    std::vector<ImTileItem> tiles;
+    std::vector<int2> perm;
+    std::vector<Key> keys;
+    const int ngeo = shared ? 1 : B;
+    int most = 1;
+    auto first = [](int m) { return (long long)std::max(-(1 << 28), std::min(1 << 28, m)) - (kMSP - 1); };
+    auto fdiv = [](long long a) { return a >= 0 ? a / kImTile : -((-a + kImTile - 1) / kImTile); };
+    for (int g = 0; g < ngeo; ++g) {
+      keys.clear();
+      for (int k = lo[g]; k < hi[g]; ++k) {
+        const long long x = first(mx[k]), y = first(my[k]);
+        const long long tx = fdiv(x), ty = fdiv(y);
+        const int dr = (int)(x - tx * kImTile), dc = (int)(y - ty * kImTile);
+        keys.push_back(Key{tx * (1ll << 32) + ty, ((dr >> 2) << 12) | ((dc >> 2) << 8) | (dr << 4) | dc, k});
+      }
+      std::sort(keys.begin(), keys.end(), [](const Key& a, const Key& b) {
+        return a.tile != b.tile ? a.tile < b.tile : a.sub != b.sub ? a.sub < b.sub : a.k < b.k;
+      });
+      const size_t t0 = tiles.size();
+      for (size_t i = 0; i < keys.size();) {
+        size_t j = i;
+        while (j < keys.size() && keys[j].tile == keys[i].tile) ++j;
+        const int k0 = keys[i].k;
+        const long long tx = fdiv(first(mx[k0])), ty = fdiv(first(my[k0]));
+        for (size_t a = i; a < j; a += kImPts)
+          tiles.push_back(ImTileItem{(int)(tx * kImTile), (int)(ty * kImTile), (int)(perm.size() + (a - i)),
+                                     (int)std::min<size_t>(kImPts, j - a), shared ? -1 : g, 0, 0, 0});
+        for (size_t a = i; a < j; ++a) {
+          const int sub = keys[a].sub;
+          perm.push_back(make_int2(keys[a].k, ((sub >> 4) & 15) | ((sub & 15) << 8)));
+        }
+        i = j;
+      }
+      if (tiles.size() == t0) tiles.push_back(ImTileItem{0, 0, 0, 0, shared ? -1 : g, 0, 0, 0});
+      const int nt = (int)(tiles.size() - t0);
+      for (int q = 0; q < nt; ++q) {
+        tiles[t0 + q].slot = q;
+        tiles[t0 + q].ntiles = nt;
+      }
+      most = std::max(most, nt);
+    }
+    // launch order: fullest CTAs first, so that the last wave holds short ones
+    std::stable_sort(tiles.begin(), tiles.end(),
+                     [](const ImTileItem& a, const ImTileItem& b) { return a.count > b.count; });
+    nim = (int)tiles.size();
+    chi_pad = std::max(chi_pad, most);
+    if (perm.empty()) perm.push_back(make_int2(0, 0));
+    d_im.upload(tiles.data(), tiles.size());
+    d_imperm.upload(perm.data(), perm.size());
+    set_smem(k_nufft_interp_mma<T, 1>, im_smem<T, 1>());
+    set_smem(k_nufft_interp_mma<T, kMmaProb>, im_smem<T, kMmaProb>());
+  }
+
+  // k_nufft_spread_mma's tiles and lists: per stored tile the virtual points
+  // (point << 1 | mirrored) with a tap on it, in (point, mirrored) order,
+  // padded with empty entries to a multiple of 8 and cut into segments.
+  void build_sm_items(const std::vector<int>& mx, const std::vector<int>& my, const std::vector<int>& lo,
+                      const std::vector<int>& hi) {
+    const int ntr = cdiv(2 * nx, kSmRows);
+    sm_cols = cdiv(ny + 1, kSmCols);
+    const int nt = ntr * sm_cols, ngeo = shared ? 1 : B;
+    // tiles of the taps v0 .. v0 + 23 along one axis (at most 8, none twice)
+    auto touch_rows = [&](long long v0, int* out) {
+      int n = 0;
+      for (int part = 0; part < 2; ++part) {  // [0, nx) as it is, [-nx, 0) wrapped to [nx, 2nx)
+        const long long a = std::max<long long>(v0, part ? -nx : 0), b = std::min<long long>(v0 + kTaps - 1, part ? -1 : nx - 1);
+        if (a > b) continue;
+        const int sh = part ? 2 * nx : 0;
+        for (int t = (int)(a + sh) / kSmRows; t <= (int)(b + sh) / kSmRows; ++t) {
+          bool seen = false;
+          for (int q = 0; q < n; ++q) seen |= out[q] == t;
+          if (!seen) out[n++] = t;
+        }
+      }
+      return n;
+    };
+    auto touch_cols = [&](long long v0, int* out) {
+      int n = 0;
+      const long long a = std::max<long long>(v0, 0), b = std::min<long long>(v0 + kTaps - 1, ny - 1);
+      if (a <= b)
+        for (int t = (int)a / kSmCols; t <= (int)b / kSmCols; ++t) out[n++] = t;
+      if (v0 <= -ny && -ny < v0 + kTaps) {  // the tap at -Ny is the last stored column
+        const int t = ny / kSmCols;
+        bool seen = false;
+        for (int q = 0; q < n; ++q) seen |= out[q] == t;
+        if (!seen) out[n++] = t;
+      }
+      return n;
+    };
+    std::vector<SmItem> items;
+    std::vector<unsigned int> flat;
+    std::vector<int> cnt(nt);
+    std::vector<size_t> at(nt);
+    int nscr = 0;
+    for (int g = 0; g < ngeo; ++g) {
+      auto each = [&](auto&& f) {
+        int rs[16], cs[16];
+        for (int k = lo[g]; k < hi[g]; ++k)
+          for (int fl = 0; fl < 2; ++fl) {
+            const long long x0 = fl ? -(long long)mx[k] - kMSP : (long long)mx[k] - (kMSP - 1);
+            const long long y0 = fl ? -(long long)my[k] - kMSP : (long long)my[k] - (kMSP - 1);
+            const int nc = touch_cols(y0, cs);
+            if (!nc) continue;
+            const int nr = touch_rows(x0, rs);
+            for (int a = 0; a < nr; ++a)
+              for (int b = 0; b < nc; ++b) f(rs[a] * sm_cols + cs[b], ((unsigned int)k << 1) | (unsigned int)fl);
+          }
+      };
+      std::fill(cnt.begin(), cnt.end(), 0);
+      each([&](int t, unsigned int) { ++cnt[t]; });
+      size_t pos = flat.size();
+      for (int t = 0; t < nt; ++t) {
+        at[t] = pos;
+        const int c8 = (cnt[t] + 7) & ~7;
+        const int nseg = std::max(1, cdiv(c8, kSmSeg));
+        for (int sg = 0; sg < nseg; ++sg)
+          items.push_back(SmItem{t, (int)(pos + (size_t)sg * kSmSeg), std::min(kSmSeg, c8 - sg * kSmSeg), sg, nseg, nscr,
+                                 g * nt + t, shared ? -1 : g});
+        if (nseg > 1) nscr += nseg;
+        pos += c8;
+      }
+      flat.resize(pos, 0xffffffffu);
+      each([&](int t, unsigned int code) { flat[at[t]++] = code; });
+    }
+    // launch order: longest segments first
+    std::stable_sort(items.begin(), items.end(), [](const SmItem& a, const SmItem& b) { return a.count > b.count; });
+    nsm = (int)items.size();
+    if (flat.empty()) flat.push_back(0xffffffffu);
+    d_smitems.upload(items.data(), items.size());
+    d_smlist.upload(flat.data(), flat.size());
+    const int pb = mma_prob(), chunks = mma_chunks();
+    d_smscratch.alloc(sizeof(double) * (size_t)std::max(nscr, 1) * chunks * pb * 256);
+    d_smtickets.alloc(sizeof(unsigned int) * (size_t)ngeo * nt * chunks);
+    MF_CK(cudaMemset(d_smtickets.p, 0, d_smtickets.bytes));
+    set_smem(k_nufft_spread_mma<T, 1>, sm_smem<T, 1>());
+    set_smem(k_nufft_spread_mma<T, kMmaProb>, sm_smem<T, kMmaProb>());
+  }
+  // problems per CTA of the two: one where each problem has its own points
+  // or the batch is a single problem, else chunks of 8
+  static constexpr int kMmaProb = 8;
+  int mma_prob() const { return shared && B > 1 ? kMmaProb : 1; }
+  int mma_chunks() const { return shared ? cdiv(B, mma_prob()) : 1; }
 
   // Tensor-core spreading: each 8 x 16 tile of the stored half grid lists
   // the virtual points (point | mirrored << 24) with a tap on it, in (point,
@@ -557,6 +746,19 @@ template <typename T> struct NufftOp : Op {
   void launch_interp(cudaStream_t s, cplx<T>* g, int gate, int qchi, cplx<T>* y2, const double2* base = nullptr,
                      double2* out = nullptr) {
     const NufftGeom<T> geo = geo_now();
+    if (interp_mma) {
+      const dim3 grid(nim, mma_chunks());
+      if (mma_prob() == 1)
+        k_nufft_interp_mma<T, 1><<<grid, 256, im_smem<T, 1>(), s>>>(
+            geo, wxd(), wyd(), d_im.as<ImTileItem>(), d_imperm.as<int2>(), g, gstride, nx, ny, inv_mm, c.st, gate, c.part,
+            qchi, chi_slots(), y2, B, base, out);
+      else
+        k_nufft_interp_mma<T, kMmaProb><<<grid, 256, im_smem<T, kMmaProb>(), s>>>(
+            geo, wxd(), wyd(), d_im.as<ImTileItem>(), d_imperm.as<int2>(), g, gstride, nx, ny, inv_mm, c.st, gate, c.part,
+            qchi, chi_slots(), y2, B, base, out);
+      MF_LAUNCH_CK();
+      return;
+    }
     // FP32: grouped kernel; FP64 (register-bound with 2G double sums): one
     // problem at a time.  Both chunk the batch's active problems.
     if (shared) {
@@ -612,8 +814,9 @@ template <typename T> struct NufftOp : Op {
   bool models_z() const override { return model; }
 
   void forward_z(cudaStream_t s, int gate, int qchi) override {
-    const int gx = shared ? cdiv(chi_slots(), 8) : chi_slots();
-    k_nufft_resid_model<T><<<dim3(gx, B), 256, 0, s>>>(geo, d_az.as<double2>(), d_y2.as<cplx<T>>(), shared ? 1 : 0,
+    const bool by_slot = shared || interp_mma;
+    const int gx = by_slot ? cdiv(chi_slots(), 8) : chi_slots();
+    k_nufft_resid_model<T><<<dim3(gx, B), 256, 0, s>>>(geo, d_az.as<double2>(), d_y2.as<cplx<T>>(), by_slot ? 1 : 0,
                                                         ippw, chi_slots(), c.st, gate, c.part, qchi);
     MF_LAUNCH_CK();
   }
@@ -645,6 +848,19 @@ template <typename T> struct NufftOp : Op {
 
   void launch_spread(cudaStream_t s, cplx<T>* g, int gate) {
     const NufftGeom<T> geo = geo_now();
+    if (spread_mma) {
+      const dim3 grid(nsm, mma_chunks());
+      if (mma_prob() == 1)
+        k_nufft_spread_mma<T, 1><<<grid, 256, sm_smem<T, 1>(), s>>>(
+            geo, wxd(), wyd(), d_smitems.as<SmItem>(), d_smlist.as<unsigned int>(), d_y2.as<cplx<T>>(), g, gstride, nx, ny,
+            sm_cols, c.st, gate, B, d_smscratch.as<double>(), d_smtickets.as<unsigned int>());
+      else
+        k_nufft_spread_mma<T, kMmaProb><<<grid, 256, sm_smem<T, kMmaProb>(), s>>>(
+            geo, wxd(), wyd(), d_smitems.as<SmItem>(), d_smlist.as<unsigned int>(), d_y2.as<cplx<T>>(), g, gstride, nx, ny,
+            sm_cols, c.st, gate, B, d_smscratch.as<double>(), d_smtickets.as<unsigned int>());
+      MF_LAUNCH_CK();
+      return;
+    }
     if constexpr (sizeof(T) == 4) {
       if (spread_tc) {
         k_nufft_spread_tc<<<dim3(nsitems, cdiv(B, kStcProb)), 256, 0, s>>>(
@@ -705,7 +921,7 @@ template <typename T> struct NufftOp : Op {
   }
 
   int chi_slots() const override { return interp_blocks(); }
-  int max_chi_slots() const override { return std::max({1, cdiv(mmax, 8), chi_pad}); }
+  int max_chi_slots() const override { return std::max({1, cdiv(mmax, 8), chi_pad}); }  // points per warp >= 1
   int tsv_slots() const override { return nx; }  // row-pass CTAs at rows_per_cta = 1
 
   LaunchShapes shapes() const override {
