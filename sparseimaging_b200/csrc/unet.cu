@@ -53,8 +53,10 @@ __host__ __device__ inline int cdiv(long a, long b) { return (int)((a + b - 1) /
 //   H/2 and the input is a's nearest 2x upsampling), channels [ca, ca+cb)
 //   from `b` ([n][cb][H][W]); when `amask` is set, a's values are multiplied
 //   by (amask > 0) (the ReLU derivative in the backward pass; amask has a's
-//   shape); out[n][co][y][x] (+)= bias[co] + sum w[co][ci][ky][kx] *
-//   in[ci][y+ky-1][x+kx-1], ReLU when relu, added to out when accumulate.
+//   shape); out[n][co][y][x] = bias[co] + sum w[co][ci][ky][kx] *
+//   in[ci][y+ky-1][x+kx-1], ReLU when relu.  Output channels [0, c1) go to
+//   `out` ([n][c1][H][W]), the others to `out2` ([n][cout-c1][H][W]): the
+//   backward pass writes the gradients of a concatenation's two producers.
 // Block: a 16 x 16 output tile, 128 threads with two vertically adjacent
 // pixels each, 16 output channels; input channels in chunks of 16 staged
 // (with halo) in shared memory with their weights.
@@ -68,7 +70,13 @@ struct ConvArgs {
   const __nv_bfloat16* w;  // [cout][ca+cb][3][3]
   const float* bias;       // [cout] or null
   float* out;
-  int cout, H, W, relu, accumulate;
+  int cout, H, W, relu;
+  float* out2;
+  int c1;
+  __device__ float* at(int n, int co, int y, int x) const {
+    return (co < c1 ? out + ((size_t)n * c1 + co) * H * W : out2 + ((size_t)n * (cout - c1) + co - c1) * H * W) +
+           (size_t)y * W + x;
+  }
 };
 
 constexpr int kCT = 16;  // tile edge
@@ -156,8 +164,7 @@ __global__ void __launch_bounds__(128) k_conv3x3(ConvArgs g) {
       if (co >= g.cout) break;
       float v = acc[p][c] + (g.bias ? g.bias[co] : 0.f);
       if (g.relu) v = fmaxf(v, 0.f);
-      float* o = g.out + (((size_t)n * g.cout + co) * g.H + y) * g.W + x;
-      *o = g.accumulate ? *o + v : v;
+      *g.at(n, co, y, x) = v;
     }
   }
 }
@@ -279,8 +286,7 @@ __global__ void __launch_bounds__(256) k_conv3x3_tc(ConvArgs g) {
         if (co >= g.cout || y >= g.H || x >= g.W) continue;
         float v = acc[m][j][e] + (g.bias ? g.bias[co] : 0.f);
         if (g.relu) v = fmaxf(v, 0.f);
-        float* o = g.out + (((size_t)n * g.cout + co) * g.H + y) * g.W + x;
-        *o = g.accumulate ? *o + v : v;
+        *g.at(n, co, y, x) = v;
       }
     }
 }
@@ -477,37 +483,50 @@ __global__ void __launch_bounds__(288) k_conv3x3_wgrad_tc(WgradArgs g) {
 
 constexpr size_t kWgradTcSmem = sizeof(uint32_t) * (2 * 16 * kWgG + 2 * 16 * kWgX);
 
-// out[i] = sum_t part[t][i] (t ascending), i < len
-__global__ void k_reduce_partials(const float* __restrict__ part, int ntiles, long len, float* __restrict__ out) {
-  long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+// Reductions.  All run as partial sums over many CTAs, the partials of a
+// group added in order by one thread per output (groups of about the square
+// root of the partials, so two short passes): deterministic, and enough CTAs
+// in flight.  One CTA per channel (16 CTAs at full resolution) and one thread
+// per weight over up to 2048 tiles took 9 of the 13.9 ms of a gradient at
+// 256 x 256, batch 8; these take 0.2 ms.
+
+// out[y][i] = sum of part[t][i] over the y-th `per` of the nt partials (t ascending), i < len
+__global__ void k_reduce_partials(const float* __restrict__ part, int nt, long len, int per, float* __restrict__ out) {
+  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= len) return;
+  const int t0 = blockIdx.y * per, t1 = min(nt, t0 + per);
   float s = 0.f;
-  for (int t = 0; t < ntiles; ++t) s += part[(size_t)t * len + i];
-  out[i] = s;
+#pragma unroll 8
+  for (int t = t0; t < t1; ++t) s += part[(size_t)t * len + i];
+  out[(size_t)blockIdx.y * len + i] = s;
 }
 
-// bias gradient: db[co] = sum_{n,y,x} g m (one block per channel, fixed order)
-__global__ void k_bias_grad(const float* __restrict__ g, const float* __restrict__ gmask, int n, int cout, int hw,
-                            float* __restrict__ db) {
-  __shared__ float sh[256];
-  const int co = blockIdx.x;
-  float s = 0.f;
-  for (int i = 0; i < n; ++i) {
-    const float* gp = g + ((size_t)i * cout + co) * hw;
-    const float* mp = gmask ? gmask + ((size_t)i * cout + co) * hw : nullptr;
-    for (int p = threadIdx.x; p < hw; p += blockDim.x) {
-      float v = gp[p];
-      if (mp && !(mp[p] > 0.f)) v = 0.f;
-      s += v;
-    }
-  }
+// sum of 256 threads' values (fixed tree), valid in thread 0
+__device__ __forceinline__ float block_sum256(float s, float* sh) {
   sh[threadIdx.x] = s;
   __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
+  for (int o = 128; o > 0; o >>= 1) {
+    if ((int)threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
     __syncthreads();
   }
-  if (threadIdx.x == 0) db[co] = sh[0];
+  return sh[0];
+}
+
+constexpr int kRedPix = 4096;  // pixels of one channel per CTA of the pixel sums
+
+// bias gradient partials: part[chunk][co] = sum of g m over a chunk of an
+// image's pixels; grid (chunks per image, cout, n)
+__global__ void __launch_bounds__(256) k_bias_grad(const float* __restrict__ g, const float* __restrict__ gmask, int hw,
+                                                   float* __restrict__ part) {
+  __shared__ float sh[256];
+  const int co = blockIdx.y, cout = gridDim.y, i = blockIdx.z;
+  const size_t base = ((size_t)i * cout + co) * hw;
+  const int p1 = min(hw, ((int)blockIdx.x + 1) * kRedPix);
+  float s = 0.f;
+#pragma unroll 4
+  for (int p = blockIdx.x * kRedPix + threadIdx.x; p < p1; p += 256) s += gmask[base + p] > 0.f ? g[base + p] : 0.f;
+  s = block_sum256(s, sh);
+  if (threadIdx.x == 0) part[((size_t)i * gridDim.x + blockIdx.x) * cout + co] = s;
 }
 
 // 2x2 max pooling (H, W even) and its gradient (to the first maximum)
@@ -566,42 +585,22 @@ __global__ void k_head(const float* __restrict__ h, int n, int c16, int hw, cons
   }
 }
 
-// head weight gradients: dw[c] = sum gpre h[c], db = sum gpre (fixed order)
-__global__ void k_head_wgrad(const float* __restrict__ h, const float* __restrict__ gpre, int n, int c16, int hw,
-                             float* __restrict__ dw, float* __restrict__ db) {
+// head gradient partials, as k_bias_grad: part[chunk][c] = sum gpre h[c]
+// (c < c16), sum gpre (c = c16: the bias), sum sq (c = c16 + 1: the loss);
+// grid (chunks per image, c16 + 2, n)
+__global__ void __launch_bounds__(256) k_head_sums(const float* __restrict__ h, const float* __restrict__ gpre,
+                                                   const float* __restrict__ sq, int c16, int hw,
+                                                   float* __restrict__ part) {
   __shared__ float sh[256];
-  const int c = blockIdx.x;  // c16 blocks for weights, one more for the bias
+  const int c = blockIdx.y, i = blockIdx.z;
+  const float* hp = h + ((size_t)i * c16 + c) * hw;
+  const float* gp = (c <= c16 ? gpre : sq) + (size_t)i * hw;
+  const int p1 = min(hw, ((int)blockIdx.x + 1) * kRedPix);
   float s = 0.f;
-  for (int i = 0; i < n; ++i)
-    for (int p = threadIdx.x; p < hw; p += blockDim.x) {
-      const float gp = gpre[(size_t)i * hw + p];
-      s += c < c16 ? gp * h[((size_t)i * c16 + c) * hw + p] : gp;
-    }
-  sh[threadIdx.x] = s;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) (c < c16 ? dw[c] : db[0]) = sh[0];
-}
-
-__global__ void k_sum(const float* __restrict__ v, long n, float* __restrict__ out) {
-  __shared__ float sh[256];
-  float s = 0.f;
-  for (long i = threadIdx.x; i < n; i += blockDim.x) s += v[i];
-  sh[threadIdx.x] = s;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) *out = sh[0];
-}
-
-__global__ void k_add(float* __restrict__ dst, const float* __restrict__ src, long n) {
-  long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) dst[i] += src[i];
+#pragma unroll 4
+  for (int p = blockIdx.x * kRedPix + threadIdx.x; p < p1; p += 256) s += c < c16 ? gp[p] * hp[p] : gp[p];
+  s = block_sum256(s, sh);
+  if (threadIdx.x == 0) part[((size_t)i * gridDim.x + blockIdx.x) * gridDim.y + c] = s;
 }
 
 // Adam on FP32 master parameters; refreshes the BF16 weight copies
@@ -675,7 +674,7 @@ struct Net {
   long head_w = 0, head_b = 0, head_wbf = 0;
   Mem p, g, m, v, wbf, wmap, wt, part;
   std::vector<Mem> act, gact;  // act[0] input, act[i + 1] output of conv i (post-ReLU)
-  Mem pool[3], gpool[3], gup, gin_tmp, out, sq, gpre, lossv, tgt;
+  Mem pool[3], gpool[3], gup, out, sq, gpre, hsum, tgt, red;
   cudaStream_t s = nullptr;
   long step = 0;
   bool cuda_cores = false;  // FP32 CUDA-core convolutions instead of the tensor cores
@@ -735,11 +734,16 @@ struct Net {
     wmap.alloc(sizeof(int) * nparam);
     UN_CK(cudaMemcpy(wmap.p, map.data(), sizeof(int) * nparam, cudaMemcpyHostToDevice));
     long maxw = 0;
-    size_t maxpart = 0;
+    size_t maxpart = 0, maxred = 0;
     for (const Conv& c : convs) {
       maxw = std::max(maxw, (long)c.cout * (c.ca + c.cb) * 9);
       const size_t tiles = (size_t)nmax * cdiv(lvH(c.level), kCT) * cdiv(lvW(c.level), kCT);
       maxpart = std::max(maxpart, tiles * (size_t)c.cout * (c.ca + c.cb) * 9);
+      // partials of the bias sums and of the second reduction pass
+      const size_t chunks = (size_t)nmax * cdiv((long)lvH(c.level) * lvW(c.level), kRedPix);
+      maxpart = std::max(maxpart, chunks * std::max(c.cout, 18));
+      maxred = std::max(maxred, (size_t)cdiv(tiles, red_per((int)tiles)) * c.cout * (c.ca + c.cb) * 9);
+      maxred = std::max(maxred, (size_t)cdiv(chunks, red_per((int)chunks)) * std::max(c.cout, 18));
     }
     wt.alloc(sizeof(__nv_bfloat16) * maxw);
     part.alloc(sizeof(float) * maxpart);
@@ -757,15 +761,14 @@ struct Net {
       pool[l].alloc(sizeof(float) * n);
       gpool[l].alloc(sizeof(float) * n);
     }
-    // largest input gradient of one conv: 32 channels at full resolution
-    // (u1 and d1a), i.e. 128 channels at a quarter of the pixels
+    // largest gradient of an upsampled input: u1's, 32 channels at full resolution
     gup.alloc(sizeof(float) * (size_t)nmax * 32 * H * W);
-    gin_tmp.alloc(sizeof(float) * (size_t)nmax * 32 * H * W);
     out.alloc(sizeof(float) * (size_t)nmax * H * W);
     sq.alloc(sizeof(float) * (size_t)nmax * H * W);
     gpre.alloc(sizeof(float) * (size_t)nmax * H * W);
     tgt.alloc(sizeof(float) * (size_t)nmax * H * W);
-    lossv.alloc(sizeof(float));
+    hsum.alloc(sizeof(float) * 18);  // the head's 16 weight gradients, its bias's, the summed squared error
+    red.alloc(sizeof(float) * maxred);
     UN_CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
     const char* cc = getenv("MFISTA_UNET_CUDA_CORES");
     cuda_cores = cc && cc[0] == '1';
@@ -807,6 +810,20 @@ struct Net {
     UN_CK(cudaStreamSynchronize(s));
   }
 
+  // partials per group of the first reduction pass
+  static int red_per(int nt) { return nt <= 16 ? nt : std::max(8, (int)ceil(sqrt((double)nt))); }
+
+  // out[i] = sum over the nt partials [nt][len] in `part`, i < len
+  void reduce(int nt, long len, float* out) {
+    const int per = red_per(nt), ng = cdiv(nt, per);
+    k_reduce_partials<<<dim3(cdiv(len, 256), ng), 256, 0, s>>>(part.as<float>(), nt, len, per,
+                                                               ng > 1 ? red.as<float>() : out);
+    UN_LAUNCH();
+    if (ng == 1) return;
+    k_reduce_partials<<<dim3(cdiv(len, 256), 1), 256, 0, s>>>(red.as<float>(), ng, len, ng, out);
+    UN_LAUNCH();
+  }
+
   const __nv_bfloat16* wb(const Conv& c) const { return wbf.as<__nv_bfloat16>() + c.wbf_off; }
 
   const float* src_a_ptr(int i) const {
@@ -837,7 +854,7 @@ struct Net {
   void conv_forward(int i, int n) {
     const Conv& c = convs[i];
     ConvArgs ga{src_a_ptr(i), nullptr, c.ca, c.a_up, src_b_ptr(i), c.cb, wb(c), p.as<float>() + c.b_off,
-                act[i + 1].as<float>(), c.cout, lvH(c.level), lvW(c.level), 1, 0};
+                act[i + 1].as<float>(), c.cout, lvH(c.level), lvW(c.level), 1, nullptr, c.cout};
     conv(ga, n);
   }
 
@@ -862,14 +879,12 @@ struct Net {
                                              gpre.as<float>());
     UN_LAUNCH();
     if (target) {
-      k_sum<<<1, 256, 0, s>>>(sq.as<float>(), n * hw, lossv.as<float>());
+      const int chunks = cdiv(hw, kRedPix);
+      k_head_sums<<<dim3(chunks, 18, n), 256, 0, s>>>(act[17].as<float>(), gpre.as<float>(), sq.as<float>(), 16, (int)hw,
+                                                      part.as<float>());
       UN_LAUNCH();
+      reduce(chunks * n, 18, hsum.as<float>());
     }
-  }
-
-  void add_into(float* dst, const float* src, long cnt) {
-    k_add<<<cdiv(cnt, 256), 256, 0, s>>>(dst, src, cnt);
-    UN_LAUNCH();
   }
 
   // gradient of conv i given gact[i+1] (w.r.t. its post-ReLU output):
@@ -888,34 +903,26 @@ struct Net {
       k_conv3x3_wgrad_tc<<<dim3(ntiles, cdiv(c.cout, 16), cdiv(cin, kCI)), 288, kWgradTcSmem, s>>>(wa);
     UN_LAUNCH();
     const long len = (long)c.cout * cin * 9;
-    k_reduce_partials<<<cdiv(len, 256), 256, 0, s>>>(part.as<float>(), ntiles, len, g.as<float>() + c.w_off);
+    reduce(ntiles, len, g.as<float>() + c.w_off);
+    const int chunks = cdiv((long)Hl * Wl, kRedPix);
+    k_bias_grad<<<dim3(chunks, c.cout, n), 256, 0, s>>>(go, mask, Hl * Wl, part.as<float>());
     UN_LAUNCH();
-    k_bias_grad<<<c.cout, 256, 0, s>>>(go, mask, n, c.cout, Hl * Wl, g.as<float>() + c.b_off);
-    UN_LAUNCH();
+    reduce(chunks * n, c.cout, g.as<float>() + c.b_off);
     if (i == 0) return;  // no gradient for the network input
-    // data: the transposed convolution of the masked gradient
+    // data: the transposed convolution of the masked gradient, straight into
+    // the producers' gradients (it is the first, for all but e1..e3 the only
+    // contribution to each; those get their pool's afterwards)
     k_flip_transpose<<<cdiv(len, 256), 256, 0, s>>>(wb(c), c.cout, cin, wt.as<__nv_bfloat16>());
     UN_LAUNCH();
-    float* gi = c.a_up ? gup.as<float>() : gin_tmp.as<float>();  // w.r.t. the (upsampled) concat input
-    ConvArgs gd{go, mask, c.cout, 0, nullptr, 0, wt.as<__nv_bfloat16>(), nullptr, gi, cin, Hl, Wl, 0, 0};
-    conv(gd, n);
     float* ga_dst = src_a_grad(i);
-    const size_t hw = (size_t)Hl * Wl;
+    float* gb_dst = c.cb ? gact[src_b(i)].as<float>() : nullptr;
+    ConvArgs gd{go, mask, c.cout, 0, nullptr, 0, wt.as<__nv_bfloat16>(), nullptr, c.a_up ? gup.as<float>() : ga_dst, cin,
+                Hl, Wl, 0, gb_dst, c.ca};
+    conv(gd, n);
     if (c.a_up) {  // sum the 2x2 blocks into a's half-resolution gradient
-      const int h = Hl / 2, w = Wl / 2;
-      for (int k = 0; k < n; ++k) {
-        k_upsample_grad<<<cdiv((long)c.ca * h * w, 256), 256, 0, s>>>(gi + (size_t)k * cin * hw, c.ca, h, w,
-                                                                      gin_tmp.as<float>() + (size_t)k * c.ca * h * w);
-        UN_LAUNCH();
-      }
-      add_into(ga_dst, gin_tmp.as<float>(), (long)n * c.ca * h * w);
-      return;
-    }
-    for (int k = 0; k < n; ++k) {  // channels [0, ca) to a's producer, [ca, cin) to b's
-      add_into(ga_dst + (size_t)k * c.ca * hw, gi + (size_t)k * cin * hw, (long)c.ca * hw);
-      if (c.cb)
-        add_into(gact[src_b(i)].as<float>() + (size_t)k * c.cb * hw, gi + ((size_t)k * cin + c.ca) * hw,
-                 (long)c.cb * hw);
+      const long cnt = (long)n * c.ca * (Hl / 2) * (Wl / 2);
+      k_upsample_grad<<<cdiv(cnt, 256), 256, 0, s>>>(gup.as<float>(), n * c.ca, Hl / 2, Wl / 2, ga_dst);
+      UN_LAUNCH();
     }
   }
 
@@ -928,12 +935,8 @@ struct Net {
   }
 
   void backward(int n) {
-    for (size_t i = 1; i + 1 < gact.size(); ++i) UN_CK(cudaMemsetAsync(gact[i].p, 0, gact[i].bytes, s));
-    for (int l = 0; l < 3; ++l) UN_CK(cudaMemsetAsync(gpool[l].p, 0, gpool[l].bytes, s));
-    const long hw = (long)H * W;
-    k_head_wgrad<<<17, 256, 0, s>>>(act[17].as<float>(), gpre.as<float>(), n, 16, (int)hw, g.as<float>() + head_w,
-                                   g.as<float>() + head_b);
-    UN_LAUNCH();
+    // the head's gradients come with the loss (forward); head_b follows head_w
+    UN_CK(cudaMemcpyAsync(g.as<float>() + head_w, hsum.p, sizeof(float) * 17, cudaMemcpyDeviceToDevice, s));
     for (int i = 16; i >= 0; --i) {
       conv_backward(i, n);
       // once the consumer of a pool output is done, route the pool gradient
@@ -951,7 +954,7 @@ struct Net {
 
   float loss(int n) {
     float sum = 0.f;
-    UN_CK(cudaMemcpyAsync(&sum, lossv.p, sizeof(float), cudaMemcpyDeviceToHost, s));
+    UN_CK(cudaMemcpyAsync(&sum, hsum.as<float>() + 17, sizeof(float), cudaMemcpyDeviceToHost, s));
     UN_CK(cudaStreamSynchronize(s));
     return sum / (float)((long)n * H * W);
   }
