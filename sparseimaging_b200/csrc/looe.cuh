@@ -12,255 +12,287 @@
 // and reports a Hessian that is not positive definite (dposv info > 0).
 //
 // Here, all in FP64 on one stream, per solution:
-//   Z = A_S gathered (M x n_s, column-major, coalesced column copies);
-//   H = Z^T Z by a tiled FP64 GEMM (lower tiles only);
-//   blocked right-looking Cholesky H = L L^T (64-wide panels: the diagonal
-//   block factored in one CTA's shared memory, the panel below by one
-//   thread per row, the trailing matrix by the GEMM);
-//   Z <- Z L^-T block by block in the same loop, so that row i of Z ends as
+//   H = A_S^T A_S, lower tiles, by matrix products over the active columns
+//   where they lie (dgemm_mma.cuh; K split so that the tiles fill the GPU);
+//   blocked right-looking Cholesky H = L L^T in 64-wide panels: the diagonal
+//   block and the inverse W_k of its factor in one CTA, the panel below as a
+//   product with W_k^T, the trailing matrix by products;
+//   Y = A_S L^-T by rows: a CTA takes 64 rows through all panels,
+//   Y_k = (Z_k - sum_{j<k} Y_j L_kj^T) W_k^T, so that row i of Y is
 //   (L^-1 a_i)^T and d_i = |row i|^2 (one triangular solve instead of the
 //   reference's two: the same quantity, other rounding);
 //   the residual, the t_i and the two sums with fixed-order reductions.
 // A non-positive pivot sets an info word that every later kernel of the
 // solution checks at entry.
+//
+// With one thread per row for the triangular solves (53 % of the time), a
+// barrier per pivot, column and update in the diagonal block (14 %) and scalar
+// 4 x 4 sums in the products (29 %, 13 TFLOP/s), a solution of 1261 active
+// pixels, M = 8000, took 9.9 ms on B200.
 #pragma once
 
+#include "dgemm_mma.cuh"
 #include "solver.cuh"
 
 namespace mf {
 namespace looe {
 
-constexpr int kPanel = 64;  // Cholesky / triangular-solve block width
-constexpr int kGT = 64;     // GEMM tile (rows and columns)
-constexpr int kGK = 16;     // GEMM k step
+constexpr int kPanel = 64;  // Cholesky / triangular-solve block width (the products' tile)
+constexpr int kSplitR = 16;  // column ranges of the residual's partial sums
+static_assert(kPanel == dg::kT, "panels are tiles of the products");
 
-// 8-byte asynchronous global -> shared copy; src_bytes 0 writes zeros
-__device__ __forceinline__ void cp_async8_zfill(void* smem_dst, const void* gmem_src, unsigned int src_bytes) {
-  const unsigned int d = (unsigned int)__cvta_generic_to_shared(smem_dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(gmem_src), "r"(src_bytes) : "memory");
+// tile (ti, tj), ti >= tj, of the e-th lower tile in row order
+__device__ __forceinline__ void lower_tile(int e, int& ti, int& tj) {
+  ti = (int)((sqrtf(8.f * (float)e + 1.f) - 1.f) * 0.5f);
+  while ((ti + 1) * (ti + 2) / 2 <= e) ++ti;
+  while (ti * (ti + 1) / 2 > e) --ti;
+  tj = e - ti * (ti + 1) / 2;
 }
 
-// C (m x n, ldc) = alpha op(A) op(B) + beta C, column-major; op(A)(i,p) is
-// A[p + i lda] when TA, else A[i + p lda]; op(B)(p,j) is B[j + p ldb] when
-// TB, else B[p + j ldb].  lower: tiles strictly above the diagonal are
-// skipped (the Cholesky reads the lower triangle only).  256 threads, a
-// 64 x 64 tile per CTA, 4 x 4 outputs per thread at rows tx + 16r and
-// columns ty + 16c.  The k steps are double-buffered: the copies of step
-// p + 1 (cp.async, element by element, zeros outside the matrices) are in
-// flight while step p is multiplied.  With beta != 0 the C tile is copied
-// into shared memory at the start, behind the k steps (the trailing
-// updates of the factorisation are rank-64: four k steps only).
-constexpr int kGLd = kGT + 1;  // shared row length (padded)
-constexpr size_t kGemmSmem = sizeof(double) * (2 * 2 * kGK * kGLd + kGT * kGT);
-template <bool TA, bool TB>
-__global__ void __launch_bounds__(256) k_looe_gemm(int m, int n, int k, double alpha, const double* __restrict__ A,
-                                                   int lda, const double* __restrict__ B, int ldb, double beta,
-                                                   double* __restrict__ C, int ldc, int lower,
-                                                   const int* __restrict__ info) {
-  if (info && *info) return;
-  const int i0 = blockIdx.x * kGT, j0 = blockIdx.y * kGT;
-  if (lower && i0 + kGT - 1 < j0) return;
-  extern __shared__ __align__(16) double gemm_smem[];
-  auto As = reinterpret_cast<double(*)[kGK][kGLd]>(gemm_smem);
-  auto Bs = reinterpret_cast<double(*)[kGK][kGLd]>(gemm_smem + 2 * kGK * kGLd);
-  double* Cs = gemm_smem + 4 * kGK * kGLd;  // [64 columns][64 rows]
+// lower tiles of A_S^T A_S over the K range of split blockIdx.y: part
+// [split][n_s x n_s]; grid (lower tiles, splits)
+__global__ void __launch_bounds__(128, 3) k_looe_gram(const double* __restrict__ A, int M, const int* __restrict__ S,
+                                                      int ns, int kchunk, double* __restrict__ part) {
+  extern __shared__ __align__(16) double looe_smem[];
+  int ti, tj;
+  lower_tile(blockIdx.x, ti, tj);
+  const bool vec = (M & 1) == 0;
+  dg::Operand<true> X(A, M, ti * kPanel, ns, vec, S), Y(A, M, tj * kPanel, ns, vec, S);
+  dg::Acc acc;
+  dg::clear(acc);
+  const int k0 = blockIdx.y * kchunk;
+  dg::tile_product_nb<8>(X, Y, k0, min(M, k0 + kchunk), looe_smem, acc);
+  double* H = part + (size_t)blockIdx.y * ns * ns;
+  dg::each(acc, [&](int r, int c, double v) {
+    const int i = ti * kPanel + r, j = tj * kPanel + c;
+    if (i < ns && j < ns) H[(size_t)i + (size_t)j * ns] = v;
+  });
+}
+
+// H = sum of the splits (in order), lower triangle, plus lambda_tsv d2(S_j) on
+// the diagonal (TSV form); H may be split 0 itself
+__global__ void k_looe_gram_sum(const double* __restrict__ part, int nsplit, double* __restrict__ H,
+                                const int* __restrict__ S, int ns, int nx, double lam) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y;
+  if (i >= ns || i < j) return;
+  const size_t e = (size_t)i + (size_t)j * ns;
+  double h = 0.0;
+  for (int q = 0; q < nsplit; ++q) h += part[(size_t)q * ns * ns + e];
+  if (i == j && lam != 0.0) {
+    const int pix = S[j], r = pix % nx, c = pix / nx;
+    const bool ri = r > 0 && r < nx - 1, ci = c > 0 && c < nx - 1;
+    h += lam * (ri ? (ci ? 8.0 : 6.0) : (ci ? 6.0 : 4.0));
+  }
+  H[e] = h;
+}
+
+// partial sums of (A x)_i over a range of the active columns: part[split][M]
+__global__ void k_looe_ax(const double* __restrict__ A, int M, const int* __restrict__ S, const double* __restrict__ xs,
+                          int ns, double* __restrict__ part) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= M) return;
+  const int per = (ns + kSplitR - 1) / kSplitR;
+  const int j0 = blockIdx.y * per, j1 = min(ns, j0 + per);
+  double s = 0.0;
+#pragma unroll 8
+  for (int j = j0; j < j1; ++j) s = fma(A[(size_t)S[j] * M + i], xs[j], s);
+  part[(size_t)blockIdx.y * M + i] = s;
+}
+
+// Cholesky of the nb x nb diagonal block at (k0, k0) (lower triangle in and
+// out) and the inverse of the factor, W [64][64] (zeros above its diagonal and
+// beyond nb); info = k0 + j + 1 at a pivot that is not > 0.  One CTA, the
+// block and the inverse in registers (a thread holds rows tx + 16 r and
+// columns ty + 16 c of both); a step broadcasts pivot column and inverse row
+// through shared memory, eliminates without square roots (L = U D^1/2) and
+// costs one barrier.
+__global__ void __launch_bounds__(256) k_looe_chol_diag(double* __restrict__ H, int ld, int k0, int nb,
+                                                        double* __restrict__ W, int* __restrict__ info) {
+  if (*info) return;
+  __shared__ double s_col[2][kPanel], s_row[2][kPanel], s_d[kPanel];
   const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
-  if (beta != 0.0) {
-    for (int e = t; e < kGT * kGT; e += 256) {
-      const int i = e & (kGT - 1), j = e >> 6;
-      const int gi = i0 + i, gj = j0 + j;
-      const bool v = gi < m && gj < n;
-      cp_async8_zfill(Cs + e, v ? C + (size_t)gi + (size_t)gj * ldc : C, v ? 8u : 0u);
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  }
-  auto stage = [&](int buf, int p0) {
-#pragma unroll
-    for (int q = 0; q < (kGT * kGK) / 256; ++q) {
-      const int e = t + 256 * q;
-      int i, p;
-      if (TA) {
-        i = e / kGK;
-        p = e % kGK;
-      } else {
-        i = e % kGT;
-        p = e / kGT;
-      }
-      const int gi = i0 + i, gp = p0 + p;
-      const bool va = gi < m && gp < k;
-      cp_async8_zfill(&As[buf][p][i], va ? (TA ? A + (size_t)gp + (size_t)gi * lda : A + (size_t)gi + (size_t)gp * lda) : A,
-                      va ? 8u : 0u);
-      int j;
-      if (TB) {
-        j = e % kGT;
-        p = e / kGT;
-      } else {
-        j = e / kGK;
-        p = e % kGK;
-      }
-      const int gj = j0 + j, gq = p0 + p;
-      const bool vb = gj < n && gq < k;
-      cp_async8_zfill(&Bs[buf][p][j], vb ? (TB ? B + (size_t)gj + (size_t)gq * ldb : B + (size_t)gq + (size_t)gj * ldb) : B,
-                      vb ? 8u : 0u);
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  double acc[4][4];
-#pragma unroll
-  for (int r = 0; r < 4; ++r)
-#pragma unroll
-    for (int c = 0; c < 4; ++c) acc[r][c] = 0.0;
-  const int nk = (k + kGK - 1) / kGK;
-  // (the C group, when there is one, is older than every step's group, so
-  // the waits below cover it too)
-  if (nk > 0) stage(0, 0);
-  for (int kt = 0; kt < nk; ++kt) {
-    if (kt + 1 < nk) stage((kt + 1) & 1, (kt + 1) * kGK);
-    else asm volatile("cp.async.commit_group;" ::: "memory");  // keeps one group per step
-    asm volatile("cp.async.wait_group 1;" ::: "memory");       // step kt has landed (this thread)
-    __syncthreads();                                           // and everyone's
-    const int bf = kt & 1;
-#pragma unroll
-    for (int p = 0; p < kGK; ++p) {
-      double a[4], b[4];
-#pragma unroll
-      for (int r = 0; r < 4; ++r) a[r] = As[bf][p][tx + 16 * r];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) b[c] = Bs[bf][p][ty + 16 * c];
-#pragma unroll
-      for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) acc[r][c] = fma(a[r], b[c], acc[r][c]);
-    }
-    __syncthreads();  // buffer bf is refilled by the copies issued next step
-  }
-  if (beta != 0.0) {
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();
-  }
+  double* blk = H + (size_t)k0 + (size_t)k0 * ld;
+  double a[4][4], w[4][4];
 #pragma unroll
   for (int r = 0; r < 4; ++r)
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-      const int li = tx + 16 * r, lj = ty + 16 * c;
-      const int gi = i0 + li, gj = j0 + lj;
-      if (gi < m && gj < n)
-        C[(size_t)gi + (size_t)gj * ldc] = alpha * acc[r][c] + (beta != 0.0 ? beta * Cs[lj * kGT + li] : 0.0);
+      const int i = tx + 16 * r, j = ty + 16 * c;
+      const double one = i == j ? 1.0 : 0.0;
+      a[r][c] = (i < nb && j < nb) ? (i >= j ? blk[(size_t)i + (size_t)j * ld] : blk[(size_t)j + (size_t)i * ld]) : one;
+      w[r][c] = one;
     }
-}
-
-// Z[:, j] = A[:, S_j] for the n_s active columns (M x n_s, column-major):
-// one CTA per column
-__global__ void k_looe_gather(const double* __restrict__ A, int M, const int* __restrict__ S,
-                              double* __restrict__ Z) {
-  const int j = blockIdx.x;
-  const double* src = A + (size_t)S[j] * M;
-  double* dst = Z + (size_t)j * M;
-  for (int i = threadIdx.x; i < M; i += blockDim.x) dst[i] = src[i];
-}
-
-// r = y - A x over the active columns (x is zero elsewhere), column order
-__global__ void k_looe_resid(const double* __restrict__ A, int M, const double* __restrict__ y,
-                             const int* __restrict__ S, const double* __restrict__ xs, int ns,
-                             double* __restrict__ r) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= M) return;
-  double s = 0.0;
-  for (int j = 0; j < ns; ++j) s = fma(A[(size_t)S[j] * M + i], xs[j], s);
-  r[i] = y[i] - s;
-}
-
-// H_jj += lambda_tsv d2(S_j) (TSV form)
-__global__ void k_looe_tsv_diag(double* __restrict__ H, int ld, const int* __restrict__ S, int ns, int nx,
-                                double lam) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= ns) return;
-  const int pix = S[j], r = pix % nx, c = pix / nx;
-  const bool ri = r > 0 && r < nx - 1, ci = c > 0 && c < nx - 1;
-  const double d2 = ri ? (ci ? 8.0 : 6.0) : (ci ? 6.0 : 4.0);
-  H[(size_t)j + (size_t)j * ld] += lam * d2;
-}
-
-// Cholesky of the nb x nb diagonal block at (k0, k0) in shared memory
-// (lower triangle in and out); info = k0 + j + 1 at a pivot that is not > 0
-__global__ void __launch_bounds__(256) k_looe_chol_diag(double* __restrict__ H, int ld, int k0, int nb,
-                                                        int* __restrict__ info) {
-  if (*info) return;
-  __shared__ double a[kPanel][kPanel + 1];
-  __shared__ int bad;
-  const int t = threadIdx.x;
-  double* blk = H + (size_t)k0 + (size_t)k0 * ld;
-  for (int e = t; e < nb * nb; e += blockDim.x) {
-    const int i = e % nb, j = e / nb;
-    a[i][j] = i >= j ? blk[(size_t)i + (size_t)j * ld] : 0.0;
-  }
-  if (t == 0) bad = 0;
+#pragma unroll
+  for (int jc = 0; jc < 4; ++jc)
+    for (int jj = 0; jj < 16; ++jj) {
+      const int j = 16 * jc + jj, buf = j & 1;
+      if (ty == jj) {
+#pragma unroll
+        for (int r = 0; r < 4; ++r) s_col[buf][tx + 16 * r] = a[r][jc];
+      }
+      if (tx == jj) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) s_row[buf][ty + 16 * c] = w[jc][c];
+      }
+      __syncthreads();
+      const double d = s_col[buf][j];
+      if (!(d > 0.0)) {  // the same for every thread
+        if (t == 0) *info = k0 + j + 1;
+        return;
+      }
+      if (t == 0) s_d[j] = d;
+      const double rd = 1.0 / d;
+      double cj[4], wj[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const int k = ty + 16 * c;
+        cj[c] = k > j ? s_col[buf][k] : 0.0;
+        wj[c] = s_row[buf][k];
+      }
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const int i = tx + 16 * r;
+        const double l = i > j ? s_col[buf][i] * rd : 0.0;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          a[r][c] = fma(-l, cj[c], a[r][c]);
+          w[r][c] = fma(-l, wj[c], w[r][c]);
+        }
+      }
+    }
   __syncthreads();
-  for (int j = 0; j < nb; ++j) {
-    if (t == 0) {
-      const double d = a[j][j];
-      if (d > 0.0) a[j][j] = sqrt(d);
-      else bad = j + 1;
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int i = tx + 16 * r, j = ty + 16 * c;
+      const bool in = i < nb && j < nb && i >= j;
+      if (in) blk[(size_t)i + (size_t)j * ld] = i == j ? sqrt(s_d[j]) : a[r][c] / sqrt(s_d[j]);
+      W[i * kPanel + j] = in ? w[r][c] / sqrt(s_d[i]) : 0.0;
     }
-    __syncthreads();
-    if (bad) {
-      if (t == 0) *info = k0 + bad;
-      return;
-    }
-    const double piv = a[j][j];
-    for (int i = j + 1 + t; i < nb; i += blockDim.x) a[i][j] /= piv;
-    __syncthreads();
-    const int w = nb - j - 1;
-    for (int e = t; e < w * w; e += blockDim.x) {
-      const int ii = j + 1 + e % w, kk = j + 1 + e / w;
-      if (ii >= kk) a[ii][kk] -= a[ii][j] * a[kk][j];
-    }
-    __syncthreads();
-  }
-  for (int e = t; e < nb * nb; e += blockDim.x) {
-    const int i = e % nb, j = e / nb;
-    if (i >= j) blk[(size_t)i + (size_t)j * ld] = a[i][j];
-  }
 }
 
-// rows [r0, r1) of X (columns 0..nb-1, leading dimension ldx) := X L^-T,
-// L the factored nb x nb diagonal block at Ld (ldl): one thread per row,
-// forward substitution x_j = (x_j - sum_{p<j} x_p L_jp) / L_jj
-__global__ void __launch_bounds__(256) k_looe_rowsolve(double* __restrict__ X, int ldx, int r0, int r1,
-                                                       const double* __restrict__ Ld, int ldl, int nb,
+// the panel below a factored diagonal block: H[k1 + i][k0 ..] := H[..] W^T, in
+// place (a CTA reads its 64 rows whole before it writes them)
+__global__ void __launch_bounds__(128, 3) k_looe_panel(double* __restrict__ H, int ld, int k0, int nb,
+                                                       const double* __restrict__ W, const int* __restrict__ info) {
+  if (*info) return;
+  extern __shared__ __align__(16) double looe_smem[];
+  const int i0 = blockIdx.x * kPanel, rows = ld - (k0 + nb);
+  double* P = H + (size_t)(k0 + nb) + (size_t)k0 * ld;
+  dg::Operand<false> X(P, ld, i0, rows, (ld & 1) == 0 && ((k0 + nb) & 1) == 0);
+  dg::Operand<true> Y(W, kPanel, 0, nb, true);
+  dg::Acc acc;
+  dg::clear(acc);
+  dg::tile_product_nb<8>(X, Y, 0, nb, looe_smem, acc);
+  dg::each(acc, [&](int r, int c, double v) {
+    if (i0 + r < rows && c < nb) P[(size_t)(i0 + r) + (size_t)c * ld] = v;
+  });
+}
+
+// trailing matrix H[k1.., k1..] -= P P^T, lower tiles, P the panel below the
+// block at k0; grid: the lower tiles
+__global__ void __launch_bounds__(128, 3) k_looe_trail(double* __restrict__ H, int ld, int k0, int nb,
                                                        const int* __restrict__ info) {
   if (*info) return;
-  __shared__ double L[kPanel][kPanel + 1];
-  for (int e = threadIdx.x; e < nb * nb; e += blockDim.x) {
-    const int i = e % nb, j = e / nb;
-    L[i][j] = i >= j ? Ld[(size_t)i + (size_t)j * ldl] : 0.0;
+  extern __shared__ __align__(16) double looe_smem[];
+  int ti, tj;
+  lower_tile(blockIdx.x, ti, tj);
+  const int k1 = k0 + nb, rows = ld - k1;
+  const double* P = H + (size_t)k1 + (size_t)k0 * ld;
+  const bool vec = (ld & 1) == 0 && (k1 & 1) == 0;
+  dg::Operand<false> X(P, ld, ti * kPanel, rows, vec), Y(P, ld, tj * kPanel, rows, vec);
+  dg::Acc acc;
+  dg::clear(acc);
+  dg::tile_product_nb<8>(X, Y, 0, nb, looe_smem, acc);
+  double* C = H + (size_t)k1 + (size_t)k1 * ld;
+  dg::each(acc, [&](int r, int c, double v) {
+    const int i = ti * kPanel + r, j = tj * kPanel + c;
+    if (i < rows && j < rows) C[(size_t)i + (size_t)j * ld] -= v;
+  });
+}
+
+// Y = A_S L^-T and the leverages d_i = |Y_i|^2 of 64 rows per CTA, panel by
+// panel (each needs the CTA's own earlier panels only).  W: [panel][64][64].
+constexpr int kRowLd = 68;  // row stride of the staged panel and of W
+constexpr size_t kRowsSmem = dg::kSmem + sizeof(double) * kPanel * kRowLd;
+static_assert(sizeof(double) * kPanel * kRowLd <= dg::kSmem, "a panel fits the products' stages");
+__global__ void __launch_bounds__(128) k_looe_rows(const double* __restrict__ A, int M, const int* __restrict__ S, int ns,
+                                                   const double* __restrict__ H, const double* __restrict__ Wall,
+                                                   double* __restrict__ Y, double* __restrict__ dlev,
+                                                   const int* __restrict__ info) {
+  if (*info) return;
+  extern __shared__ __align__(16) double looe_smem[];
+  double* s_t = looe_smem;                                  // [64][68], over the stages
+  double* s_w = looe_smem + dg::kSmem / sizeof(double);     // [64][68]
+  const int i0 = blockIdx.x * kPanel;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  double d[2] = {0.0, 0.0};
+  const bool vy = (M & 1) == 0, vh = (ns & 1) == 0;
+  for (int k0 = 0; k0 < ns; k0 += kPanel) {
+    const int nb = min(kPanel, ns - k0);
+    const double* W = Wall + (size_t)(k0 / kPanel) * kPanel * kPanel;
+    for (int e = threadIdx.x; e < kPanel * kPanel / 2; e += 128)
+      dg::copy2(s_w + (e >> 5) * kRowLd + 2 * (e & 31), W + 2 * e, 2, true);
+    cp_async_commit();
+    dg::Acc acc;
+    dg::clear(acc);
+    dg::Operand<false> X(Y, M, i0, M, vy), L(H, ns, k0, ns, vh);
+    dg::tile_product_nb<8>(X, L, 0, k0, looe_smem, acc);
+    // the right-hand side into shared memory
+    dg::each(acc, [&](int r, int c, double v) {
+      s_t[r * kRowLd + c] = (i0 + r < M && c < nb) ? A[(size_t)S[k0 + c] * M + i0 + r] - v : 0.0;
+    });
+    cp_async_wait<0>();
+    __syncthreads();
+    dg::clear(acc);
+#pragma unroll 2
+    for (int kk = 0; kk < kPanel; kk += 4) {
+      double a[2], b[8];
+#pragma unroll
+      for (int m = 0; m < 2; ++m) a[m] = s_t[(16 * warp + 8 * m + g) * kRowLd + kk + t];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) b[j] = s_w[(8 * j + g) * kRowLd + kk + t];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        dmma_884(acc[0][j], a[0], b[j]);
+        dmma_884(acc[1][j], a[1], b[j]);
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int i = i0 + 16 * warp + 8 * m + g, c = 8 * j + 2 * t + h;
+          const double v = acc[m][j][h];
+          d[m] = fma(v, v, d[m]);  // zero beyond nb and M
+          if (i < M && c < nb) Y[(size_t)i + (size_t)(k0 + c) * M] = v;
+        }
+    __syncthreads();  // Y_k is read, and s_t and s_w are written, by the next panel
   }
-  __syncthreads();
-  const int i = r0 + blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= r1) return;
-  double* row = X + i;
-  for (int j = 0; j < nb; ++j) {
-    double s = row[(size_t)j * ldx];
-    for (int p = 0; p < j; ++p) s -= row[(size_t)p * ldx] * L[j][p];
-    row[(size_t)j * ldx] = s / L[j][j];
+#pragma unroll
+  for (int m = 0; m < 2; ++m) {
+    d[m] += __shfl_xor_sync(0xffffffffu, d[m], 1);
+    d[m] += __shfl_xor_sync(0xffffffffu, d[m], 2);
+    const int i = i0 + 16 * warp + 8 * m + g;
+    if (t == 0 && i < M) dlev[i] = d[m];
   }
 }
 
-// per row i: d_i = |Z_i|^2 (columns in order), t = r_i / (1 - d_i),
-// s = t^2 / 2; per-CTA partial sums of s and s^2
-__global__ void __launch_bounds__(256) k_looe_terms(const double* __restrict__ Z, int M, int ns,
-                                                    const double* __restrict__ r, double* __restrict__ part,
+// per row i: t = (y - A x)_i / (1 - d_i), s = t^2 / 2; per-CTA partial sums of
+// s and s^2
+__global__ void __launch_bounds__(256) k_looe_terms(const double* __restrict__ y, const double* __restrict__ ax, int nax,
+                                                    const double* __restrict__ dlev, int M, double* __restrict__ part,
                                                     const int* __restrict__ info) {
   __shared__ double sh[2][256];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   double s = 0.0, s2 = 0.0;
   if (!*info && i < M) {
-    double d = 0.0;
-    for (int j = 0; j < ns; ++j) {
-      const double z = Z[(size_t)j * M + i];
-      d = fma(z, z, d);
-    }
-    const double tt = r[i] / (1.0 - d);
+    double v = 0.0;
+    for (int q = 0; q < nax; ++q) v += ax[(size_t)q * M + i];
+    const double tt = (y[i] - v) / (1.0 - (nax > 0 ? dlev[i] : 0.0));
     s = tt * tt / 2;
     s2 = s * s;
   }
@@ -304,36 +336,53 @@ __global__ void k_looe_final(const double* __restrict__ part, int nblk, int M, c
 
 // Host driver: LOOE of B solutions X [B][N] of the DFT problem (y [M], A
 // column-major M x N); lambda_tsv per solution (null: 0).  Kernels per
-// solution: 5 (+1 TSV) + ceil(n_s/64) x (up to 5).
+// solution: 6 + 3 ceil(n_s / 64).
 struct Looe {
   int M, N, NX;
   cudaStream_t s = nullptr;
-  DevMem d_A, d_y, d_S, d_xs, d_r, d_Z, d_H, d_part, d_info, d_out;
+  DevMem d_A, d_y, d_S, d_xs, d_ax, d_Y, d_H, d_Hs, d_W, d_lev, d_part, d_info, d_out;
+  int sms = 148;
 
   Looe(const double* y, const double* A, int M_, int N_, int NX_) : M(M_), N(N_), NX(NX_) {
     MF_CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    int dev = 0;
+    MF_CK(cudaGetDevice(&dev));
+    MF_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     d_A.upload(A, (size_t)M * N);
     d_y.upload(y, (size_t)M);
-    d_r.alloc(sizeof(double) * M);
+    d_S.alloc(sizeof(int) * N);
+    d_xs.alloc(sizeof(double) * N);
+    d_ax.alloc(sizeof(double) * kSplitR * (size_t)M);
+    d_lev.alloc(sizeof(double) * M);
     d_part.alloc(sizeof(double) * 2 * (size_t)cdiv(M, 256));
     d_info.alloc(sizeof(int));
     d_out.alloc(sizeof(double) * 3);
-    set_smem(k_looe_gemm<false, false>, kGemmSmem);
-    set_smem(k_looe_gemm<false, true>, kGemmSmem);
-    set_smem(k_looe_gemm<true, false>, kGemmSmem);
-    set_smem(k_looe_gemm<true, true>, kGemmSmem);
+    set_smem(k_looe_gram, dg::kSmem);
+    set_smem(k_looe_panel, dg::kSmem);
+    set_smem(k_looe_trail, dg::kSmem);
+    set_smem(k_looe_rows, kRowsSmem);
   }
   ~Looe() {
     if (s) cudaStreamDestroy(s);
   }
 
-  template <bool TA, bool TB>
-  void gemm(int m, int n, int k, double alpha, const double* A, int lda, const double* B, int ldb, double beta,
-            double* C, int ldc, int lower) {
-    if (m <= 0 || n <= 0) return;
-    k_looe_gemm<TA, TB><<<dim3(cdiv(m, kGT), cdiv(n, kGT)), 256, kGemmSmem, s>>>(m, n, k, alpha, A, lda, B, ldb, beta,
-                                                                                  C, ldc, lower, d_info.as<int>());
-    MF_LAUNCH_CK();
+  static void grow(DevMem& d, size_t bytes) {
+    if (d.bytes < bytes) d.alloc(bytes);
+  }
+
+  // K splits of the lower tiles: the fewest (at most 4) whose CTAs spread over
+  // the SMs with the least idle time in the last round
+  int gram_splits(int tiles) const {
+    int best = 1;
+    double load = 0.0;
+    for (int q = 1; q <= 4 && M / q >= 512; ++q) {
+      const double x = (double)tiles * q / sms, l = x / ceil(x);
+      if (l > load + 0.05) {
+        load = l;
+        best = q;
+      }
+    }
+    return best;
   }
 
   // (looe_m, looe_std, positive) of one solution x [N]
@@ -346,49 +395,45 @@ struct Looe {
         xs.push_back(x[j]);
       }
     const int ns = (int)S.size();
-    if (ns > 0) {
-      d_S.upload(S.data(), S.size());
-      d_xs.upload(xs.data(), xs.size());
-      if (d_Z.bytes < sizeof(double) * (size_t)M * ns) d_Z.alloc(sizeof(double) * (size_t)M * ns);
-      if (d_H.bytes < sizeof(double) * (size_t)ns * ns) d_H.alloc(sizeof(double) * (size_t)ns * ns);
-    }
-    MF_CK(cudaMemsetAsync(d_info.p, 0, sizeof(int), s));
-    double* Z = d_Z.as<double>();
-    double* H = d_H.as<double>();
+    const int np = cdiv(ns, kPanel), tiles = np * (np + 1) / 2;
     const int* info = d_info.as<int>();
-    k_looe_resid<<<cdiv(M, 256), 256, 0, s>>>(d_A.as<double>(), M, d_y.as<double>(), d_S.as<int>(),
-                                                d_xs.as<double>(), ns, d_r.as<double>());
-    MF_LAUNCH_CK();
+    MF_CK(cudaMemsetAsync(d_info.p, 0, sizeof(int), s));
     if (ns > 0) {
-      k_looe_gather<<<ns, 256, 0, s>>>(d_A.as<double>(), M, d_S.as<int>(), Z);
+      const int nsplit = gram_splits(tiles);
+      const int kchunk = cdiv(cdiv(M, nsplit), dg::kStep) * dg::kStep;
+      MF_CK(cudaMemcpyAsync(d_S.p, S.data(), sizeof(int) * ns, cudaMemcpyHostToDevice, s));
+      MF_CK(cudaMemcpyAsync(d_xs.p, xs.data(), sizeof(double) * ns, cudaMemcpyHostToDevice, s));
+      grow(d_Y, sizeof(double) * (size_t)M * ns);
+      grow(d_H, sizeof(double) * (size_t)ns * ns);
+      grow(d_Hs, sizeof(double) * (size_t)nsplit * ns * ns);
+      grow(d_W, sizeof(double) * (size_t)np * kPanel * kPanel);
+      double* H = d_H.as<double>();
+      const double* A = d_A.as<double>();
+      k_looe_ax<<<dim3(cdiv(M, 256), kSplitR), 256, 0, s>>>(A, M, d_S.as<int>(), d_xs.as<double>(), ns, d_ax.as<double>());
       MF_LAUNCH_CK();
-      gemm<true, false>(ns, ns, M, 1.0, Z, M, Z, M, 0.0, H, ns, 1);  // H = Z^T Z
-      if (lam_tsv != 0.0) {
-        k_looe_tsv_diag<<<cdiv(ns, 256), 256, 0, s>>>(H, ns, d_S.as<int>(), ns, NX, lam_tsv);
-        MF_LAUNCH_CK();
-      }
+      k_looe_gram<<<dim3(tiles, nsplit), 128, dg::kSmem, s>>>(A, M, d_S.as<int>(), ns, kchunk, d_Hs.as<double>());
+      MF_LAUNCH_CK();
+      k_looe_gram_sum<<<dim3(cdiv(ns, 256), ns), 256, 0, s>>>(d_Hs.as<double>(), nsplit, H, d_S.as<int>(), ns, NX, lam_tsv);
+      MF_LAUNCH_CK();
       for (int k0 = 0; k0 < ns; k0 += kPanel) {
-        const int nb = std::min(kPanel, ns - k0), k1 = k0 + nb, rem = ns - k1;
-        const double* Ld = H + k0 + (size_t)k0 * ns;
-        k_looe_chol_diag<<<1, 256, 0, s>>>(H, ns, k0, nb, d_info.as<int>());
+        const int nb = std::min(kPanel, ns - k0), nt = cdiv(ns - k0 - nb, kPanel);
+        double* W = d_W.as<double>() + (size_t)(k0 / kPanel) * kPanel * kPanel;
+        k_looe_chol_diag<<<1, 256, 0, s>>>(H, ns, k0, nb, W, d_info.as<int>());
         MF_LAUNCH_CK();
-        if (rem > 0) {
-          k_looe_rowsolve<<<cdiv(rem, 256), 256, 0, s>>>(H + (size_t)k0 * ns, ns, k1, ns, Ld, ns, nb, info);
+        if (nt > 0) {
+          k_looe_panel<<<nt, 128, dg::kSmem, s>>>(H, ns, k0, nb, W, info);
           MF_LAUNCH_CK();
-          // trailing H22 -= L21 L21^T (lower tiles)
-          gemm<false, true>(rem, rem, nb, -1.0, H + k1 + (size_t)k0 * ns, ns, H + k1 + (size_t)k0 * ns, ns, 1.0,
-                            H + k1 + (size_t)k1 * ns, ns, 1);
+          k_looe_trail<<<nt * (nt + 1) / 2, 128, dg::kSmem, s>>>(H, ns, k0, nb, info);
+          MF_LAUNCH_CK();
         }
-        // Z[:, k0:k1] := Z[:, k0:k1] L_kk^-T, then Z[:, k1:] -= Z[:, k0:k1] L21^T
-        k_looe_rowsolve<<<cdiv(M, 256), 256, 0, s>>>(Z + (size_t)k0 * M, M, 0, M, Ld, ns, nb, info);
-        MF_LAUNCH_CK();
-        if (rem > 0)
-          gemm<false, true>(M, rem, nb, -1.0, Z + (size_t)k0 * M, M, H + k1 + (size_t)k0 * ns, ns, 1.0,
-                            Z + (size_t)k1 * M, M, 0);
       }
+      k_looe_rows<<<cdiv(M, kPanel), 128, kRowsSmem, s>>>(A, M, d_S.as<int>(), ns, H, d_W.as<double>(), d_Y.as<double>(),
+                                                         d_lev.as<double>(), info);
+      MF_LAUNCH_CK();
     }
     const int nblk = cdiv(M, 256);
-    k_looe_terms<<<nblk, 256, 0, s>>>(Z, M, ns, d_r.as<double>(), d_part.as<double>(), info);
+    k_looe_terms<<<nblk, 256, 0, s>>>(d_y.as<double>(), d_ax.as<double>(), ns > 0 ? kSplitR : 0, d_lev.as<double>(), M,
+                                      d_part.as<double>(), info);
     MF_LAUNCH_CK();
     k_looe_final<<<1, 32, 0, s>>>(d_part.as<double>(), nblk, M, info, d_out.as<double>());
     MF_LAUNCH_CK();
