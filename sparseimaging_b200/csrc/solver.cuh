@@ -1230,7 +1230,7 @@ struct TcGemm {
 };
 
 // ---------------------------------------------------------------------------
-// DFT operator: FP64 (GEMV for one problem, register-blocked GEMM for a
+// DFT operator: FP64 (GEMV for one problem, matrix products for a
 // batch), or the split-BF16 tensor-core GEMMs with FP64 defect correction
 // ---------------------------------------------------------------------------
 struct DftOp : Op {
@@ -1263,10 +1263,12 @@ struct DftOp : Op {
     g.nchunk = cdiv(N, g.chunk);
     gemm = B > 1 || tcm;  // the anchors of the split-BF16 form use the FP64 GEMMs
     if (gemm) {  // split-K so that the tiles fill the GPU
-      g.chunk = std::max(kGK, cdiv(cdiv(N, 4), kGK) * kGK);
-      g.nchunk = cdiv(N, g.chunk);
-      mchunk = std::max(kGK, cdiv(cdiv(M, 8), kGK) * kGK);
-      nmchunk = cdiv(M, mchunk);
+      g.chunk = k_chunk(M, N);
+      g.nchunk = std::max(1, cdiv(N, g.chunk));
+      mchunk = k_chunk(N, M);
+      nmchunk = std::max(1, cdiv(M, mchunk));
+      set_smem(k_dft_az_gemm, dg::kSmem);
+      set_smem(k_dft_atr_gemm, dg::kSmem);
       d_atr.alloc(sizeof(double) * (size_t)B * nmchunk * std::max(N, 1));
     }
     d_part.alloc(sizeof(double) * (size_t)B * g.nchunk * std::max(M, 1));
@@ -1277,6 +1279,38 @@ struct DftOp : Op {
     // the uploads above ran on the legacy stream; the solver's streams do
     // not wait for it
     MF_CK(cudaDeviceSynchronize());
+  }
+
+  // K per chunk of a product with `rows` x B outputs: the split whose CTAs
+  // load the fullest SM least (CTAs of an SM share its FP64 pipe), each chunk
+  // charged 64 of K for its start, its partials and their sum; at least 64 of
+  // K a chunk, at most 16 chunks
+  int k_chunk(int rows, int K) const {
+    int dev = 0, sms = 148;
+    MF_CK(cudaGetDevice(&dev));
+    MF_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const long tiles = (long)cdiv(rows, kGT) * cdiv(B, kGT);
+    int best = kGK;
+    double cost = 1e300;
+    for (int q = 1; q <= 16 && (q == 1 || K / q >= 64); ++q) {
+      const int chunk = std::max(kGK, cdiv(cdiv(K, q), kGK) * kGK);
+      const double t = (double)cdiv(tiles * q, sms) * (chunk + 64);
+      if (t < cost) {
+        cost = t;
+        best = chunk;
+      }
+    }
+    return best;
+  }
+
+  void launch_az(cudaStream_t s, const double* src, int gate) {
+    k_dft_az_gemm<<<dim3(cdiv(g.M, kGT), g.nchunk, cdiv(B, kGT)), 128, dg::kSmem, s>>>(g, src, c.xstride, c.st, gate, B);
+    MF_LAUNCH_CK();
+  }
+  void launch_atr(cudaStream_t s, const DftGeom& gg, int gate) {
+    k_dft_atr_gemm<<<dim3(cdiv(g.N, kGT), nmchunk, cdiv(B, kGT)), 128, dg::kSmem, s>>>(gg, d_atr.as<double>(), mchunk,
+                                                                                       nmchunk, c.st, gate, B);
+    MF_LAUNCH_CK();
   }
 
   static tc::Planes planes(DevMem* d, int np) {
@@ -1336,12 +1370,13 @@ struct DftOp : Op {
 
   // FP64 A z -> residual (and chi^2 partials)
   void forward_fp64(cudaStream_t s, const double* src, int gate, int qchi, bool store) {
-    if (gemm)
-      k_dft_az_gemm<<<dim3(cdiv(g.M, kGT), g.nchunk, cdiv(B, kGT)), 256, 0, s>>>(g, src, c.xstride, c.st, gate, B);
-    else
+    if (gemm) {
+      launch_az(s, src, gate);
+    } else {
       k_dft_az<<<dim3(std::max(1, cdiv(g.M, 256)), g.nchunk, B), 256, g.chunk * sizeof(double), s>>>(
           g, src, c.xstride, c.st, gate);
-    MF_LAUNCH_CK();
+      MF_LAUNCH_CK();
+    }
     k_dft_resid<<<dim3(std::max(1, cdiv(g.M, 256)), B), 256, 0, s>>>(g, c.st, gate, c.part, qchi, store ? 1 : 0);
     MF_LAUNCH_CK();
   }
@@ -1370,9 +1405,7 @@ struct DftOp : Op {
       return;
     }
     if (gemm) {
-      k_dft_atr_gemm<<<dim3(cdiv(g.N, kGT), nmchunk, cdiv(B, kGT)), 256, 0, s>>>(g, d_atr.as<double>(), mchunk,
-                                                                                 nmchunk, c.st, kGateGrad, B);
-      MF_LAUNCH_CK();
+      launch_atr(s, g, kGateGrad);
       k_dft_atr_finish<<<dim3(cdiv(g.N, 256), B), 256, 0, s>>>(g, d_atr.as<double>(), nmchunk, c.dfdx, c.xstride,
                                                                z_tsv, c.prm, c.tsvNX, c.tsvNY, c.st, kGateGrad);
       MF_LAUNCH_CK();
@@ -1387,9 +1420,7 @@ struct DftOp : Op {
   void atr_fp64(cudaStream_t s, const double* resid, double* out, long ostride, int gate) {
     DftGeom gg = g;
     gg.resid = const_cast<double*>(resid);
-    k_dft_atr_gemm<<<dim3(cdiv(g.N, kGT), nmchunk, cdiv(B, kGT)), 256, 0, s>>>(gg, d_atr.as<double>(), mchunk,
-                                                                               nmchunk, c.st, gate, B);
-    MF_LAUNCH_CK();
+    launch_atr(s, gg, gate);
     k_dft_atr_finish<<<dim3(cdiv(g.N, 256), B), 256, 0, s>>>(gg, d_atr.as<double>(), nmchunk, out, ostride, nullptr,
                                                              c.prm, c.tsvNX, c.tsvNY, c.st, gate);
     MF_LAUNCH_CK();
@@ -1404,8 +1435,7 @@ struct DftOp : Op {
   // FP64 anchor terms: ax_a = A x_a, r_a = y - ax_a, g_a = A^T r_a
   void refresh_anchor(cudaStream_t s, int gate) override {
     if (!tcm) return;
-    k_dft_az_gemm<<<dim3(cdiv(g.M, kGT), g.nchunk, cdiv(B, kGT)), 256, 0, s>>>(g, c.xa, c.xstride, c.st, gate, B);
-    MF_LAUNCH_CK();
+    launch_az(s, c.xa, gate);
     k_dft_anchor<<<dim3(std::max(1, cdiv(g.M, 256)), B), 256, 0, s>>>(g, c.st, gate, d_axa.as<double>(),
                                                                       d_ra.as<double>());
     MF_LAUNCH_CK();
@@ -1431,9 +1461,7 @@ struct DftOp : Op {
         return fwd.bytes();
       }
       if (!gemm) return -1;
-      k_dft_az_gemm<<<dim3(cdiv(g.M, kGT), g.nchunk, cdiv(B, kGT)), 256, 0, s>>>(g, c.z, c.xstride, c.st, kGateAll,
-                                                                                 B);
-      MF_LAUNCH_CK();
+      launch_az(s, c.z, kGateAll);
       return 8.0 * g.M * g.N + 8.0 * B * g.N + 8.0 * B * g.nchunk * g.M;
     }
     if (kernel == 1) {
@@ -1442,9 +1470,7 @@ struct DftOp : Op {
         return adj.bytes();
       }
       if (!gemm) return -1;
-      k_dft_atr_gemm<<<dim3(cdiv(g.N, kGT), nmchunk, cdiv(B, kGT)), 256, 0, s>>>(g, d_atr.as<double>(), mchunk,
-                                                                                 nmchunk, c.st, kGateAll, B);
-      MF_LAUNCH_CK();
+      launch_atr(s, g, kGateAll);
       return 8.0 * g.M * g.N + 8.0 * B * g.M + 8.0 * B * nmchunk * g.N;
     }
     return -1;
