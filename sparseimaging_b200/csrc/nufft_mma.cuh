@@ -90,6 +90,64 @@ template <typename T, int PB> constexpr size_t im_smem() {
   return (PB > 1 ? 2 : 1) * ImWindow<T>::kBytes + im_red_bytes(PB);
 }
 
+// what a warp keeps of its unit of 16 points
+struct ImUnit {
+  const double* wx;           // row weights
+  unsigned int oa, ob;        // first ones of points g and g + 8
+  int dra, drb;               // their first rows, in the window
+  bool va, vb, mixed;         // mixed: some lane of the warp has mirrored cells
+  unsigned int mir;           // bit kk: this lane's imaginary cell of column step kk is mirrored
+  double a0[kImSteps], a1[kImSteps];  // their column weights at the lane's columns
+};
+
+// row steps [s0, s1) of 4 window rows from rlo, NK column steps of 4 from w's
+// column; TWO: the unit has a second block of 8 points.  Both are template
+// arguments because a matrix instruction whose predicate is off still takes
+// its time on the pipe.
+template <int NK, bool TWO, typename T, int LD>
+__device__ __forceinline__ void interp_rows(const ImUnit& u, const T* w, int rlo, int s0, int s1, int lane,
+                                            double (&y0)[2], double (&y1)[2]) {
+  const int g = lane >> 2, t = lane & 3;
+  for (int s = s0; s < s1; ++s) {
+    const int r = rlo + 4 * s;
+    const int ja = r + t - u.dra, jb = r + t - u.drb;
+    const double wa = (u.va && ja >= 0 && ja < kTaps) ? u.wx[(size_t)u.oa + ja] : 0.0;
+    const double wb = (TWO && u.vb && jb >= 0 && jb < kTaps) ? u.wx[(size_t)u.ob + jb] : 0.0;
+    const T* brow = w + 2 * ((r + (g >> 1)) * LD + t) + (g & 1);
+    double d0[2][2] = {{0.0, 0.0}, {0.0, 0.0}}, d1[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+    double b[NK];
+#pragma unroll
+    for (int kk = 0; kk < NK; ++kk) b[kk] = (double)brow[8 * kk];
+    if (u.mixed) {
+#pragma unroll
+      for (int kk = 0; kk < NK; ++kk) b[kk] = ((u.mir >> kk) & 1u) ? -b[kk] : b[kk];
+    }
+#pragma unroll
+    for (int kk = 0; kk < NK; ++kk) {
+      dmma_884(d0[kk & 1], u.a0[kk], b[kk]);
+      if (TWO) dmma_884(d1[kk & 1], u.a1[kk], b[kk]);
+    }
+    y0[0] = fma(wa, d0[0][0] + d0[1][0], y0[0]);
+    y0[1] = fma(wa, d0[0][1] + d0[1][1], y0[1]);
+    if (TWO) {
+      y1[0] = fma(wb, d1[0][0] + d1[1][0], y1[0]);
+      y1[1] = fma(wb, d1[0][1] + d1[1][1], y1[1]);
+    }
+  }
+}
+
+template <bool TWO, typename T, int LD>
+__device__ __forceinline__ void interp_unit(const ImUnit& u, int nk, const T* w, int rlo, int s0, int s1, int lane,
+                                            double (&y0)[2], double (&y1)[2]) {
+  switch (nk) {  // 24 columns at least, 39 at most
+    case 6: interp_rows<6, TWO, T, LD>(u, w, rlo, s0, s1, lane, y0, y1); break;
+    case 7: interp_rows<7, TWO, T, LD>(u, w, rlo, s0, s1, lane, y0, y1); break;
+    case 8: interp_rows<8, TWO, T, LD>(u, w, rlo, s0, s1, lane, y0, y1); break;
+    case 9: interp_rows<9, TWO, T, LD>(u, w, rlo, s0, s1, lane, y0, y1); break;
+    default: interp_rows<kImSteps, TWO, T, LD>(u, w, rlo, s0, s1, lane, y0, y1); break;
+  }
+}
+
 template <typename T, int PB>
 __global__ void __launch_bounds__(256, 2)
     k_nufft_interp_mma(NufftGeom<T> geo, const double* __restrict__ wxd, const double* __restrict__ wyd,
@@ -177,17 +235,24 @@ __global__ void __launch_bounds__(256, 2)
   const int ns = (rhi - rlo + 3) >> 2, nk = (chi_ - clo + 3) >> 2;
   rlo = min(rlo, kImWin - 4 * ns);
   clo = min(clo, kImWin - 4 * nk);
-  double a0[kImSteps], a1[kImSteps];
-  unsigned int mir = 0;  // bit kk: column clo + 4 kk + t is mirrored (imaginary lanes only)
+  ImUnit u;
+  u.wx = wxd;
+  u.oa = (unsigned int)ka * kTaps;
+  u.ob = (unsigned int)kb * kTaps;
+  u.dra = dra;
+  u.drb = drb;
+  u.va = va;
+  u.vb = vb;
+  u.mir = 0;
 #pragma unroll
   for (int kk = 0; kk < kImSteps; ++kk) {
     const int c = clo + 4 * kk + t;
     const int ja = c - dca, jb = c - dcb;
-    a0[kk] = (va && kk < nk && ja >= 0 && ja < kTaps) ? wyd[(size_t)ka * kTaps + ja] : 0.0;
-    a1[kk] = (vb && kk < nk && jb >= 0 && jb < kTaps) ? wyd[(size_t)kb * kTaps + jb] : 0.0;
-    if ((g & 1) && half_col(tl.col0 + c, ny) < 0) mir |= 1u << kk;
+    u.a0[kk] = (va && kk < nk && ja >= 0 && ja < kTaps) ? wyd[(size_t)ka * kTaps + ja] : 0.0;
+    u.a1[kk] = (vb && kk < nk && jb >= 0 && jb < kTaps) ? wyd[(size_t)kb * kTaps + jb] : 0.0;
+    if ((g & 1) && half_col(tl.col0 + c, ny) < 0) u.mir |= 1u << kk;
   }
-  const bool mixed = __any_sync(all, mir != 0);
+  u.mixed = __any_sync(all, u.mir != 0);
   const int per = (ns + ng - 1) / ng;
   const int s0 = grp * per, s1 = on ? min(ns, s0 + per) : 0;
   for (int i = 0; i < nact; ++i) {
@@ -196,28 +261,11 @@ __global__ void __launch_bounds__(256, 2)
     if (PB > 1) cp_async_wait<1>();
     else cp_async_wait<0>();
     __syncthreads();  // window i has landed for every thread
-    const T* w = reinterpret_cast<const T*>(win + (size_t)(PB > 1 ? (i & 1) : 0) * kImWin * LD);
+    const T* w = reinterpret_cast<const T*>(win + (size_t)(PB > 1 ? (i & 1) : 0) * kImWin * LD + clo);
     double y0[2] = {0.0, 0.0}, y1[2] = {0.0, 0.0};
-    for (int s = s0; s < s1; ++s) {
-      const int r = rlo + 4 * s;
-      const int ja = r + t - dra, jb = r + t - drb;
-      const double wa = (va && ja >= 0 && ja < kTaps) ? wxd[(size_t)ka * kTaps + ja] : 0.0;
-      const double wb = (vb && jb >= 0 && jb < kTaps) ? wxd[(size_t)kb * kTaps + jb] : 0.0;
-      const T* brow = w + 2 * ((r + (g >> 1)) * LD + clo + t) + (g & 1);
-      double d0[2][2] = {{0.0, 0.0}, {0.0, 0.0}}, d1[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
-#pragma unroll
-      for (int kk = 0; kk < kImSteps; ++kk) {
-        if (kk < nk) {
-          double b = (double)brow[8 * kk];
-          if (mixed && ((mir >> kk) & 1u)) b = -b;
-          dmma_884(d0[kk & 1], a0[kk], b);
-          if (two) dmma_884(d1[kk & 1], a1[kk], b);
-        }
-      }
-      y0[0] = fma(wa, d0[0][0] + d0[1][0], y0[0]);
-      y0[1] = fma(wa, d0[0][1] + d0[1][1], y0[1]);
-      y1[0] = fma(wb, d1[0][0] + d1[1][0], y1[0]);
-      y1[1] = fma(wb, d1[0][1] + d1[1][1], y1[1]);
+    if (s0 < s1) {
+      if (two) interp_unit<true, T, LD>(u, nk, w, rlo, s0, s1, lane, y0, y1);
+      else interp_unit<false, T, LD>(u, nk, w, rlo, s0, s1, lane, y0, y1);
     }
     // over the four rows of a step (lanes t)
 #pragma unroll
