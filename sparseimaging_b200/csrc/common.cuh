@@ -204,7 +204,10 @@ template <typename T> struct FftDev {
   int n;
   int nst;
   int radix[kMaxStages];
-  const cplx<T>* tw;  // tw[k] = exp(-2 pi i k / n), k < n
+  // FP32 (fft_smem.cuh): tw[k] = exp(-2 pi i k / n), k < n.  FP64
+  // (fft_reg.cuh): stage by stage (Ns the product of the radices before it),
+  // radix R: [r - 1][k] = exp(-2 pi i k r / (Ns R)), r < R, k < Ns; n - 1 in all
+  const cplx<T>* tw;
 };
 
 }  // namespace mf

@@ -40,6 +40,7 @@
 
 #include "common.cuh"
 #include "fft_smem.cuh"
+#include "fft_reg.cuh"
 #include "nufft_ops.cuh"
 
 #include "../../include/mfista_b200.h"
@@ -90,6 +91,25 @@ __global__ void k_noalloc_twiddles(cplx<double>* __restrict__ tw, int n) {
   tw[k] = mk<double>(c, -s);
 }
 
+// the FFT's twiddles, stage by stage (FftDev); one thread per value
+__global__ void k_noalloc_stage_twiddles(cplx<double>* __restrict__ tw, FftDev<double> f) {
+  int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= f.n - 1) return;
+  int at = e, Ns = 1;
+  for (int s = 0; s < f.nst; ++s) {
+    const int R = f.radix[s], m = (R - 1) * Ns;
+    if (at < m) {
+      const int r = 1 + at / Ns, k = at % Ns;
+      double si, co;
+      sincospi(2.0 * (double)((long)k * r) / (double)((long)Ns * R), &si, &co);
+      tw[e] = mk<double>(co, -si);
+      return;
+    }
+    at -= m;
+    Ns *= R;
+  }
+}
+
 // one active problem over points [0, m)
 __global__ void k_noalloc_state(ProbState* st, int* lo, int* hi, int m) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
@@ -108,23 +128,12 @@ __global__ void k_noalloc_split(const double2* __restrict__ ax, int m, double* _
   out_i[k] = ax[k].y;
 }
 
-// same radix order as the allocating operator's FFT plans
-bool factor(int n, FftDev<double>& f) {
+// the allocating operator's FFT plans
+bool factor(int n, int log2max, FftDev<double>& f) {
   memset(&f, 0, sizeof(f));
   f.n = n;
-  int m = n;
-  auto push = [&](int r) {
-    if (f.nst >= kMaxStages) return false;
-    f.radix[f.nst++] = r;
-    return true;
-  };
-  while (m % 4 == 0) { if (!push(4)) return false; m /= 4; }
-  while (m % 2 == 0) { if (!push(2)) return false; m /= 2; }
-  while (m % 3 == 0) { if (!push(3)) return false; m /= 3; }
-  while (m % 5 == 0) { if (!push(5)) return false; m /= 5; }
-  for (int p = 7; m > 1 && p <= kMaxGenericRadix; p += 2)
-    while (m % p == 0) { if (!push(p)) return false; m /= p; }
-  return m == 1;
+  f.nst = fft_radices(n, f.radix, log2max);
+  return f.nst > 0 || n == 1;
 }
 
 inline int cdiv_i(long a, long b) { return (int)((a + b - 1) / b); }
@@ -157,10 +166,10 @@ extern "C" int mfista_nufft_forward_noalloc(const double* u_dx, const double* v_
   // an error pending from the caller's own work: report it, do not consume it
   if (cudaPeekAtLastError() != cudaSuccess) return MFISTA_ERR_CUDA;
   FftDev<double> fh, fcol;
-  if (!factor(Ny, fh) || !factor(2 * Nx, fcol)) return MFISTA_ERR_ARG;
+  if (!factor(Ny, kRowsLog2Max, fh) || !factor(2 * Nx, kColsLog2Max, fcol)) return MFISTA_ERR_ARG;
   // one row / one column per CTA, ping-pong buffers in shared memory
-  const size_t smem_rows = (size_t)2 * (Ny + 1) * sizeof(cplx<double>);
-  const size_t smem_cols = (size_t)2 * (2 * Nx + 1) * sizeof(cplx<double>);
+  const size_t smem_rows = rows_smem_bytes<double>(Ny, 1);
+  const size_t smem_cols = cols_smem_bytes<double>(2 * Nx, 1);
   if (smem_rows > kSmemDefault || smem_cols > kSmemDefault) return MFISTA_ERR_ARG;
 
   // device address of the scratch array on the current device (once per device)
@@ -202,15 +211,15 @@ extern "C" int mfista_nufft_forward_noalloc(const double* u_dx, const double* v_
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int T = 256;
   k_noalloc_state<<<1, 32, 0, s>>>(st, lo, hi, M);
-  k_noalloc_twiddles<<<cdiv_i(Ny, T), T, 0, s>>>(const_cast<cplx<double>*>(fh.tw), Ny);
-  k_noalloc_twiddles<<<cdiv_i(2 * Nx, T), T, 0, s>>>(const_cast<cplx<double>*>(fcol.tw), 2 * Nx);
+  k_noalloc_stage_twiddles<<<cdiv_i(Ny, T), T, 0, s>>>(const_cast<cplx<double>*>(fh.tw), fh);
+  k_noalloc_stage_twiddles<<<cdiv_i(2 * Nx, T), T, 0, s>>>(const_cast<cplx<double>*>(fcol.tw), fcol);
   k_noalloc_twiddles<<<cdiv_i(2 * Ny, T), T, 0, s>>>(tw_2h, 2 * Ny);
   k_noalloc_grid_index<<<cdiv_i(M, T), T, 0, s>>>(u_dx, v_dy, M, Nx, Ny, mx, my);
   k_nufft_prep_points<double><<<cdiv_i(M, T), T, 0, s>>>(u_dx, v_dy, mx, my, M, Nx, Ny, wx, wy);
   k_nufft_prep_e4<<<cdiv_i((long)Nx * Ny, T), T, 0, s>>>(e4, Nx, Ny);
-  k_nufft_rows_fwd<double><<<dim3(Nx, 1), T, smem_rows, s>>>(x, (long)Nx * Ny, e4, grid, 0, Nx, Ny, fh, tw_2h, st,
+  k_nufft_rows_fwd_reg<double><<<dim3(Nx, 1), T, smem_rows, s>>>(x, (long)Nx * Ny, e4, grid, 0, Nx, Ny, fh, tw_2h, st,
                                                               kGateAll, 1, nullptr, DynUnits{nullptr, 0});
-  k_nufft_cols<double><<<dim3(Ny + 1, 1), T, smem_cols, s>>>(grid, 0, Nx, Ny, fcol, -1, 1, 1, 0, st, kGateAll,
+  k_nufft_cols_reg<double><<<dim3(Ny + 1, 1), T, smem_cols, s>>>(grid, 0, Nx, Ny, fcol, -1, 1, 1, 0, st, kGateAll,
                                                               DynUnits{nullptr, 0});
   NufftGeom<double> geo;
   memset(&geo, 0, sizeof(geo));

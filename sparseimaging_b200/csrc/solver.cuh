@@ -20,6 +20,7 @@
 #include "common.cuh"
 #include "dft_ops.cuh"
 #include "dft_tc.cuh"
+#include "fft_reg.cuh"
 #include "fft_smem.cuh"
 #include "fftvar_ops.cuh"
 #include "fgp.cuh"
@@ -84,28 +85,72 @@ template <typename T> void make_twiddles(int n, DevMem& mem) {
   mem.upload(h.data(), h.size());
 }
 
+// The FP64 operators transform through registers (fft_reg.cuh), the FP32 ones
+// in shared memory (fft_smem.cuh).
+template <typename T> constexpr bool kRegFft = sizeof(T) == 8;
+
 template <typename T> struct FftHost {
   FftDev<T> dev;
   DevMem tw;
-  void init(int n) {
+  // log2max: the largest power-of-two radix of the FP64 form
+  void init(int n, int log2max) {
     memset(&dev, 0, sizeof(dev));
     dev.n = n;
-    int m = n;
-    auto push = [&](int r) {
-      if (dev.nst >= kMaxStages) throw Error(MFISTA_ERR_ARG, "FFT length has too many factors");
-      dev.radix[dev.nst++] = r;
-    };
-    while (m % 4 == 0) { push(4); m /= 4; }
-    while (m % 2 == 0) { push(2); m /= 2; }
-    while (m % 3 == 0) { push(3); m /= 3; }
-    while (m % 5 == 0) { push(5); m /= 5; }
-    for (int f = 7; m > 1 && f <= kMaxGenericRadix; f += 2)
-      while (m % f == 0) { push(f); m /= f; }
-    if (m > 1) throw Error(MFISTA_ERR_ARG, "FFT length " + std::to_string(n) + " has a prime factor above 16");
-    make_twiddles<T>(n, tw);
+    const char* bad = " has a prime factor above 16";
+    if constexpr (kRegFft<T>) {
+      dev.nst = fft_radices(n, dev.radix, log2max);
+      if (dev.nst == 0 && n > 1) throw Error(MFISTA_ERR_ARG, "FFT length " + std::to_string(n) + bad);
+      std::vector<cplx<T>> h;
+      int Ns = 1;
+      for (int s = 0; s < dev.nst; ++s) {
+        const int R = dev.radix[s];
+        for (int r = 1; r < R; ++r)
+          for (int k = 0; k < Ns; ++k) {
+            const long double a = 2.0L * 3.14159265358979323846264338327950288L * (long double)((long)k * r * (n / (Ns * R))) / (long double)n;
+            h.push_back(mk<T>((T)cosl(a), (T)(-sinl(a))));
+          }
+        Ns *= R;
+      }
+      if (h.empty()) h.push_back(mk<T>(1, 0));
+      tw.upload(h.data(), h.size());
+    } else {
+      int m = n;
+      auto push = [&](int r) {
+        if (dev.nst >= kMaxStages) throw Error(MFISTA_ERR_ARG, "FFT length has too many factors");
+        dev.radix[dev.nst++] = r;
+      };
+      while (m % 4 == 0) { push(4); m /= 4; }
+      while (m % 2 == 0) { push(2); m /= 2; }
+      while (m % 3 == 0) { push(3); m /= 3; }
+      while (m % 5 == 0) { push(5); m /= 5; }
+      for (int f = 7; m > 1 && f <= kMaxGenericRadix; f += 2)
+        while (m % f == 0) { push(f); m /= f; }
+      if (m > 1) throw Error(MFISTA_ERR_ARG, "FFT length " + std::to_string(n) + bad);
+      make_twiddles<T>(n, tw);
+    }
     dev.tw = tw.as<cplx<T>>();
   }
 };
+
+// dynamic shared memory of the row passes (rows of length h) and of the column
+// passes (length n)
+template <typename T> size_t fft_rows_smem(int h, int rows) {
+  if constexpr (kRegFft<T>) return rows_smem_bytes<T>(h, rows);
+  else return (size_t)2 * rows * (h + 1) * sizeof(cplx<T>);
+}
+template <typename T> size_t fft_cols_smem(int n, int cols) {
+  if constexpr (kRegFft<T>) return cols_smem_bytes<T>(n, cols);
+  else return (size_t)2 * cols * (n + 1) * sizeof(cplx<T>);
+}
+
+// Threads of a CTA of the row passes, FP64: 128 where they do the first
+// stage's items (rows x length / radix) in one or two full rounds (64 x 128
+// rows of 128, two rounds: 44 us forward and back, 51 with 256 threads), else
+// 256 (11 x 100 rows of 100, 160 items: 19 us, 25 with 128 threads)
+template <typename T> int rows_threads(const FftDev<T>& f, int rows) {
+  const int items = rows * (f.n / (f.nst ? f.radix[0] : 1));
+  return kRegFft<T> && (items <= 128 || items == 256) ? 128 : 256;
+}
 
 // Raises a kernel's dynamic shared-memory limit to at least `bytes`.  The
 // limit is per kernel and process-wide, so it is never lowered: another plan
@@ -288,6 +333,19 @@ template <typename T> struct NufftOp : Op {
   long gstride = 0;
   double inv_mm = 0;
 
+  // the FFT passes of this precision
+  static auto nufft_rows_fwd_kernel() {
+    if constexpr (kRegFft<T>) return k_nufft_rows_fwd_reg<T>;
+    else return k_nufft_rows_fwd<T>;
+  }
+  static auto nufft_cols_kernel() {
+    if constexpr (kRegFft<T>) return k_nufft_cols_reg<T>;
+    else return k_nufft_cols<T>;
+  }
+  static auto nufft_rows_inv_kernel() {
+    if constexpr (kRegFft<T>) return k_nufft_rows_inv_reg<T>;
+    else return k_nufft_rows_inv<T>;
+  }
   // forward_only: no adjoint (the FP64 operator of the anchors)
   NufftOp(Ctx& ctx, const NufftInput& in, bool correct = false, bool forward_only = false) : c(ctx) {
     if (const char* f = getenv("MFISTA_INTERP_FLY")) interp_fly = f[0] == '1';
@@ -371,8 +429,8 @@ template <typename T> struct NufftOp : Op {
       MF_LAUNCH_CK();
     }
     // FFTs: rows as complex length Ny, columns length 2Nx
-    fh.init(ny);
-    fcol.init(2 * nx);
+    fh.init(ny, kRowsLog2Max);
+    fcol.init(2 * nx, kColsLog2Max);
     make_twiddles<T>(2 * ny, tw2h);
     gstride = (long)2 * nx * (ny + 1);
     d_grid.alloc(sizeof(cplx<T>) * (size_t)B * gstride);
@@ -380,15 +438,15 @@ template <typename T> struct NufftOp : Op {
     d_y2.alloc(sizeof(cplx<T>) * (size_t)y2n);
     inv_mm = 1.0 / ((double)(2 * nx) * (double)(2 * ny));
     // launch shapes: keep the ping-pong buffers within shared memory
-    auto rows_smem = [&](int r) { return (size_t)2 * r * (ny + 1) * sizeof(cplx<T>); };
-    auto cols_smem = [&](int cc) { return (size_t)2 * cc * (2 * nx + 1) * sizeof(cplx<T>); };
+    auto rows_smem = [&](int r) { return fft_rows_smem<T>(ny, r); };
+    auto cols_smem = [&](int cc) { return fft_cols_smem<T>(2 * nx, cc); };
     while (rpc > 1 && rows_smem(rpc) > 96 * 1024) rpc /= 2;
     while (cpc > 1 && cols_smem(cpc) > 96 * 1024) cpc /= 2;
     smem_rows = rows_smem(rpc);
     smem_cols = cols_smem(cpc);
-    set_smem(k_nufft_rows_fwd<T>, smem_rows);
-    set_smem(k_nufft_rows_inv<T>, smem_rows);
-    set_smem(k_nufft_cols<T>, smem_cols);
+    set_smem(nufft_rows_fwd_kernel(), smem_rows);
+    set_smem(nufft_rows_inv_kernel(), smem_rows);
+    set_smem(nufft_cols_kernel(), smem_cols);
     set_smem(k_nufft_spread_shared<T>, spread_smem());
     MF_CK(cudaFuncSetAttribute(k_nufft_spread_shared<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     if (correct && sizeof(T) == 4) {
@@ -785,7 +843,7 @@ template <typename T> struct NufftOp : Op {
 
   void launch_rows_fwd(cudaStream_t s, const double* src, int gate, const double* sub) {
     const DynUnits d = dyn(gate, rpc);
-    k_nufft_rows_fwd<T><<<dim3(fft_grid(d, nx, rpc), B), 256, smem_rows, s>>>(
+    nufft_rows_fwd_kernel()<<<dim3(fft_grid(d, nx, rpc), B), rows_threads(fh.dev, rpc), smem_rows, s>>>(
         src, c.xstride, geo.e4, d_grid.as<cplx<T>>(), gstride, nx, ny, fh.dev, tw2h.as<cplx<T>>(), c.st, gate, rpc,
         sub, d);
     MF_LAUNCH_CK();
@@ -841,7 +899,7 @@ template <typename T> struct NufftOp : Op {
 
   void launch_cols_fwd(cudaStream_t s, int gate) {
     const DynUnits d = dyn(gate, cpc);
-    k_nufft_cols<T><<<dim3(fft_grid(d, ny + 1, cpc), B), 256, smem_cols, s>>>(
+    nufft_cols_kernel()<<<dim3(fft_grid(d, ny + 1, cpc), B), 256, smem_cols, s>>>(
         d_grid.as<cplx<T>>(), gstride, nx, ny, fcol.dev, -1, cpc, 1, 0, c.st, gate, d);
     MF_LAUNCH_CK();
   }
@@ -909,12 +967,12 @@ template <typename T> struct NufftOp : Op {
     cplx<T>* g = d_grid.as<cplx<T>>();
     launch_spread(s, g, kGateGrad);
     const DynUnits dc = dyn(kGateGrad, cpc);
-    k_nufft_cols<T><<<dim3(fft_grid(dc, ny + 1, cpc), B), 256, smem_cols, s>>>(g, gstride, nx, ny, fcol.dev, +1, cpc,
+    nufft_cols_kernel()<<<dim3(fft_grid(dc, ny + 1, cpc), B), 256, smem_cols, s>>>(g, gstride, nx, ny, fcol.dev, +1, cpc,
                                                                                0, 1, c.st, kGateGrad, dc);
     MF_LAUNCH_CK();
     TsvFuse tf{z_tsv, c.prm, c.tsvNX, c.tsvNY};
     const DynUnits dr = qtsv < 0 ? dyn(kGateGrad, rpc) : DynUnits{nullptr, 0};
-    k_nufft_rows_inv<T><<<dim3(fft_grid(dr, nx, rpc), B), 256, smem_rows, s>>>(
+    nufft_rows_inv_kernel()<<<dim3(fft_grid(dr, nx, rpc), B), rows_threads(fh.dev, rpc), smem_rows, s>>>(
         g, gstride, c.dfdx, c.xstride, geo.e4, nx, ny, inv_mm, fh.dev, tw2h.as<cplx<T>>(), tf, c.part, qtsv, c.st,
         kGateGrad, rpc, dr);
     MF_LAUNCH_CK();
@@ -934,8 +992,8 @@ template <typename T> struct NufftOp : Op {
   }
 
   void set_shapes(const LaunchShapes& sh) override {
-    auto rows_smem = [&](int r) { return (size_t)2 * r * (ny + 1) * sizeof(cplx<T>); };
-    auto cols_smem = [&](int cc) { return (size_t)2 * cc * (2 * nx + 1) * sizeof(cplx<T>); };
+    auto rows_smem = [&](int r) { return fft_rows_smem<T>(ny, r); };
+    auto cols_smem = [&](int cc) { return fft_cols_smem<T>(2 * nx, cc); };
     if (shared && sh.interp_ppw && (sh.interp_ppw < 1 || sh.interp_ppw > kMaxInterpPpw))
       throw Error(MFISTA_ERR_ARG, "interp_ppw must be 1..32");
     if (shared && sh.spread_cluster && (sh.spread_cluster < 1 || sh.spread_cluster > 16))
@@ -953,13 +1011,13 @@ template <typename T> struct NufftOp : Op {
     if (sh.rows_per_cta) {
       rpc = sh.rows_per_cta;
       smem_rows = rows_smem(rpc);
-      set_smem(k_nufft_rows_fwd<T>, smem_rows);
-      set_smem(k_nufft_rows_inv<T>, smem_rows);
+      set_smem(nufft_rows_fwd_kernel(), smem_rows);
+      set_smem(nufft_rows_inv_kernel(), smem_rows);
     }
     if (sh.cols_per_cta) {
       cpc = sh.cols_per_cta;
       smem_cols = cols_smem(cpc);
-      set_smem(k_nufft_cols<T>, smem_cols);
+      set_smem(nufft_cols_kernel(), smem_cols);
     }
   }
   double fscale() const override { return 0.5; }
@@ -983,18 +1041,18 @@ template <typename T> struct NufftOp : Op {
         launch_rows_fwd(s, c.z, kGateTrial, nullptr);
         return B * N * 8 + N * 8 + B * half_rows * cs;
       case 3:
-        k_nufft_cols<T><<<dim3(cdiv(ny + 1, cpc), B), 256, smem_cols, s>>>(g, gstride, nx, ny, fcol.dev, -1, cpc, 1, 0,
+        nufft_cols_kernel()<<<dim3(cdiv(ny + 1, cpc), B), 256, smem_cols, s>>>(g, gstride, nx, ny, fcol.dev, -1, cpc, 1, 0,
                                                                            c.st, kGateTrial, DynUnits{nullptr, 0});
         MF_LAUNCH_CK();
         return B * (half_rows + G) * cs;
       case 4:
-        k_nufft_cols<T><<<dim3(cdiv(ny + 1, cpc), B), 256, smem_cols, s>>>(g, gstride, nx, ny, fcol.dev, +1, cpc, 0, 1,
+        nufft_cols_kernel()<<<dim3(cdiv(ny + 1, cpc), B), 256, smem_cols, s>>>(g, gstride, nx, ny, fcol.dev, +1, cpc, 0, 1,
                                                                            c.st, kGateGrad, DynUnits{nullptr, 0});
         MF_LAUNCH_CK();
         return B * (G + half_rows) * cs;
       case 5: {
         TsvFuse tf{c.z, c.prm, c.tsvNX, c.tsvNY};
-        k_nufft_rows_inv<T><<<dim3(cdiv(nx, rpc), B), 256, smem_rows, s>>>(
+        nufft_rows_inv_kernel()<<<dim3(cdiv(nx, rpc), B), rows_threads(fh.dev, rpc), smem_rows, s>>>(
             g, gstride, c.dfdx, c.xstride, geo.e4, nx, ny, inv_mm, fh.dev, tw2h.as<cplx<T>>(), tf, c.part, kQTsvZ,
             c.st, kGateGrad, rpc, DynUnits{nullptr, 0});
         MF_LAUNCH_CK();
@@ -1031,6 +1089,19 @@ template <typename T> struct FftVarOp : Op {
   std::unique_ptr<FftVarOp<double>> exact;
   DevMem d_axa;
 
+  // the FFT passes of this precision
+  static auto fftv_rows_fwd_kernel() {
+    if constexpr (kRegFft<T>) return k_fftv_rows_fwd_reg<T>;
+    else return k_fftv_rows_fwd<T>;
+  }
+  static auto fftv_cols_kernel() {
+    if constexpr (kRegFft<T>) return k_fftv_cols_reg<T>;
+    else return k_fftv_cols<T>;
+  }
+  static auto fftv_rows_inv_kernel() {
+    if constexpr (kRegFft<T>) return k_fftv_rows_inv_reg<T>;
+    else return k_fftv_rows_inv<T>;
+  }
   FftVarOp(Ctx& ctx, const FftVarInput& in, bool correct = false) : c(ctx) {
     NX = in.NX;
     NY = in.NY;
@@ -1059,8 +1130,8 @@ template <typename T> struct FftVarOp : Op {
     geo.mask_h = d_mask.as<double>();
     geo.yf_h = d_yf.as<double2>();
     geo.geo_stride = 0;
-    fh.init(NY / 2);
-    fnx.init(NX);
+    fh.init(NY / 2, kRowsLog2Max);
+    fnx.init(NX, kColsLog2Max);
     make_twiddles<T>(NY, tw2h);
     hstride = (long)NX * NYh;
     d_H.alloc(sizeof(cplx<T>) * (size_t)B * hstride);
@@ -1082,22 +1153,22 @@ template <typename T> struct FftVarOp : Op {
   void set_rpc_cpc(int r, int cc) {
     rpc = r;
     cpc = cc;
-    smem_rows = (size_t)2 * rpc * (NY / 2 + 1) * sizeof(cplx<T>);
-    smem_cols = (size_t)2 * cpc * (NX + 1) * sizeof(cplx<T>);
-    set_smem(k_fftv_rows_fwd<T>, smem_rows);
-    set_smem(k_fftv_rows_inv<T>, smem_rows);
-    set_smem(k_fftv_cols<T>, smem_cols);
+    smem_rows = fft_rows_smem<T>(NY / 2, rpc);
+    smem_cols = fft_cols_smem<T>(NX, cpc);
+    set_smem(fftv_rows_fwd_kernel(), smem_rows);
+    set_smem(fftv_rows_inv_kernel(), smem_rows);
+    set_smem(fftv_cols_kernel(), smem_cols);
   }
 
   void launch_rows_fwd(cudaStream_t s, const double* src, int gate, const double* sub) {
-    k_fftv_rows_fwd<T><<<dim3(cdiv(NX, rpc), B), 256, smem_rows, s>>>(src, c.xstride, d_H.as<cplx<T>>(), hstride, NX,
+    fftv_rows_fwd_kernel()<<<dim3(cdiv(NX, rpc), B), rows_threads(fh.dev, rpc), smem_rows, s>>>(src, c.xstride, d_H.as<cplx<T>>(), hstride, NX,
                                                                       NY, fh.dev, tw2h.as<cplx<T>>(), c.st, gate, rpc,
                                                                       sub);
     MF_LAUNCH_CK();
   }
 
   void launch_cols_fwd(cudaStream_t s, int gate, int qchi, bool store, const double2* base, double2* raw_out) {
-    k_fftv_cols<T><<<dim3(cdiv(NYh, cpc), B), 256, smem_cols, s>>>(d_H.as<cplx<T>>(), hstride, NX, NYh, fnx.dev, -1,
+    fftv_cols_kernel()<<<dim3(cdiv(NYh, cpc), B), 256, smem_cols, s>>>(d_H.as<cplx<T>>(), hstride, NX, NYh, fnx.dev, -1,
                                                                    cpc, geo, sqrtn, c.st, gate, c.part, qchi,
                                                                    store ? 1 : 0, base, raw_out);
     MF_LAUNCH_CK();
@@ -1125,10 +1196,10 @@ template <typename T> struct FftVarOp : Op {
 
   void adjoint(cudaStream_t s, const double* z_tsv, int qtsv) override {
     cplx<T>* H = d_H.as<cplx<T>>();
-    k_fftv_cols<T><<<dim3(cdiv(NYh, cpc), B), 256, smem_cols, s>>>(H, hstride, NX, NYh, fnx.dev, +1, cpc, geo, sqrtn,
+    fftv_cols_kernel()<<<dim3(cdiv(NYh, cpc), B), 256, smem_cols, s>>>(H, hstride, NX, NYh, fnx.dev, +1, cpc, geo, sqrtn,
                                                                    c.st, kGateGrad, c.part, -1, 0, nullptr, nullptr);
     MF_LAUNCH_CK();
-    k_fftv_rows_inv<T><<<dim3(cdiv(NX, rpc), B), 256, smem_rows, s>>>(
+    fftv_rows_inv_kernel()<<<dim3(cdiv(NX, rpc), B), rows_threads(fh.dev, rpc), smem_rows, s>>>(
         H, hstride, c.dfdx, c.xstride, NX, NY, fh.dev, tw2h.as<cplx<T>>(), z_tsv, c.prm, c.tsvNX, c.tsvNY, c.part,
         qtsv, c.st, kGateGrad, rpc);
     MF_LAUNCH_CK();
