@@ -35,9 +35,50 @@ struct FgpArgs {
   long scratch_stride;  // bytes per problem
 };
 
+// projection of a pixel's duals (P_pqiso, c/mfista_TV_lib.c:160-187): divided by
+// their norm where it exceeds 1 (hp, hq: the pixel has a right / lower
+// neighbour; a single dual is clamped).  Inside the unit ball nothing is
+// computed, so a warp whose duals all lie there skips the root.
+template <typename T>
+__device__ __forceinline__ void fgp_project(bool hp, bool hq, T rp, T sq, T& np, T& nq) {
+  np = rp;
+  nq = sq;
+  if (hp && hq) {
+    const T n2 = fma(rp, rp, sq * sq);
+    if (!(n2 <= 1)) {
+      if constexpr (sizeof(T) == 8) {  // a third of the instructions of a root and two divisions
+        const T inv = rsqrt(n2);
+        np = rp * inv;
+        nq = sq * inv;
+      } else {
+        const T tmp = sqrt(n2);
+        np = rp / tmp;
+        nq = sq / tmp;
+      }
+    }
+  } else if (hp) {
+    if (!(fabs(rp) <= 1)) np = rp / fabs(rp);
+  } else if (hq) {
+    if (!(fabs(sq) <= 1)) nq = sq / fabs(sq);
+  }
+}
+
+// betas[2 k], [2 k + 1]: (1 + (t_k - 1) / t_{k+1}) and -(t_k - 1) / t_{k+1},
+// t_0 = 1
+static __global__ void k_fgp_betas(double* __restrict__ betas, int iters) {
+  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+  double tt = 1.0;
+  for (int it = 0; it < iters; ++it) {
+    double tnew = (1 + sqrt(1 + 4 * tt * tt)) / 2;
+    betas[2 * it] = 1 + (tt - 1) / tnew;
+    betas[2 * it + 1] = -(tt - 1) / tnew;
+    tt = tnew;
+  }
+}
+
 // slab arrays: xv, p, q, r, s, b — each rows_per_cta x NX values of T
 template <typename T, bool SMEM>
-__global__ void k_fgp(FgpArgs a) {
+__global__ void k_fgp(FgpArgs a, const double* __restrict__ betas) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = (int)cluster.block_rank();
@@ -125,7 +166,6 @@ __global__ void k_fgp(FgpArgs a) {
     return v;
   };
   cluster.sync();
-  double tt = 1.0;
   for (int it = 0; it <= a.iters; ++it) {
     const bool last = it == a.iters;
     const T* pr = last ? PP : RR;
@@ -148,9 +188,8 @@ __global__ void k_fgp(FgpArgs a) {
       break;
     }
     cluster.sync();
-    double tnew = (1 + sqrt(1 + 4 * tt * tt)) / 2;
-    const T beta1 = (T)(1 + (tt - 1) / tnew);
-    const T beta2 = (T)(-(tt - 1) / tnew);
+    const T beta1 = (T)betas[2 * it];
+    const T beta2 = (T)betas[2 * it + 1];
     // phase B
     {
       const T* xb = (j1 < NY && nrow > 0 && rank + 1 < csize) ? peer(XV, rank + 1) : nullptr;
@@ -165,35 +204,187 @@ __global__ void k_fgp(FgpArgs a) {
           T below = (jl + 1 < nrow) ? XV[t + NX] : xb[i];
           sq = SS[t] + alpha3 * (xv - below);
         }
-        T np = 0, nq = 0;
-        if (hp && hq) {
-          T tmp = sqrt(rp * rp + sq * sq);
-          if (tmp < 1) tmp = 1;
-          np = rp / tmp;
-          nq = sq / tmp;
-        } else if (hp) {
-          T tmp = fabs(rp);
-          if (tmp < 1) tmp = 1;
-          np = rp / tmp;
-        } else if (hq) {
-          T tmp = fabs(sq);
-          if (tmp < 1) tmp = 1;
-          nq = sq / tmp;
-        }
+        T np, nq;
+        fgp_project<T>(hp, hq, rp, sq, np, nq);
         if (hp) {
-          RR[t] = np * beta1 + beta2 * PP[t];
+          RR[t] = fma(np, beta1, beta2 * PP[t]);
           PP[t] = np;
         }
         if (hq) {
-          SS[t] = nq * beta1 + beta2 * QQ[t];
+          SS[t] = fma(nq, beta1, beta2 * QQ[t]);
           QQ[t] = nq;
         }
       }
     }
-    tt = tnew;
     cluster.sync();
   }
 }
 #undef FGP_FOR_LOCAL
+
+// ---------------------------------------------------------------------------
+// The same iteration with the dual variables in registers, for images whose
+// slab rows fit a CTA's threads.  A thread owns NR consecutive rows of one
+// column; shared memory carries only what neighbours need (the fast duals r, s
+// and the image x: 7 accesses a pixel, 18 with all six arrays there), and one
+// cluster barrier an iteration suffices: a CTA forms the image row below its
+// slab itself, from that row's r and s, and every CTA pushes its first r, s row
+// and its last s row into its neighbours' halo buffers (two sets, by parity)
+// when it updates them.  Arithmetic and its order per pixel are k_fgp's, so
+// both give the same bits.
+//
+// Bound by the chain of an iteration (barrier, shared-memory hops, the FP64
+// root) with few problems and by the FP64 / FP32 pipes with many.  Measured on
+// B200, 50 iterations, us (k_fgp before -> here, NR = 1, 16 CTAs a problem):
+// one problem of 64 x 64 FP64 101 -> 55, 128 x 128 219 -> 73 (FP32 189 -> 74);
+// 13 of 96 x 96 FP32 166 -> 105 (NR = 2).
+// ---------------------------------------------------------------------------
+constexpr int kFgpThreads = 1024;
+
+template <typename T> size_t fgp_reg_smem(int rows, int NX) { return sizeof(T) * (size_t)(3 * rows + 7) * NX; }
+
+template <typename T, int NR>
+__global__ void __launch_bounds__(kFgpThreads, 1) k_fgp_reg(FgpArgs a, const double* __restrict__ betas) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = (int)cluster.block_rank();
+  const int b = blockIdx.y;
+  const ProbState& S = a.st[b];
+  // uniform over the cluster (same problem): safe to return before barriers
+  if (!gate_ok(S, kGateTrial)) return;
+  const ProbParams P = a.prm[b];
+  const int NX = a.NX, NY = a.NY, rpc = a.rows_per_cta;
+  const int j0 = rank * rpc;
+  const int j1 = min(NY, j0 + rpc);
+  const int nrow = max(0, j1 - j0);
+  T* RR = reinterpret_cast<T*>(smem_raw);   // [rpc][NX]
+  T* SS = RR + (size_t)rpc * NX;            // [rpc][NX]
+  T* XX = SS + (size_t)rpc * NX;            // [rpc + 1][NX]
+  T* HS = XX + (size_t)(rpc + 1) * NX;      // s of the row above, [2][NX]
+  T* HR = HS + 2 * NX;                      // r of the row below, [2][NX]
+  T* HB = HR + 2 * NX;                      // s of the row below, [2][NX]
+  const double c = S.c;
+  const double lam_tv = P.lambda_tv / c;
+  const double lam_l1 = P.lambda_l1 / c;
+  const bool nonneg = P.nonneg == 1;
+  const float* box = P.box_flag == 1 ? a.box : nullptr;
+  const double* z = a.z + (size_t)b * a.xstride;
+  const double* d = a.dfdx + (size_t)b * a.xstride;
+  auto rhs = [&](int f) -> T {
+    double bv;
+    if (nonneg) bv = ((1.0 * (-P.lambda_l1 / c)) + d[f] * (1.0 / c)) + z[f];
+    else bv = d[f] * (1.0 / c) + z[f];
+    return (T)bv;
+  };
+  const T alpha1 = (T)(-lam_tv);
+  const T alpha3 = (T)(1.0 / (8 * lam_tv));
+  const T eta = (T)lam_l1;
+  auto prox = [&](T v, int f) -> T {
+    if (nonneg) {
+      if (box && box[f] == 0.0f) return 0;
+      return v < 0 ? T(0) : v;
+    }
+    if (box) {
+      if (box[f] == 0.0f || (v < eta && v > -eta)) return 0;
+      return v >= eta ? v - eta : v + eta;
+    }
+    if (v >= eta) return v - eta;
+    if (v <= -eta) return v + eta;
+    return 0;
+  };
+  // thread -> column i, rows jl0 .. jl0 + NR - 1 of the slab
+  const int grp = (int)threadIdx.x / NX, i = (int)threadIdx.x - grp * NX;
+  const int jl0 = grp * NR;
+  const int mine = max(0, min(NR, nrow - jl0));
+  // the thread of the slab's last row also forms the row below it
+  const bool below = j1 < NY && mine > 0 && jl0 + mine == nrow;
+  T p[NR], q[NR], r[NR], s[NR], bb[NR], x[NR];
+#pragma unroll
+  for (int k = 0; k < NR; ++k) {
+    p[k] = q[k] = r[k] = s[k] = x[k] = 0;
+    bb[k] = k < mine ? rhs((j0 + jl0 + k) * NX + i) : T(0);
+    if (k < mine) RR[(jl0 + k) * NX + i] = SS[(jl0 + k) * NX + i] = 0;
+  }
+  const T bbelow = below ? rhs(j1 * NX + i) : T(0);
+  if (grp == 0)
+    for (int h = 0; h < 2; ++h) HS[h * NX + i] = HR[h * NX + i] = HB[h * NX + i] = 0;
+  // one pixel of b - lambda_tv Lpq(r, s), as k_fgp forms it
+  auto image = [&](T left, T here, T above, T self, T bv, int j) -> T {
+    T v = 0;
+    if (i >= 1) v -= left;
+    if (i < NX - 1) v += here;
+    if (j >= 1) v -= above;
+    if (j < NY - 1) v += self;
+    T w = v * alpha1 + bv;
+    return prox(w, j * NX + i);
+  };
+  cluster.sync();
+  for (int it = 0; it <= a.iters; ++it) {
+    const bool last = it == a.iters;
+    const int par = it & 1;
+    // phase A (with p, q in r, s after the last update)
+#pragma unroll
+    for (int k = 0; k < NR; ++k)
+      if (k < mine) {
+        const int jl = jl0 + k, t = jl * NX + i, j = j0 + jl;
+        const T left = i >= 1 ? RR[t - 1] : T(0);
+        const T above = k > 0 ? s[k > 0 ? k - 1 : 0] : jl > 0 ? SS[t - NX] : HS[par * NX + i];
+        x[k] = image(left, r[k], above, s[k], bb[k], j);
+        if (last) a.xnew[(size_t)b * a.xstride + (size_t)j * NX + i] = (double)x[k];
+        else XX[t] = x[k];
+      }
+    if (last) break;
+    T xb = 0;  // image row below the slab
+    if (below) {
+      const T left = i >= 1 ? HR[par * NX + i - 1] : T(0);
+      T above = 0;
+#pragma unroll
+      for (int k = 0; k < NR; ++k)
+        if (k == mine - 1) above = s[k];
+      xb = image(left, HR[par * NX + i], above, HB[par * NX + i], bbelow, j1);
+    }
+    __syncthreads();
+    const T beta1 = (T)betas[2 * it];
+    const T beta2 = (T)betas[2 * it + 1];
+    const bool lead = it + 1 == a.iters;  // the next phase A is the last one: hand on p, q
+    T* up = rank > 0 ? cluster.map_shared_rank(HR, rank - 1) : nullptr;        // its row below is my first
+    T* down = j1 < NY ? cluster.map_shared_rank(HS, rank + 1) : nullptr;       // its row above is my last
+    // phase B
+#pragma unroll
+    for (int k = 0; k < NR; ++k)
+      if (k < mine) {
+        const int jl = jl0 + k, t = jl * NX + i, j = j0 + jl;
+        const bool hp = i < NX - 1, hq = j < NY - 1;
+        T rp = 0, sq = 0;
+        if (hp) rp = r[k] + alpha3 * (x[k] - XX[t + 1]);
+        if (hq) {
+          const T xd = jl + 1 == nrow ? xb : k + 1 < NR ? x[k + 1 < NR ? k + 1 : k] : XX[t + NX];
+          sq = s[k] + alpha3 * (x[k] - xd);
+        }
+        T np, nq;
+        fgp_project<T>(hp, hq, rp, sq, np, nq);
+        if (hp) {
+          r[k] = fma(np, beta1, beta2 * p[k]);
+          p[k] = np;
+        }
+        if (hq) {
+          s[k] = fma(nq, beta1, beta2 * q[k]);
+          q[k] = nq;
+        }
+        if (lead) {
+          r[k] = p[k];
+          s[k] = q[k];
+        }
+        RR[t] = r[k];
+        SS[t] = s[k];
+        if (jl == 0 && up) {
+          up[(par ^ 1) * NX + i] = r[k];
+          up[2 * NX + (par ^ 1) * NX + i] = s[k];
+        }
+        if (jl + 1 == nrow && down) down[(par ^ 1) * NX + i] = s[k];
+      }
+    cluster.sync();
+  }
+}
+
 
 }  // namespace mf

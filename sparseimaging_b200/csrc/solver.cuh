@@ -1581,6 +1581,8 @@ struct Solver {
   bool fgp_smem = true;
   size_t fgp_smem_bytes = 0;
   long fgp_scratch_stride = 0;
+  int fgp_nr = 0, fgp_threads = 256;  // k_fgp_reg: rows per thread (0: k_fgp)
+  DevMem d_betas;
   int per_step_launches = 0;
   int loop_unroll = 4;  // steps per pass of the device loop (MFISTA_LOOP_UNROLL)
   // the gradient block under an IF node (MFISTA_GRAD_IF=1), or launched
@@ -1705,10 +1707,10 @@ struct Solver {
     MF_CK(cudaDeviceSynchronize());
   }
 
-  template <typename K> int max_clusters(K kern, int cs, size_t smem) {
+  template <typename K> int max_clusters(K kern, int cs, size_t smem, int threads = 256) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(cs, 1, 1);
-    cfg.blockDim = dim3(256, 1, 1);
+    cfg.blockDim = dim3(threads, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1730,6 +1732,34 @@ struct Solver {
     if (smem) set_smem(kern, smem);
   }
 
+  struct FgpShape {
+    int cs = 0, rpc = 0, nr = 0, threads = 256;
+    size_t bytes = 0;
+    double cost = 1e300;
+  };
+
+  // Time of an FGP launch in units of one problem with k_fgp_reg<1> and 16
+  // CTAs, from the clusters that are resident at once: whole rounds and a rest.
+  // `one`: a round with a CTA per SM; share[k]: what a round costs when k + 1
+  // CTAs share an SM (their pipes and barriers overlap in part).
+  double fgp_cost(int resident, int cs, double one, const double (&share)[4], int sms) const {
+    if (resident < 1) return 1e300;
+    auto round = [&](int n) { return n ? one * share[std::min(3, cdiv((long)n * cs, sms) - 1)] : 0.0; };
+    return (ctx.B / resident) * round(resident) + round(ctx.B % resident);
+  }
+
+  // k_fgp_reg with NR rows a thread and cs CTAs a problem, if it fits and is
+  // expected to be faster than `best`
+  template <typename T, int NR> void try_fgp_reg(int cs, double one, int sms, FgpShape& best) {
+    const int NX = ctx.tsvNX, rows = cdiv(ctx.tsvNY, cs), groups = cdiv(rows, NR);
+    const size_t bytes = fgp_reg_smem<T>(rows, NX);
+    if ((long)groups * NX > kFgpThreads || bytes > 200 * 1024) return;
+    prep_fgp_kernel(k_fgp_reg<T, NR>, cs, bytes);
+    const double share[4] = {1.0, 1.25, 1.5, 1.75};
+    const double cost = fgp_cost(max_clusters(k_fgp_reg<T, NR>, cs, bytes, groups * NX), cs, one, share, sms);
+    if (cost < best.cost) best = FgpShape{cs, rows, NR, groups * NX, bytes, cost};
+  }
+
   // Picks the FGP cluster shape: slabs in shared memory with 8 or 16 CTAs
   // when they fit and such a cluster can be resident, else global slabs.
   template <typename T> void pick_fgp_shape() {
@@ -1738,12 +1768,38 @@ struct Solver {
     // few problems: 16 CTAs per problem (more SMs busy, half the rows per CTA);
     // otherwise 8 (the GPU is full either way, fewer cluster-wide barriers)
     const bool few = ctx.B * 8 < 148;
+    int dev = 0, sms = 148;
+    MF_CK(cudaGetDevice(&dev));
+    MF_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    // duals in registers: with one and two rows a thread and 16 and 8 CTAs a
+    // problem (measured at 64, 96 and 128 pixels a side: a round of one problem
+    // takes 1, 1.55, 1.08 and 2 times the first)
+    FgpShape best;
+    try_fgp_reg<T, 1>(16, 1.0, sms, best);
+    try_fgp_reg<T, 1>(8, 1.08, sms, best);
+    try_fgp_reg<T, 2>(16, 1.55, sms, best);
+    try_fgp_reg<T, 2>(8, 2.0, sms, best);
+    d_betas.alloc(sizeof(double) * 2 * (size_t)std::max(fgp_iter, 1));
+    k_fgp_betas<<<1, 32, 0, stream>>>(d_betas.as<double>(), fgp_iter);
+    MF_LAUNCH_CK();
+    auto use_reg = [&]() {
+      fgp_cs = best.cs;
+      fgp_rpc = best.rpc;
+      fgp_nr = best.nr;
+      fgp_threads = best.threads;
+      fgp_smem_bytes = best.bytes;
+    };
     for (int cs : {few ? 16 : 8, few ? 8 : 16}) {
       int rpc = cdiv(NY, cs);
       size_t bytes = (size_t)6 * rpc * NX * sizeof(T);
       if (bytes > limit) continue;
       prep_fgp_kernel(k_fgp<T, true>, cs, bytes);
-      if (max_clusters(k_fgp<T, true>, cs, bytes) > 0) {
+      const int resident = max_clusters(k_fgp<T, true>, cs, bytes);
+      if (resident > 0) {
+        // many small problems: its CTAs hide each other's barriers better (64 of
+        // 96 x 96 in FP64: 374 us, k_fgp_reg 475)
+        const double share[4] = {1.0, 1.8, 2.0, 2.2};
+        if (best.cost < fgp_cost(resident, cs, 2.8, share, sms)) return use_reg();
         fgp_cs = cs;
         fgp_rpc = rpc;
         fgp_smem = true;
@@ -1751,6 +1807,7 @@ struct Solver {
         return;
       }
     }
+    if (best.nr) return use_reg();
     fgp_cs = 8;
     fgp_rpc = cdiv(NY, fgp_cs);
     fgp_smem = false;
@@ -1782,7 +1839,7 @@ struct Solver {
     a.scratch_stride = fgp_scratch_stride;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(fgp_cs, ctx.B, 1);
-    cfg.blockDim = dim3(256, 1, 1);
+    cfg.blockDim = dim3(fgp_threads, 1, 1);
     cfg.dynamicSmemBytes = fgp_smem_bytes;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
@@ -1792,12 +1849,23 @@ struct Solver {
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
+    const double* be = d_betas.as<double>();
+    if (fgp_nr) {
+      if (precision == MFISTA_FP32) {
+        if (fgp_nr == 1) MF_CK(cudaLaunchKernelEx(&cfg, k_fgp_reg<float, 1>, a, be));
+        else MF_CK(cudaLaunchKernelEx(&cfg, k_fgp_reg<float, 2>, a, be));
+      } else {
+        if (fgp_nr == 1) MF_CK(cudaLaunchKernelEx(&cfg, k_fgp_reg<double, 1>, a, be));
+        else MF_CK(cudaLaunchKernelEx(&cfg, k_fgp_reg<double, 2>, a, be));
+      }
+      return;
+    }
     if (precision == MFISTA_FP32) {
-      if (fgp_smem) MF_CK(cudaLaunchKernelEx(&cfg, k_fgp<float, true>, a));
-      else MF_CK(cudaLaunchKernelEx(&cfg, k_fgp<float, false>, a));
+      if (fgp_smem) MF_CK(cudaLaunchKernelEx(&cfg, k_fgp<float, true>, a, be));
+      else MF_CK(cudaLaunchKernelEx(&cfg, k_fgp<float, false>, a, be));
     } else {
-      if (fgp_smem) MF_CK(cudaLaunchKernelEx(&cfg, k_fgp<double, true>, a));
-      else MF_CK(cudaLaunchKernelEx(&cfg, k_fgp<double, false>, a));
+      if (fgp_smem) MF_CK(cudaLaunchKernelEx(&cfg, k_fgp<double, true>, a, be));
+      else MF_CK(cudaLaunchKernelEx(&cfg, k_fgp<double, false>, a, be));
     }
   }
 
