@@ -167,6 +167,34 @@ __device__ __forceinline__ int active_chunk(const ProbState* __restrict__ st, in
   return min(max(base_rank - lo, 0), PB);
 }
 
+// This CTA's share of the active problems when gridDim.y >= ceil(B / PB) CTAs
+// divide them evenly: fewer active problems make every share smaller instead
+// of leaving the last CTAs without work.
+template <int PB>
+__device__ __forceinline__ int active_share(const ProbState* __restrict__ st, int gate, int B, int* list, int* s_cnt,
+                                            const int* __restrict__ lists) {
+  const int gl = lists ? gate_list_slot(gate) : -1;
+  const int n = gl >= 0 ? lists[(size_t)gl * (B + 1)] : B;
+  const int per = (n + (int)gridDim.y - 1) / (int)gridDim.y;
+  const int lo = (int)blockIdx.y * per;
+  const int cnt = min(max(n - lo, 0), per);
+  if (gl >= 0) {
+    const int* L = lists + (size_t)gl * (B + 1);
+    if ((int)threadIdx.x < cnt) list[threadIdx.x] = L[1 + lo + threadIdx.x];
+    __syncthreads();
+    return cnt;
+  }
+  // outside the device loop: the passing ones of problems [lo, lo + per)
+  if (threadIdx.x < 32) {
+    const bool on = (int)threadIdx.x < cnt && gate_ok(st[lo + threadIdx.x], gate);
+    const unsigned int bal = __ballot_sync(0xffffffffu, on);
+    if (on) list[__popc(bal & ((1u << threadIdx.x) - 1u))] = lo + threadIdx.x;
+    if (threadIdx.x == 0) s_cnt[0] = __popc(bal);
+  }
+  __syncthreads();
+  return s_cnt[0];
+}
+
 // deterministic reductions --------------------------------------------------
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll

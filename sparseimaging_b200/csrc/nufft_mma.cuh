@@ -58,26 +58,33 @@ __device__ __forceinline__ void cp_async_cell(cplx<T>* dst, const cplx<T>* src, 
 // as m8n8k4 products: A = wy (in registers for all problems), B = the window's
 // cells (one 8-byte shared load per lane serves both blocks of 8 points), so
 // nothing of a matrix tile is idle for a single problem.  Only the rows and
-// columns that the 16 points reach are walked.  A CTA with few points splits
-// its window rows over the warps.
+// columns that the 16 points reach are walked, in up to four row groups whose
+// sums are added as (0 + 1) + (2 + 3); a CTA with few points gives its warps
+// one or two groups each.  Bound by the FP64 pipe where the chip is full and
+// by the length of one CTA's chain where it is not, so the points per CTA
+// (32, 64 or 128) and the problems per CTA follow the amount of work
+// (NufftOp::build_im_tiles): 128-point CTAs of 8 problems throughout took 215
+// us an iteration at 100 x 100 with 11 problems (166 here), 106 at 64 x 64
+// with one (93).
 // Signs: the reference negates the imaginary part of direct taps (NU_SIGN) and
 // keeps that of mirrored ones; a tap is direct or mirrored by its column alone,
 // so the imaginary parts of mirrored columns are flipped at the fragment and
 // the sum is negated once.
-// A problem's sums depend neither on the chunk nor on its slot in it.
+// A problem's sums depend neither on its CTA's points nor on the other
+// problems: groups and chi^2 slots (32 points) are the same for every cut.
 // ---------------------------------------------------------------------------
 constexpr int kImTile = 16;
 constexpr int kImWin = kImTile + kTaps;  // 40: 39 used, a multiple of 4
-constexpr int kImPts = 128;              // points per CTA: 8 warps x 16
+constexpr int kImPts = 128;              // points per CTA at most: 8 warps x 16
 constexpr int kImSteps = kImWin / 4;     // column steps of 4
+constexpr int kImGroup = 3;              // row steps of 4 per row group: at most four groups
 
 struct ImTileItem {
   int row0, col0;    // window origin, virtual
   int start, count;  // perm[start, start + count)
   int prob;          // its problem (points of its own), or -1 (shared points)
-  int slot;          // chi^2 slot
-  int ntiles;        // CTAs (= chi^2 slots written) of this problem
-  int pad;
+  int slot, nslot;   // first chi^2 slot (one per 32 points), slots of the problem
+  int item, nitem;   // CTA of the problem, CTAs of the problem
 };
 
 // row stride of the staged window: the four rows of a B fragment hit all banks
@@ -86,9 +93,12 @@ template <typename T> struct ImWindow {
   static constexpr size_t kBytes = sizeof(cplx<T>) * (size_t)kImWin * kLd;
 };
 constexpr size_t im_red_bytes(int pb) { return sizeof(double2) * (size_t)pb * 8 * 16; }
+constexpr int kImBuf = 3;  // staged windows in flight
 template <typename T, int PB> constexpr size_t im_smem() {
-  return (PB > 1 ? 2 : 1) * ImWindow<T>::kBytes + im_red_bytes(PB);
+  return (PB > 1 ? kImBuf : 1) * ImWindow<T>::kBytes + im_red_bytes(PB);
 }
+
+__device__ __forceinline__ double2 im_add(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 
 // what a warp keeps of its unit of 16 points
 struct ImUnit {
@@ -160,7 +170,7 @@ __global__ void __launch_bounds__(256, 2)
   constexpr int kCells = (kImWin * kImWin + 255) / 256;
   extern __shared__ __align__(16) unsigned char im_smem_raw[];
   cplx<T>* win = reinterpret_cast<cplx<T>*>(im_smem_raw);
-  double2* s_red = reinterpret_cast<double2*>(im_smem_raw + (PB > 1 ? 2 : 1) * ImWindow<T>::kBytes);
+  double* s_red = reinterpret_cast<double*>(im_smem_raw + (PB > 1 ? kImBuf : 1) * ImWindow<T>::kBytes);
   __shared__ int s_list[PB];
   __shared__ int s_cnt[8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -168,7 +178,7 @@ __global__ void __launch_bounds__(256, 2)
   const ImTileItem tl = tiles[blockIdx.x];
   int nact;
   if (PB > 1) {
-    nact = active_chunk<PB>(st, gate, B, blockIdx.y, s_list, s_cnt, geo.act_lists);
+    nact = active_share<PB>(st, gate, B, s_list, s_cnt, geo.act_lists);
   } else {
     const int b = tl.prob >= 0 ? tl.prob : (int)blockIdx.y;
     nact = gate_ok(st[b], gate) ? 1 : 0;
@@ -204,14 +214,16 @@ __global__ void __launch_bounds__(256, 2)
         cp_async_cell<T>(w + (v / kImWin) * LD + v % kImWin, gr + max(cell[i], 0), cell[i] >= 0);
     }
   };
-  stage(0, 0);
-  cp_async_commit();
-  // chi^2 slots beyond this problem's tiles: zero
+  for (int i = 0; i < (PB > 1 ? kImBuf - 1 : 1); ++i) {
+    if (i < nact) stage(i, i);
+    cp_async_commit();
+  }
+  // chi^2 slots beyond this problem's: zero
   if ((int)threadIdx.x < nact && qchi >= 0)
-    for (int sl = tl.slot + tl.ntiles; sl < nslots; sl += tl.ntiles) part.at(qchi, s_list[threadIdx.x])[sl] = 0.0;
+    for (int sl = tl.nslot + tl.item; sl < nslots; sl += tl.nitem) part.at(qchi, s_list[threadIdx.x])[sl] = 0.0;
 
-  // warps over (unit of 16 points, row group): nu units, ng groups of rows
-  const int nu = max(1, (tl.count + 15) >> 4), ng = 8 / nu;
+  // warps over (unit of 16 points, row groups): nu units, ng warps a unit
+  const int nu = max(1, (tl.count + 15) >> 4), ng = nu > 4 ? 1 : nu > 2 ? 2 : 4;
   const int unit = warp % nu, grp = warp / nu;
   const bool on = grp < ng;
   const int p0 = tl.start + unit * 16;
@@ -253,47 +265,50 @@ __global__ void __launch_bounds__(256, 2)
     if ((g & 1) && half_col(tl.col0 + c, ny) < 0) u.mir |= 1u << kk;
   }
   u.mixed = __any_sync(all, u.mir != 0);
-  const int per = (ns + ng - 1) / ng;
-  const int s0 = grp * per, s1 = on ? min(ns, s0 + per) : 0;
+  const int q0 = grp * (4 / ng), q1 = on ? q0 + 4 / ng : q0;
   for (int i = 0; i < nact; ++i) {
-    if (PB > 1 && i + 1 < nact) stage(i + 1, (i + 1) & 1);
-    if (PB > 1) cp_async_commit();
-    if (PB > 1) cp_async_wait<1>();
+    if (PB > 1) cp_async_wait<kImBuf - 2>();
     else cp_async_wait<0>();
-    __syncthreads();  // window i has landed for every thread
-    const T* w = reinterpret_cast<const T*>(win + (size_t)(PB > 1 ? (i & 1) : 0) * kImWin * LD + clo);
-    double y0[2] = {0.0, 0.0}, y1[2] = {0.0, 0.0};
-    if (s0 < s1) {
-      if (two) interp_unit<true, T, LD>(u, nk, w, rlo, s0, s1, lane, y0, y1);
-      else interp_unit<false, T, LD>(u, nk, w, rlo, s0, s1, lane, y0, y1);
+    __syncthreads();  // window i has landed for every thread, and everyone is done with window i - 1
+    if (PB > 1) {
+      if (i + kImBuf - 1 < nact) stage(i + kImBuf - 1, (i + kImBuf - 1) % kImBuf);
+      cp_async_commit();
     }
-    // over the four rows of a step (lanes t)
-#pragma unroll
-    for (int o = 1; o <= 2; o <<= 1) {
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        y0[q] += __shfl_xor_sync(all, y0[q], o);
-        y1[q] += __shfl_xor_sync(all, y1[q], o);
+    const T* w = reinterpret_cast<const T*>(win + (size_t)(PB > 1 ? i % kImBuf : 0) * kImWin * LD + clo);
+    double tot = 0.0, even = 0.0;
+    for (int q = q0; q < q1; ++q) {
+      double y0[2] = {0.0, 0.0}, y1[2] = {0.0, 0.0};
+      const int s0 = kImGroup * q, s1 = min(ns, s0 + kImGroup);
+      if (s0 < s1) {
+        if (two) interp_unit<true, T, LD>(u, nk, w, rlo, s0, s1, lane, y0, y1);
+        else interp_unit<false, T, LD>(u, nk, w, rlo, s0, s1, lane, y0, y1);
       }
+      // over the four rows of a step (lanes t): lane t ends with component
+      // t & 1 of point g + 8 (t >> 1)
+      const bool im = (t & 1) != 0, hi = (t & 2) != 0;
+      const double m0 = (im ? y0[1] : y0[0]) + __shfl_xor_sync(all, im ? y0[0] : y0[1], 1);
+      const double m1 = (im ? y1[1] : y1[0]) + __shfl_xor_sync(all, im ? y1[0] : y1[1], 1);
+      const double v = (hi ? m1 : m0) + __shfl_xor_sync(all, hi ? m0 : m1, 2);
+      if (ng == 4) tot = v;
+      else if (q & 1) tot += even + v;  // (groups 0 + 1) + (groups 2 + 3)
+      else even = v;
     }
-    if (on && t < 2) {
-      const double2 v = t == 0 ? make_double2(y0[0], y0[1]) : make_double2(y1[0], y1[1]);
-      s_red[(i * 8 + warp) * 16 + 8 * t + g] = v;
-    }
-    if (PB > 1) __syncthreads();  // the buffer just read is refilled by the copies issued next
+    if (on) s_red[((i * 8 + warp) * 16 + 8 * (t >> 1) + g) * 2 + (t & 1)] = tot;
   }
-  if (PB == 1) __syncthreads();
-  // residual, chi^2 and models: a warp per problem, lanes over the points
-  for (int i = warp; i < nact; i += 8) {
+  __syncthreads();
+  // residual, chi^2 and models: a warp per (problem, 32 points)
+  const int nq = (nu + 1) >> 1;
+  for (int e0 = warp; e0 < nact * nq; e0 += 8) {
+    const int i = e0 / nq, j0 = 32 * (e0 - i * nq);
     const int b = s_list[i];
+    const int j = j0 + lane;
     double chi = 0.0;
-    for (int j = lane; j < tl.count; j += 32) {
-      double fr = 0.0, fi = 0.0;
-      for (int q = 0; q < ng; ++q) {  // row groups in order
-        const double2 v = s_red[(i * 8 + (j >> 4) + q * nu) * 16 + (j & 15)];
-        fr += v.x;
-        fi += v.y;
-      }
+    if (j < tl.count) {
+      const double2* v = reinterpret_cast<const double2*>(s_red) + (i * 8 + (j >> 4)) * 16 + (j & 15);
+      double2 f = v[0];
+      if (ng == 2) f = im_add(f, v[nu * 16]);
+      if (ng == 4) f = im_add(im_add(f, v[nu * 16]), im_add(v[2 * nu * 16], v[3 * nu * 16]));
+      double fr = f.x, fi = f.y;
       const int k = perm[tl.start + j].x;
       const size_t e = (size_t)b * geo.y2_bstride + k;
       fr *= inv_mm;
@@ -306,11 +321,11 @@ __global__ void __launch_bounds__(256, 2)
       if (ax_out) ax_out[e] = make_double2(fr, fi);
       const double wgt = geo.weight[k];
       const double rr = (geo.vis_r[k] - fr) * wgt, ri = (geo.vis_i[k] - fi) * wgt;
-      chi += rr * rr + ri * ri;
+      chi = rr * rr + ri * ri;
       if (y2) y2[e] = mk<T>((T)(rr * wgt), (T)(ri * wgt));
     }
     chi = warp_sum(chi);
-    if (lane == 0 && qchi >= 0) part.at(qchi, b)[tl.slot] = chi;
+    if (lane == 0 && qchi >= 0) part.at(qchi, b)[tl.slot + (j0 >> 5)] = chi;
   }
 }
 

@@ -324,7 +324,7 @@ template <typename T> struct NufftOp : Op {
   bool interp_mma = false, spread_mma = false;
   DevMem d_im, d_imperm, d_smitems, d_smlist, d_smscratch, d_smtickets;
   DevMem d_wxd, d_wyd;  // FP64 weights of an FP32 operator (wxd(), wyd())
-  int nim = 0, nsm = 0, sm_cols = 0;
+  int nim = 0, im_chunks = 1, nsm = 0, sm_cols = 0;
   // chi^2 partial slots every interpolation kernel of this operator writes
   // (at least its own CTA count; the extra CTAs write zeros), so that the
   // CUDA-core, tensor-core and FP64 kernels fill the same slots
@@ -531,9 +531,17 @@ template <typename T> struct NufftOp : Op {
     std::vector<int2> perm;
     std::vector<Key> keys;
     const int ngeo = shared ? 1 : B;
-    int most = 1;
+    int most = 1, im_pts = kImPts;
     auto first = [](int m) { return (long long)std::max(-(1 << 28), std::min(1 << 28, m)) - (kMSP - 1); };
     auto fdiv = [](long long a) { return a >= 0 ? a / kImTile : -((-a + kImTile - 1) / kImTile); };
+    auto items = [&](int pts) {
+      int n = 0;
+      for (size_t i = 0, j; i < keys.size(); i = j) {
+        for (j = i; j < keys.size() && keys[j].tile == keys[i].tile;) ++j;
+        n += cdiv((int)(j - i), pts);
+      }
+      return n;
+    };
     for (int g = 0; g < ngeo; ++g) {
       keys.clear();
       for (int k = lo[g]; k < hi[g]; ++k) {
@@ -545,39 +553,67 @@ template <typename T> struct NufftOp : Op {
       std::sort(keys.begin(), keys.end(), [](const Key& a, const Key& b) {
         return a.tile != b.tile ? a.tile < b.tile : a.sub != b.sub ? a.sub < b.sub : a.k < b.k;
       });
+      // Points per CTA, shared points (the sums do not depend on it).  Small
+      // CTAs fill the chip when there is little work and even out the load;
+      // large ones stage fewer windows.  Microseconds per iteration with 32 /
+      // 64 / 128: 64 x 64, 1 problem 93 / 102 / 107; 128 x 128, 4 problems
+      // 136 / 128 / 137; 16 problems 218 / 203 / 217; 256 x 256, 32 problems
+      // 338 / 328 / 323.  Points of their own (a window for every CTA): 103 /
+      // 78 / 66 us the launch at 16 frames of 128 x 128.
+      if (shared) {
+        const long long n64 = (long long)items(64) * B;
+        im_pts = n64 < 200 ? 32 : n64 < 8000 ? 64 : kImPts;
+      }
       const size_t t0 = tiles.size();
+      int slots = 0;
       for (size_t i = 0; i < keys.size();) {
         size_t j = i;
         while (j < keys.size() && keys[j].tile == keys[i].tile) ++j;
         const int k0 = keys[i].k;
         const long long tx = fdiv(first(mx[k0])), ty = fdiv(first(my[k0]));
-        for (size_t a = i; a < j; a += kImPts)
-          tiles.push_back(ImTileItem{(int)(tx * kImTile), (int)(ty * kImTile), (int)(perm.size() + (a - i)),
-                                     (int)std::min<size_t>(kImPts, j - a), shared ? -1 : g, 0, 0, 0});
+        for (size_t a = i; a < j; a += im_pts) {
+          const int cnt = (int)std::min<size_t>(im_pts, j - a);
+          tiles.push_back(ImTileItem{(int)(tx * kImTile), (int)(ty * kImTile), (int)(perm.size() + (a - i)), cnt,
+                                     shared ? -1 : g, slots, 0, 0, 0});
+          slots += cdiv(cnt, 32);
+        }
         for (size_t a = i; a < j; ++a) {
           const int sub = keys[a].sub;
           perm.push_back(make_int2(keys[a].k, ((sub >> 4) & 15) | ((sub & 15) << 8)));
         }
         i = j;
       }
-      if (tiles.size() == t0) tiles.push_back(ImTileItem{0, 0, 0, 0, shared ? -1 : g, 0, 0, 0});
+      if (tiles.size() == t0) {
+        tiles.push_back(ImTileItem{0, 0, 0, 0, shared ? -1 : g, 0, 0, 0, 0});
+        slots = 1;
+      }
       const int nt = (int)(tiles.size() - t0);
       for (int q = 0; q < nt; ++q) {
-        tiles[t0 + q].slot = q;
-        tiles[t0 + q].ntiles = nt;
+        tiles[t0 + q].nslot = slots;
+        tiles[t0 + q].item = q;
+        tiles[t0 + q].nitem = nt;
       }
-      most = std::max(most, nt);
+      most = std::max(most, slots);
     }
     // launch order: fullest CTAs first, so that the last wave holds short ones
     std::stable_sort(tiles.begin(), tiles.end(),
                      [](const ImTileItem& a, const ImTileItem& b) { return a.count > b.count; });
     nim = (int)tiles.size();
+    // Problems per CTA: as many as leave two CTAs for each SM.  More share the
+    // weights and the set-up; fewer balance (100 x 100, 11 problems: 190 us
+    // an iteration with 8 or 6, 172 with 4, 166 with 3, 167 with 2, 181 with 1)
+    im_chunks = 1;
+    if (shared)
+      for (int c = kImProb; c >= 1; --c) {
+        im_chunks = cdiv(B, c);
+        if ((long long)nim * im_chunks >= 320) break;
+      }
     chi_pad = std::max(chi_pad, most);
     if (perm.empty()) perm.push_back(make_int2(0, 0));
     d_im.upload(tiles.data(), tiles.size());
     d_imperm.upload(perm.data(), perm.size());
     set_smem(k_nufft_interp_mma<T, 1>, im_smem<T, 1>());
-    set_smem(k_nufft_interp_mma<T, kMmaProb>, im_smem<T, kMmaProb>());
+    set_smem(k_nufft_interp_mma<T, kImProb>, im_smem<T, kImProb>());
   }
 
   // k_nufft_spread_mma's tiles and lists: per stored tile the virtual points
@@ -666,7 +702,7 @@ template <typename T> struct NufftOp : Op {
   }
   // problems per CTA of the two: one where each problem has its own points
   // or the batch is a single problem, else chunks of 8
-  static constexpr int kMmaProb = 8;
+  static constexpr int kMmaProb = 8, kImProb = 6;
   int mma_prob() const { return shared && B > 1 ? kMmaProb : 1; }
   int mma_chunks() const { return shared ? cdiv(B, mma_prob()) : 1; }
 
@@ -805,13 +841,13 @@ template <typename T> struct NufftOp : Op {
                      double2* out = nullptr) {
     const NufftGeom<T> geo = geo_now();
     if (interp_mma) {
-      const dim3 grid(nim, mma_chunks());
+      const dim3 grid(nim, im_chunks);
       if (mma_prob() == 1)
         k_nufft_interp_mma<T, 1><<<grid, 256, im_smem<T, 1>(), s>>>(
             geo, wxd(), wyd(), d_im.as<ImTileItem>(), d_imperm.as<int2>(), g, gstride, nx, ny, inv_mm, c.st, gate, c.part,
             qchi, chi_slots(), y2, B, base, out);
       else
-        k_nufft_interp_mma<T, kMmaProb><<<grid, 256, im_smem<T, kMmaProb>(), s>>>(
+        k_nufft_interp_mma<T, kImProb><<<grid, 256, im_smem<T, kImProb>(), s>>>(
             geo, wxd(), wyd(), d_im.as<ImTileItem>(), d_imperm.as<int2>(), g, gstride, nx, ny, inv_mm, c.st, gate, c.part,
             qchi, chi_slots(), y2, B, base, out);
       MF_LAUNCH_CK();

@@ -80,3 +80,18 @@ def test_batches_match_tap_by_tap(gpulib, shared, b):
     x, y = run(), _taps(run)
     assert np.linalg.norm(x) > 0
     assert rel(x, y) < 1e-10  # four steps of operators that agree to 1e-12
+
+
+@pytest.mark.parametrize("name,b", [("dense", 24), ("uniform", 20)])
+def test_cut_of_points_keeps_bits(gpulib, name, b):
+    """One problem alone (32 or 64 points per interpolation CTA) and in a batch
+    large enough for the next size (64 or 128) and several chunks: same bits."""
+    u, v, nx = _points(name)
+    rng = np.random.default_rng(3)
+    data = (u, v, rng.standard_normal(u.size), rng.standard_normal(u.size), np.full(u.size, 2.0))
+    probs = [dict(lambda_l1=0.02 * (k + 1), lambda_tsv=0.01, cinit=1e7, maxiter=3, nonneg_flag=0) for k in range(b)]
+    x = gpulib.nufft_batch(*data, nx, nx, probs, 0.0)[0]
+    for k in (0, b - 1):
+        alone = gpulib.nufft_batch(*data, nx, nx, [probs[k]], 0.0)[0]
+        assert np.linalg.norm(x[k]) > 0
+        np.testing.assert_array_equal(alone[0], x[k])
