@@ -58,7 +58,7 @@ __device__ __forceinline__ void cp_async_cell(cplx<T>* dst, const cplx<T>* src, 
 // as m8n8k4 products: A = wy (in registers for all problems), B = the window's
 // cells (one 8-byte shared load per lane serves both blocks of 8 points), so
 // nothing of a matrix tile is idle for a single problem.  Only the rows and
-// columns that the 16 points reach are walked, in up to four row groups whose
+// columns that the 16 points reach are walked, in four row groups whose
 // sums are added as (0 + 1) + (2 + 3); a CTA with few points gives its warps
 // one or two groups each.  Bound by the FP64 pipe where the chip is full and
 // by the length of one CTA's chain where it is not, so the points per CTA
@@ -68,8 +68,8 @@ __device__ __forceinline__ void cp_async_cell(cplx<T>* dst, const cplx<T>* src, 
 // with one (93).
 // Signs: the reference negates the imaginary part of direct taps (NU_SIGN) and
 // keeps that of mirrored ones; a tap is direct or mirrored by its column alone,
-// so the imaginary parts of mirrored columns are flipped at the fragment and
-// the sum is negated once.
+// so the imaginary parts of mirrored columns are flipped at the fragment (at
+// the sum, when all columns of the unit are) and the sum is negated once.
 // A problem's sums depend neither on its CTA's points nor on the other
 // problems: groups and chi^2 slots (32 points) are the same for every cut.
 // ---------------------------------------------------------------------------
@@ -77,7 +77,6 @@ constexpr int kImTile = 16;
 constexpr int kImWin = kImTile + kTaps;  // 40: 39 used, a multiple of 4
 constexpr int kImPts = 128;              // points per CTA at most: 8 warps x 16
 constexpr int kImSteps = kImWin / 4;     // column steps of 4
-constexpr int kImGroup = 3;              // row steps of 4 per row group: at most four groups
 
 struct ImTileItem {
   int row0, col0;    // window origin, virtual
@@ -93,7 +92,7 @@ template <typename T> struct ImWindow {
   static constexpr size_t kBytes = sizeof(cplx<T>) * (size_t)kImWin * kLd;
 };
 constexpr size_t im_red_bytes(int pb) { return sizeof(double2) * (size_t)pb * 8 * 16; }
-constexpr int kImBuf = 3;  // staged windows in flight
+constexpr int kImBuf = 2;   // staged windows
 template <typename T, int PB> constexpr size_t im_smem() {
   return (PB > 1 ? kImBuf : 1) * ImWindow<T>::kBytes + im_red_bytes(PB);
 }
@@ -118,6 +117,7 @@ template <int NK, bool TWO, typename T, int LD>
 __device__ __forceinline__ void interp_rows(const ImUnit& u, const T* w, int rlo, int s0, int s1, int lane,
                                             double (&y0)[2], double (&y1)[2]) {
   const int g = lane >> 2, t = lane & 3;
+#pragma unroll 1
   for (int s = s0; s < s1; ++s) {
     const int r = rlo + 4 * s;
     const int ja = r + t - u.dra, jb = r + t - u.drb;
@@ -244,6 +244,7 @@ __global__ void __launch_bounds__(256, 2)
   // rows and columns of the window that the unit's points reach, in steps of 4
   int rlo = __reduce_min_sync(all, lane < np ? drq : kImWin), rhi = __reduce_max_sync(all, lane < np ? drq + kTaps : 0);
   int clo = __reduce_min_sync(all, lane < np ? dcq : kImWin), chi_ = __reduce_max_sync(all, lane < np ? dcq + kTaps : 0);
+  if (np == 0) rlo = rhi = clo = chi_ = 0;
   const int ns = (rhi - rlo + 3) >> 2, nk = (chi_ - clo + 3) >> 2;
   rlo = min(rlo, kImWin - 4 * ns);
   clo = min(clo, kImWin - 4 * nk);
@@ -264,7 +265,11 @@ __global__ void __launch_bounds__(256, 2)
     u.a1[kk] = (vb && kk < nk && jb >= 0 && jb < kTaps) ? wyd[(size_t)kb * kTaps + jb] : 0.0;
     if ((g & 1) && half_col(tl.col0 + c, ny) < 0) u.mir |= 1u << kk;
   }
-  u.mixed = __any_sync(all, u.mir != 0);
+  // mirrored as a whole (lanes of imaginary cells agree on all columns): the
+  // sign goes to the sum
+  const unsigned int cols = (1u << nk) - 1u;
+  const bool flip = __all_sync(all, !(g & 1) || (u.mir & cols) == cols);
+  u.mixed = !flip && __any_sync(all, (u.mir & cols) != 0);
   const int q0 = grp * (4 / ng), q1 = on ? q0 + 4 / ng : q0;
   for (int i = 0; i < nact; ++i) {
     if (PB > 1) cp_async_wait<kImBuf - 2>();
@@ -278,8 +283,8 @@ __global__ void __launch_bounds__(256, 2)
     double tot = 0.0, even = 0.0;
     for (int q = q0; q < q1; ++q) {
       double y0[2] = {0.0, 0.0}, y1[2] = {0.0, 0.0};
-      const int s0 = kImGroup * q, s1 = min(ns, s0 + kImGroup);
-      if (s0 < s1) {
+      const int s0 = (q * ns) >> 2, s1 = ((q + 1) * ns) >> 2;  // 6 row steps at least
+      {
         if (two) interp_unit<true, T, LD>(u, nk, w, rlo, s0, s1, lane, y0, y1);
         else interp_unit<false, T, LD>(u, nk, w, rlo, s0, s1, lane, y0, y1);
       }
@@ -288,7 +293,8 @@ __global__ void __launch_bounds__(256, 2)
       const bool im = (t & 1) != 0, hi = (t & 2) != 0;
       const double m0 = (im ? y0[1] : y0[0]) + __shfl_xor_sync(all, im ? y0[0] : y0[1], 1);
       const double m1 = (im ? y1[1] : y1[0]) + __shfl_xor_sync(all, im ? y1[0] : y1[1], 1);
-      const double v = (hi ? m1 : m0) + __shfl_xor_sync(all, hi ? m0 : m1, 2);
+      double v = (hi ? m1 : m0) + __shfl_xor_sync(all, hi ? m0 : m1, 2);
+      if (im && flip) v = -v;
       if (ng == 4) tot = v;
       else if (q & 1) tot += even + v;  // (groups 0 + 1) + (groups 2 + 3)
       else even = v;
@@ -338,8 +344,11 @@ __global__ void __launch_bounds__(256, 2)
 //   D[(row, re/im)][col] = sum_p (wx_p[row] y_p[re/im]) wy_p[col],
 // four rows x {re, im} by eight columns, K = points, so a single problem fills
 // the matrix tile.  A CTA takes up to kSmSeg list entries and up to PB
-// problems: its warps go over (problem, block) and, with one problem, over the
-// even and odd steps of 4 points too.  Each block's sum is the even steps'
+// problems: its warps go over (pair of problems, blocks, even or odd steps of
+// 4 points).  A pair shares a warp's weights and their index arithmetic, and
+// with half of the steps a warp needs few enough registers for three CTAs an
+// SM: 146 us at 128 x 128 with 64 problems, against 199 with a problem and
+// both parities to a warp and two CTAs.  Each block's sum is the even steps'
 // plus the odd steps' whatever the mapping, and longer lists are cut into
 // segments whose partial tiles the tile's last CTA adds in segment order, so
 // neither the batch nor the order of the CTAs changes a result.
@@ -364,17 +373,20 @@ struct SmPoint {
   int fl;      // mirrored
 };
 
+// (the exchange of the parities' sums reuses the residuals' space)
+constexpr size_t sm_exchange(int pb) { return sizeof(double) * 64 * (pb > 1 ? 8 * 4 : 8); }
 template <typename T, int PB> constexpr size_t sm_smem() {
-  return (size_t)kSmSeg * sizeof(SmPoint) + sizeof(double2) * (size_t)PB * kSmSeg + sizeof(double) * 4 * 64;
+  const size_t y = sizeof(double2) * (size_t)PB * kSmSeg;
+  return (size_t)kSmSeg * sizeof(SmPoint) + (y > sm_exchange(PB) ? y : sm_exchange(PB));
 }
 
-// the products of the warp's MB x NB blocks (from mb0, nb0) over its CH step
-// parities (from ch0)
-template <int MB, int NB, int CH>
-__device__ __forceinline__ void spread_products(const SmPoint* s_pt, const double* s_yp, int count, int mb0, int nb0,
+// the products of NP problems' MB x NB blocks (from mb0, nb0) over the steps
+// of parity ch0; problem p's residuals at s_yp + p kSmSeg
+template <int MB, int NB, int NP>
+__device__ __forceinline__ void spread_products(const SmPoint* s_pt, const double2* s_yp, int count, int mb0, int nb0,
                                                 int ch0, int row_base, int col_base, int nx, int ny, int lane,
                                                 const double* __restrict__ wxd, const double* __restrict__ wyd,
-                                                double (&acc)[CH][MB][NB][2]) {
+                                                double (&d)[2][4][2]) {
   const int g = lane >> 2, t = lane & 3;
   constexpr int kOut = 1 << 28;  // no tap reaches it
   int mr[MB], mc[NB];
@@ -388,40 +400,37 @@ __device__ __forceinline__ void spread_products(const SmPoint* s_pt, const doubl
     const int col = col_base + 8 * (nb0 + n) + g;
     mc[n] = col < ny ? col : col == ny ? -ny : kOut;
   }
+  const SmPoint* pt = s_pt + 4 * ch0 + t;
+  const double* yp = reinterpret_cast<const double*>(s_yp + 4 * ch0 + t) + (g & 1);
+#pragma unroll 4
+  for (int e = 0; e < count; e += 8) {
+    const SmPoint p = pt[e];
+    double a[MB], b[NB];
 #pragma unroll
-  for (int c = 0; c < CH; ++c)
+    for (int m = 0; m < MB; ++m) {
+      const int j = mr[m] - p.x0;
+      a[m] = (unsigned)j < (unsigned)kTaps ? __ldg(wxd + p.k24 + (p.fl ? kTaps - 1 - j : j)) : 0.0;
+    }
 #pragma unroll
-    for (int m = 0; m < MB; ++m)
+    for (int n = 0; n < NB; ++n) {
+      const int j = mc[n] - p.y0;
+      b[n] = (unsigned)j < (unsigned)kTaps ? __ldg(wyd + p.k24 + (p.fl ? kTaps - 1 - j : j)) : 0.0;
+    }
 #pragma unroll
-      for (int n = 0; n < NB; ++n) acc[c][m][n][0] = acc[c][m][n][1] = 0.0;
-#pragma unroll 2
-  for (int e0 = 0; e0 < count; e0 += 8) {
-#pragma unroll
-    for (int c = 0; c < CH; ++c) {
-      const int e = e0 + 4 * (ch0 + c) + t;
-      const SmPoint p = s_pt[e];
-      const double y = s_yp[2 * e + (g & 1)];
-      double a[MB], b[NB];
+    for (int q = 0; q < NP; ++q) {
+      const double y = yp[2 * (q * kSmSeg + e)];
 #pragma unroll
       for (int m = 0; m < MB; ++m) {
-        const int j = mr[m] - p.x0;
-        a[m] = (unsigned)j < (unsigned)kTaps ? __ldg(wxd + p.k24 + (p.fl ? kTaps - 1 - j : j)) * y : 0.0;
+        const double ay = a[m] * y;
+#pragma unroll
+        for (int n = 0; n < NB; ++n) dmma_884(d[q][m * NB + n], ay, b[n]);
       }
-#pragma unroll
-      for (int n = 0; n < NB; ++n) {
-        const int j = mc[n] - p.y0;
-        b[n] = (unsigned)j < (unsigned)kTaps ? __ldg(wyd + p.k24 + (p.fl ? kTaps - 1 - j : j)) : 0.0;
-      }
-#pragma unroll
-      for (int m = 0; m < MB; ++m)
-#pragma unroll
-        for (int n = 0; n < NB; ++n) dmma_884(acc[c][m][n], a[m], b[n]);
     }
   }
 }
 
 template <typename T, int PB>
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(256, PB > 1 ? 3 : 2)
     k_nufft_spread_mma(NufftGeom<T> geo, const double* __restrict__ wxd, const double* __restrict__ wyd,
                        const SmItem* __restrict__ items, const unsigned int* __restrict__ vlist,
                        const cplx<T>* __restrict__ y2, cplx<T>* __restrict__ gall, long gstride, int nx, int ny,
@@ -430,14 +439,14 @@ __global__ void __launch_bounds__(256, 2)
   extern __shared__ __align__(16) unsigned char sm_smem_raw[];
   SmPoint* s_pt = reinterpret_cast<SmPoint*>(sm_smem_raw);
   double2* s_y = reinterpret_cast<double2*>(sm_smem_raw + (size_t)kSmSeg * sizeof(SmPoint));  // [PB][kSmSeg]
-  double* s_ex = reinterpret_cast<double*>(s_y + (size_t)PB * kSmSeg);                        // [4 blocks][64]
+  double* s_ex = reinterpret_cast<double*>(s_y);  // [warp][block][64], after the products
   __shared__ int s_list[PB];
   __shared__ int s_cnt[8];
   __shared__ unsigned int s_ticket;
   const SmItem it = items[blockIdx.x];
   int nact;
   if (PB > 1) {
-    nact = active_chunk<PB>(st, gate, B, blockIdx.y, s_list, s_cnt, geo.act_lists);
+    nact = active_share<PB>(st, gate, B, s_list, s_cnt, geo.act_lists);
   } else {
     const int b = it.prob >= 0 ? it.prob : (int)blockIdx.y;
     nact = gate_ok(st[b], gate) ? 1 : 0;
@@ -471,61 +480,62 @@ __global__ void __launch_bounds__(256, 2)
     }
   }
   __syncthreads();
-  // warps over (problem, block of the tile): the more warps a problem gets,
-  // the fewer blocks each takes
-  const int wpp = nact > 4 ? 1 : nact > 2 ? 2 : nact > 1 ? 4 : 8;  // warps per problem
-  const int prob = warp / wpp, sub = warp - prob * wpp;
-  const bool on = prob < nact;
-  const double* yp = reinterpret_cast<const double*>(s_y + (size_t)(on ? prob : 0) * kSmSeg);
-  const int count = on ? it.count : 0;
-  double d[4][2];  // blocks 2 mb + nb of the tile held by this warp: [blk0, blk0 + nblk)
-  int blk0 = 0, nblk = 0;
-  if (PB > 1 && wpp == 1) {
-    double acc[2][2][2][2];
-    spread_products<2, 2, 2>(s_pt, yp, count, 0, 0, 0, row_base, col_base, nx, ny, lane, wxd, wyd, acc);
+  // warps over (pair of problems, blocks of the tile, parity of the steps):
+  // the fewer pairs, the fewer blocks a warp takes
+  const int ch = warp & 1, groups = nact > 4 ? 1 : nact > 2 ? 2 : 4;
+  const int pair = (warp >> 1) / groups, sub = (warp >> 1) - pair * groups;
+  const int nblk_w = 4 / groups, blk0 = sub * nblk_w;
+  const int np = min(2, nact - 2 * pair);  // problems of the warp (< 1: none)
+  double acc[2][4][2];
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
+  for (int q = 0; q < 2; ++q)
 #pragma unroll
-      for (int h = 0; h < 2; ++h) d[q][h] = acc[0][q >> 1][q & 1][h] + acc[1][q >> 1][q & 1][h];
-    nblk = 4;
-  } else if (PB > 1 && wpp == 2) {
-    double acc[2][1][2][2];
-    spread_products<1, 2, 2>(s_pt, yp, count, sub, 0, 0, row_base, col_base, nx, ny, lane, wxd, wyd, acc);
-#pragma unroll
-    for (int q = 0; q < 2; ++q)
-#pragma unroll
-      for (int h = 0; h < 2; ++h) d[q][h] = acc[0][0][q][h] + acc[1][0][q][h];
-    blk0 = 2 * sub;
-    nblk = 2;
-  } else if (PB > 1 && wpp == 4) {
-    double acc[2][1][1][2];
-    spread_products<1, 1, 2>(s_pt, yp, count, sub >> 1, sub & 1, 0, row_base, col_base, nx, ny, lane, wxd, wyd, acc);
-#pragma unroll
-    for (int h = 0; h < 2; ++h) d[0][h] = acc[0][0][0][h] + acc[1][0][0][h];
-    blk0 = sub;
-    nblk = 1;
+    for (int m = 0; m < 4; ++m) acc[q][m][0] = acc[q][m][1] = 0.0;
+  const double2* yp = s_y + (size_t)2 * pair * kSmSeg;
+  if (PB > 1 && groups == 1) {
+    if (np == 2)
+      spread_products<2, 2, 2>(s_pt, yp, it.count, 0, 0, ch, row_base, col_base, nx, ny, lane, wxd, wyd, acc);
+    else if (np == 1)
+      spread_products<2, 2, 1>(s_pt, yp, it.count, 0, 0, ch, row_base, col_base, nx, ny, lane, wxd, wyd, acc);
+  } else if (PB > 1 && groups == 2) {
+    if (np == 2)
+      spread_products<1, 2, 2>(s_pt, yp, it.count, sub, 0, ch, row_base, col_base, nx, ny, lane, wxd, wyd, acc);
+    else if (np == 1)
+      spread_products<1, 2, 1>(s_pt, yp, it.count, sub, 0, ch, row_base, col_base, nx, ny, lane, wxd, wyd, acc);
   } else {
-    double acc[1][1][1][2];
-    const int blk = sub & 3;
-    spread_products<1, 1, 1>(s_pt, yp, count, blk >> 1, blk & 1, sub >> 2, row_base, col_base, nx, ny, lane, wxd, wyd,
-                             acc);
-    if (sub >> 2) {
-      s_ex[blk * 64 + 2 * lane] = acc[0][0][0][0];
-      s_ex[blk * 64 + 2 * lane + 1] = acc[0][0][0][1];
-    }
-    __syncthreads();  // (uniform: nact == 1)
-    blk0 = blk;
-    nblk = (sub >> 2) ? 0 : 1;
-#pragma unroll
-    for (int h = 0; h < 2; ++h) d[0][h] = acc[0][0][0][h] + s_ex[blk * 64 + 2 * lane + h];
+    if (PB > 1 && np == 2)
+      spread_products<1, 1, 2>(s_pt, yp, it.count, sub >> 1, sub & 1, ch, row_base, col_base, nx, ny, lane, wxd, wyd,
+                               acc);
+    else if (np == 1)
+      spread_products<1, 1, 1>(s_pt, yp, it.count, sub >> 1, sub & 1, ch, row_base, col_base, nx, ny, lane, wxd, wyd,
+                               acc);
   }
-  if (!on) nblk = 0;
+  // even plus odd steps: warp c of the two parities keeps the pair's problem c
+  // and hands over the other
+  __syncthreads();  // the residuals have been read
+  constexpr int kBlkW = PB > 1 ? 4 : 1;  // blocks per warp at most
+#pragma unroll
+  for (int m = 0; m < kBlkW; ++m)
+    if (m < nblk_w)
+      *reinterpret_cast<double2*>(s_ex + (warp * kBlkW + m) * 64 + 2 * lane) =
+          ch ? make_double2(acc[0][m][0], acc[0][m][1]) : make_double2(acc[1][m][0], acc[1][m][1]);
+  __syncthreads();
+  const int prob = 2 * pair + ch;
+  const int nblk = prob < nact ? nblk_w : 0;
+  double d[4][2];  // the problem's blocks 2 mb + nb: [blk0, blk0 + nblk)
+#pragma unroll
+  for (int m = 0; m < kBlkW; ++m)
+    if (m < nblk) {
+      const double2 v = *reinterpret_cast<const double2*>(s_ex + ((warp ^ 1) * kBlkW + m) * 64 + 2 * lane);
+      d[m][0] = (ch ? acc[1][m][0] : acc[0][m][0]) + v.x;
+      d[m][1] = (ch ? acc[1][m][1] : acc[0][m][1]) + v.y;
+    }
   constexpr int kPart = 4 * 64;  // doubles of one problem's tile
   if (it.nseg > 1) {
     const size_t cs = (size_t)gridDim.y * PB * kPart;
     double* mine = scratch + (size_t)(it.scratch + it.seg) * cs + ((size_t)blockIdx.y * PB + prob) * kPart;
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
+    for (int q = 0; q < kBlkW; ++q)
       if (q < nblk) *reinterpret_cast<double2*>(mine + (blk0 + q) * 64 + 2 * lane) = make_double2(d[q][0], d[q][1]);
     __threadfence();
     __syncthreads();
@@ -534,11 +544,11 @@ __global__ void __launch_bounds__(256, 2)
     if (s_ticket != (unsigned int)(it.nseg - 1)) return;
     __threadfence();
 #pragma unroll
-    for (int q = 0; q < 4; ++q) d[q][0] = d[q][1] = 0.0;
+    for (int q = 0; q < kBlkW; ++q) d[q][0] = d[q][1] = 0.0;
     for (int sg = 0; sg < it.nseg; ++sg) {
       const double* p = scratch + (size_t)(it.scratch + sg) * cs + ((size_t)blockIdx.y * PB + prob) * kPart;
 #pragma unroll
-      for (int q = 0; q < 4; ++q)
+      for (int q = 0; q < kBlkW; ++q)
         if (q < nblk) {
           const double2 v = __ldcg(reinterpret_cast<const double2*>(p + (blk0 + q) * 64 + 2 * lane));
           d[q][0] += v.x;
@@ -553,7 +563,7 @@ __global__ void __launch_bounds__(256, 2)
   const int g = lane >> 2, t = lane & 3;
   cplx<T>* gr = gall + (size_t)s_list[prob] * gstride;
 #pragma unroll
-  for (int q = 0; q < 4; ++q)
+  for (int q = 0; q < kBlkW; ++q)
     if (q < nblk) {
       const double other = __shfl_xor_sync(0xffffffffu, (g & 1) ? d[q][0] : d[q][1], 4);
       const double re = (g & 1) ? other : d[q][0], im = (g & 1) ? d[q][1] : other;

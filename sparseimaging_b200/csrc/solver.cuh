@@ -534,6 +534,24 @@ template <typename T> struct NufftOp : Op {
     int most = 1, im_pts = kImPts;
     auto first = [](int m) { return (long long)std::max(-(1 << 28), std::min(1 << 28, m)) - (kMSP - 1); };
     auto fdiv = [](long long a) { return a >= 0 ? a / kImTile : -((-a + kImTile - 1) / kImTile); };
+    // units of 16 points that reach few rows and columns: a tile's points are
+    // halved (at a multiple of 16) along their longer side
+    auto kd = [&](auto&& self, size_t a, size_t b) -> void {
+      if (b - a <= 16) return;
+      int lo[2] = {15, 15}, hi[2] = {0, 0};
+      for (size_t i = a; i < b; ++i) {
+        const int p[2] = {(keys[i].sub >> 4) & 15, keys[i].sub & 15};
+        for (int d = 0; d < 2; ++d) lo[d] = std::min(lo[d], p[d]), hi[d] = std::max(hi[d], p[d]);
+      }
+      const int sh = hi[0] - lo[0] >= hi[1] - lo[1] ? 4 : 0;
+      const size_t m = a + 16 * (((b - a + 15) / 16) / 2);
+      std::nth_element(keys.begin() + a, keys.begin() + m, keys.begin() + b, [sh](const Key& x, const Key& y) {
+        const int p = (x.sub >> sh) & 15, q = (y.sub >> sh) & 15, p2 = (x.sub >> (4 - sh)) & 15, q2 = (y.sub >> (4 - sh)) & 15;
+        return p != q ? p < q : p2 != q2 ? p2 < q2 : x.k < y.k;
+      });
+      self(self, a, m);
+      self(self, m, b);
+    };
     auto items = [&](int pts) {
       int n = 0;
       for (size_t i = 0, j; i < keys.size(); i = j) {
@@ -571,6 +589,7 @@ template <typename T> struct NufftOp : Op {
         while (j < keys.size() && keys[j].tile == keys[i].tile) ++j;
         const int k0 = keys[i].k;
         const long long tx = fdiv(first(mx[k0])), ty = fdiv(first(my[k0]));
+        kd(kd, i, j);
         for (size_t a = i; a < j; a += im_pts) {
           const int cnt = (int)std::min<size_t>(im_pts, j - a);
           tiles.push_back(ImTileItem{(int)(tx * kImTile), (int)(ty * kImTile), (int)(perm.size() + (a - i)), cnt,
