@@ -1,7 +1,7 @@
 // FP64 matrix products on mma.sync m8n8k4.f64: the tile loop shared by the
 // batched DFT operator (dft_ops.cuh) and the leave-one-out error (looe.cuh).
 //
-// A CTA of 128 threads forms a 64 x 64 tile of X Y^T, X and Y given by rows:
+// A CTA of 128 threads (or 256, below) forms a 64 x 64 tile of X Y^T, X and Y given by rows:
 // an operand is stored either with K contiguous (kK) or with its rows
 // contiguous (column-major, !kK).  K runs in steps of 16 through a ring of
 // three shared-memory stages filled by cp.async (zeros outside the matrices);
@@ -43,19 +43,20 @@ __device__ __forceinline__ void copy2(double* dst, const double* src, int n, boo
 // (i, k) at base + i + (size_t)k ld.  A thread keeps its four row pointers.
 // vec: every row start (kK) or line start (!kK) is 16-byte aligned and K
 // ranges and tiles begin at even offsets.
-template <bool kK> struct Operand {
+template <bool kK, int NT = 128> struct Operand {
+  static constexpr int kRows = NT / 8, kLines = NT / 32;  // rows (kK) or K lines (!kK) staged per round
   const double* base;
   size_t ld;
   int i0, n;  // first row of the tile, rows of the matrix
   bool vec;
-  const double* rp[4];
+  const double* rp[kT / kRows];
   unsigned int ok;
 
   __device__ __forceinline__ Operand(const double* b, size_t l, int i0_, int n_, bool v, const int* idx = nullptr)
       : base(b), ld(l), i0(i0_), n(n_), vec(v), ok(0) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int i = i0 + (int)(threadIdx.x >> 3) + 16 * q;
+    for (int q = 0; q < kT / kRows; ++q) {
+      const int i = i0 + (int)(threadIdx.x >> 3) + kRows * q;
       rp[q] = base;
       if (kK && i < n) {
         rp[q] = base + (size_t)(idx ? idx[i] : i) * ld;
@@ -64,16 +65,16 @@ template <bool kK> struct Operand {
     }
   }
 
-  // K [k0, min(k0 + 16, k1)) into a stage; 128 threads
+  // K [k0, min(k0 + 16, k1)) into a stage; NT threads
   __device__ __forceinline__ void stage(double* s, int k0, int k1) const {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < (kK ? kT / kRows : kStep / kLines); ++q) {
       if (kK) {
-        const int r = (int)(threadIdx.x >> 3) + 16 * q, kk = (int)(threadIdx.x & 7) * 2;
+        const int r = (int)(threadIdx.x >> 3) + kRows * q, kk = (int)(threadIdx.x & 7) * 2;
         const int m = ((ok >> q) & 1u) ? max(0, min(2, k1 - k0 - kk)) : 0;
         copy2(s + r * kLdK + kk, m ? rp[q] + k0 + kk : base, m, vec);
       } else {
-        const int kk = (int)(threadIdx.x >> 5) + 4 * q, r = (int)(threadIdx.x & 31) * 2;
+        const int kk = (int)(threadIdx.x >> 5) + kLines * q, r = (int)(threadIdx.x & 31) * 2;
         const int m = k0 + kk < k1 ? max(0, min(2, n - i0 - r)) : 0;
         copy2(s + kk * kLdM + r, m ? base + (size_t)(k0 + kk) * ld + i0 + r : base, m, vec);
       }
@@ -86,14 +87,16 @@ template <bool kK> __device__ __forceinline__ double frag(const double* s, int r
   return kK ? s[r * kLdK + k] : s[k * kLdM + r];
 }
 
-using Acc = double[2][8][2];
+template <int NB> using AccNb = double[2][NB][2];
+using Acc = AccNb<8>;
 
 // acc[mb][nb] += the warp's 16 x 8 NB block of X Y^T over K [k0, k1): the
-// first NB blocks of 8 columns (the rest of the tile is not needed)
-template <int NB, bool kA, bool kB>
-__device__ __forceinline__ void tile_product_nb(const Operand<kA>& X, const Operand<kB>& Y, int k0, int k1, double* smem,
-                                                Acc& acc) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+// first NB blocks of 8 columns (the rest of the tile is not needed), or, with
+// eight warps, blocks 4 (warp / 4) .. + 3
+template <int NB, bool kA, bool kB, int NT, int NA>
+__device__ __forceinline__ void tile_product_nb(const Operand<kA, NT>& X, const Operand<kB, NT>& Y, int k0, int k1,
+                                                double* smem, double (&acc)[2][NA][2]) {
+  const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) & 3, cb = NT > 128 ? (threadIdx.x >> 7) * NB : 0;
   const int g = lane >> 2, t = lane & 3;
   const int ns = (max(0, k1 - k0) + kStep - 1) / kStep;
   auto load = [&](int s) {
@@ -117,7 +120,7 @@ __device__ __forceinline__ void tile_product_nb(const Operand<kA>& X, const Oper
 #pragma unroll
       for (int m = 0; m < 2; ++m) a[m] = frag<kA>(sx, 16 * warp + 8 * m + g, kk + t);
 #pragma unroll
-      for (int j = 0; j < NB; ++j) b[j] = frag<kB>(sy, 8 * j + g, kk + t);
+      for (int j = 0; j < NB; ++j) b[j] = frag<kB>(sy, 8 * (cb + j) + g, kk + t);
 #pragma unroll
       for (int j = 0; j < NB; ++j) {
         dmma_884(acc[0][j], a[0], b[j]);
@@ -141,24 +144,26 @@ __device__ __forceinline__ void tile_product(const Operand<kA>& X, const Operand
   else tile_product_nb<1, kA, kB>(X, Y, k0, k1, smem, acc);
 }
 
-__device__ __forceinline__ void clear(Acc& acc) {
+template <int NB> __device__ __forceinline__ void clear(double (&acc)[2][NB][2]) {
 #pragma unroll
   for (int m = 0; m < 2; ++m)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[m][j][0] = acc[m][j][1] = 0.0;
+    for (int j = 0; j < NB; ++j) acc[m][j][0] = acc[m][j][1] = 0.0;
 }
 
-// f(row, column, value) for the thread's elements of the tile
-template <typename F> __device__ __forceinline__ void each(const Acc& acc, F f) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+// f(row, column, value) for the thread's elements of the tile; the value may
+// be changed where acc is not const
+template <int NB, typename A, typename F> __device__ __forceinline__ void each_of(A& acc, F f) {
+  const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) & 3, cb = NB < 8 ? (threadIdx.x >> 7) * NB : 0;
   const int g = lane >> 2, t = lane & 3;
 #pragma unroll
   for (int m = 0; m < 2; ++m)
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
+    for (int j = 0; j < NB; ++j)
 #pragma unroll
-      for (int h = 0; h < 2; ++h) f(16 * warp + 8 * m + g, 8 * j + 2 * t + h, acc[m][j][h]);
+      for (int h = 0; h < 2; ++h) f(16 * warp + 8 * m + g, 8 * (cb + j) + 2 * t + h, acc[m][j][h]);
 }
+template <typename F> __device__ __forceinline__ void each(const Acc& acc, F f) { each_of<8>(acc, f); }
 
 }  // namespace dg
 }  // namespace mf

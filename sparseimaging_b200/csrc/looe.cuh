@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(128, 3) k_looe_panel(double* __restrict__ H, i
 
 // trailing matrix H[k1.., k1..] -= P P^T, lower tiles, P the panel below the
 // block at k0; grid: the lower tiles
-__global__ void __launch_bounds__(128, 3) k_looe_trail(double* __restrict__ H, int ld, int k0, int nb,
+__global__ void __launch_bounds__(256, 2) k_looe_trail(double* __restrict__ H, int ld, int k0, int nb,
                                                        const int* __restrict__ info) {
   if (*info) return;
   extern __shared__ __align__(16) double looe_smem[];
@@ -201,14 +201,22 @@ __global__ void __launch_bounds__(128, 3) k_looe_trail(double* __restrict__ H, i
   const int k1 = k0 + nb, rows = ld - k1;
   const double* P = H + (size_t)k1 + (size_t)k0 * ld;
   const bool vec = (ld & 1) == 0 && (k1 & 1) == 0;
-  dg::Operand<false> X(P, ld, ti * kPanel, rows, vec), Y(P, ld, tj * kPanel, rows, vec);
-  dg::Acc acc;
+  dg::Operand<false, 256> X(P, ld, ti * kPanel, rows, vec), Y(P, ld, tj * kPanel, rows, vec);
+  dg::AccNb<4> acc, old;
   dg::clear(acc);
-  dg::tile_product_nb<8>(X, Y, 0, nb, looe_smem, acc);
   double* C = H + (size_t)k1 + (size_t)k1 * ld;
-  dg::each(acc, [&](int r, int c, double v) {
-    const int i = ti * kPanel + r, j = tj * kPanel + c;
-    if (i < rows && j < rows) C[(size_t)i + (size_t)j * ld] -= v;
+  auto at = [&](int r, int c) { return (size_t)(ti * kPanel + r) + (size_t)(tj * kPanel + c) * ld; };
+  auto in = [&](int r, int c) { return ti * kPanel + r < rows && tj * kPanel + c < rows; };
+  dg::each_of<4>(old, [&](int r, int c, double& v) { v = in(r, c) ? C[at(r, c)] : 0.0; });  // in flight behind the product
+  dg::tile_product_nb<4>(X, Y, 0, nb, looe_smem, acc);
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) old[m][j][h] -= acc[m][j][h];
+  dg::each_of<4>(old, [&](int r, int c, double v) {
+    if (in(r, c)) C[at(r, c)] = v;
   });
 }
 
@@ -217,7 +225,7 @@ __global__ void __launch_bounds__(128, 3) k_looe_trail(double* __restrict__ H, i
 constexpr int kRowLd = 68;  // row stride of the staged panel and of W
 constexpr size_t kRowsSmem = dg::kSmem + sizeof(double) * kPanel * kRowLd;
 static_assert(sizeof(double) * kPanel * kRowLd <= dg::kSmem, "a panel fits the products' stages");
-__global__ void __launch_bounds__(128) k_looe_rows(const double* __restrict__ A, int M, const int* __restrict__ S, int ns,
+__global__ void __launch_bounds__(256, 2) k_looe_rows(const double* __restrict__ A, int M, const int* __restrict__ S, int ns,
                                                    const double* __restrict__ H, const double* __restrict__ Wall,
                                                    double* __restrict__ Y, double* __restrict__ dlev,
                                                    const int* __restrict__ info) {
@@ -226,35 +234,44 @@ __global__ void __launch_bounds__(128) k_looe_rows(const double* __restrict__ A,
   double* s_t = looe_smem;                                  // [64][68], over the stages
   double* s_w = looe_smem + dg::kSmem / sizeof(double);     // [64][68]
   const int i0 = blockIdx.x * kPanel;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) & 3, half = threadIdx.x >> 7, g = lane >> 2, t = lane & 3;
   double d[2] = {0.0, 0.0};
   const bool vy = (M & 1) == 0, vh = (ns & 1) == 0;
   for (int k0 = 0; k0 < ns; k0 += kPanel) {
     const int nb = min(kPanel, ns - k0);
     const double* W = Wall + (size_t)(k0 / kPanel) * kPanel * kPanel;
-    for (int e = threadIdx.x; e < kPanel * kPanel / 2; e += 128)
+    for (int e = threadIdx.x; e < kPanel * kPanel / 2; e += 256)
       dg::copy2(s_w + (e >> 5) * kRowLd + 2 * (e & 31), W + 2 * e, 2, true);
     cp_async_commit();
-    dg::Acc acc;
+    dg::AccNb<4> acc, rhs;
     dg::clear(acc);
-    dg::Operand<false> X(Y, M, i0, M, vy), L(H, ns, k0, ns, vh);
-    dg::tile_product_nb<8>(X, L, 0, k0, looe_smem, acc);
-    // the right-hand side into shared memory
-    dg::each(acc, [&](int r, int c, double v) {
-      s_t[r * kRowLd + c] = (i0 + r < M && c < nb) ? A[(size_t)S[k0 + c] * M + i0 + r] - v : 0.0;
+    dg::each_of<4>(rhs, [&](int r, int c, double& v) {  // in flight behind the product
+      v = (i0 + r < M && c < nb) ? A[(size_t)S[k0 + c] * M + i0 + r] : 0.0;
+    });
+    dg::Operand<false, 256> X(Y, M, i0, M, vy), L(H, ns, k0, ns, vh);
+    dg::tile_product_nb<4>(X, L, 0, k0, looe_smem, acc);
+    // the right-hand side into shared memory (beyond nb the product is not zero)
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) rhs[m][j][h] -= acc[m][j][h];
+    dg::each_of<4>(rhs, [&](int r, int c, double v) {
+      s_t[r * kRowLd + c] = (i0 + r < M && c < nb) ? v : 0.0;
     });
     cp_async_wait<0>();
     __syncthreads();
     dg::clear(acc);
 #pragma unroll 2
     for (int kk = 0; kk < kPanel; kk += 4) {
-      double a[2], b[8];
+      double a[2], b[4];
 #pragma unroll
       for (int m = 0; m < 2; ++m) a[m] = s_t[(16 * warp + 8 * m + g) * kRowLd + kk + t];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) b[j] = s_w[(8 * j + g) * kRowLd + kk + t];
+      for (int j = 0; j < 4; ++j) b[j] = s_w[(32 * half + 8 * j + g) * kRowLd + kk + t];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
+      for (int j = 0; j < 4; ++j) {
         dmma_884(acc[0][j], a[0], b[j]);
         dmma_884(acc[1][j], a[1], b[j]);
       }
@@ -262,22 +279,28 @@ __global__ void __launch_bounds__(128) k_looe_rows(const double* __restrict__ A,
 #pragma unroll
     for (int m = 0; m < 2; ++m)
 #pragma unroll
-      for (int j = 0; j < 8; ++j)
+      for (int j = 0; j < 4; ++j)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          const int i = i0 + 16 * warp + 8 * m + g, c = 8 * j + 2 * t + h;
+          const int i = i0 + 16 * warp + 8 * m + g, c = 32 * half + 8 * j + 2 * t + h;
           const double v = acc[m][j][h];
           d[m] = fma(v, v, d[m]);  // zero beyond nb and M
           if (i < M && c < nb) Y[(size_t)i + (size_t)(k0 + c) * M] = v;
         }
     __syncthreads();  // Y_k is read, and s_t and s_w are written, by the next panel
   }
+  __shared__ double s_half[kPanel];
 #pragma unroll
   for (int m = 0; m < 2; ++m) {
     d[m] += __shfl_xor_sync(0xffffffffu, d[m], 1);
     d[m] += __shfl_xor_sync(0xffffffffu, d[m], 2);
+    if (t == 0 && half) s_half[16 * warp + 8 * m + g] = d[m];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int m = 0; m < 2; ++m) {
     const int i = i0 + 16 * warp + 8 * m + g;
-    if (t == 0 && i < M) dlev[i] = d[m];
+    if (t == 0 && !half && i < M) dlev[i] = d[m] + s_half[16 * warp + 8 * m + g];
   }
 }
 
@@ -423,11 +446,11 @@ struct Looe {
         if (nt > 0) {
           k_looe_panel<<<nt, 128, dg::kSmem, s>>>(H, ns, k0, nb, W, info);
           MF_LAUNCH_CK();
-          k_looe_trail<<<nt * (nt + 1) / 2, 128, dg::kSmem, s>>>(H, ns, k0, nb, info);
+          k_looe_trail<<<nt * (nt + 1) / 2, 256, dg::kSmem, s>>>(H, ns, k0, nb, info);
           MF_LAUNCH_CK();
         }
       }
-      k_looe_rows<<<cdiv(M, kPanel), 128, kRowsSmem, s>>>(A, M, d_S.as<int>(), ns, H, d_W.as<double>(), d_Y.as<double>(),
+      k_looe_rows<<<cdiv(M, kPanel), 256, kRowsSmem, s>>>(A, M, d_S.as<int>(), ns, H, d_W.as<double>(), d_Y.as<double>(),
                                                          d_lev.as<double>(), info);
       MF_LAUNCH_CK();
     }
