@@ -11,7 +11,7 @@
 //   LOOE_m = mean s,  LOOE_std = sqrt(sum s^2 / (M-1) - LOOE_m^2 M / (M-1)),
 // and reports a Hessian that is not positive definite (dposv info > 0).
 //
-// Here, all in FP64 on one stream, per solution:
+// Here, all in FP64, per solution:
 //   H = A_S^T A_S, lower tiles, by matrix products over the active columns
 //   where they lie (dgemm_mma.cuh; K split so that the tiles fill the GPU);
 //   blocked right-looking Cholesky H = L L^T in 64-wide panels: the diagonal
@@ -28,7 +28,10 @@
 // With one thread per row for the triangular solves (53 % of the time), a
 // barrier per pivot, column and update in the diagonal block (14 %) and scalar
 // 4 x 4 sums in the products (29 %, 13 TFLOP/s), a solution of 1261 active
-// pixels, M = 8000, took 9.9 ms on B200.
+// pixels, M = 8000, took 9.9 ms on B200; here 2.2 ms: the triangular solves
+// 820 us (12.7 GFLOP, 125 CTAs), the diagonal blocks 20 x 27 us (a chain of
+// pivots each), the Gram product 486 us, trailing updates 19 x 8 us, panels
+// 19 x 7 us.  A call with three solutions: 32 ms -> 8.9 ms.
 #pragma once
 
 #include "dgemm_mma.cuh"
@@ -360,37 +363,96 @@ __global__ void k_looe_final(const double* __restrict__ part, int nblk, int M, c
 // Host driver: LOOE of B solutions X [B][N] of the DFT problem (y [M], A
 // column-major M x N); lambda_tsv per solution (null: 0).  Kernels per
 // solution: 6 + 3 ceil(n_s / 64).
+//
+// Only the columns of A that some solution uses go to the device, in runs (a
+// gap of at most kGap columns is copied along rather than splitting a copy).
+// Solutions run on up to kLanes streams, each with its own scratch: one
+// solution's factorisation is a chain of small kernels (840 of 2190 us at 1261
+// active pixels) and its other kernels leave SMs idle, which the next one's
+// fill.  Lanes beyond the first are taken only while all scratch stays within
+// kLaneBytes, and given up when their memory cannot be had; the results do
+// not depend on them.
 struct Looe {
-  int M, N, NX;
-  cudaStream_t s = nullptr;
-  DevMem d_A, d_y, d_S, d_xs, d_ax, d_Y, d_H, d_Hs, d_W, d_lev, d_part, d_info, d_out;
+  static constexpr int kLanes = 4, kGap = 2;
+  static constexpr size_t kLaneBytes = (size_t)1 << 30;
+
+  struct Lane {
+    cudaStream_t s = nullptr;
+    DevMem mem;
+    std::vector<int> idx;    // of the solution in flight: pixels, then columns of the device's A
+    std::vector<double> xs;  // its active values
+    ~Lane() {
+      if (s) cudaStreamDestroy(s);
+    }
+  };
+  // a lane's scratch, in doubles from its start
+  struct Layout {
+    size_t xs, ax, Y, H, Hs, W, lev, part, out, info, idx, total;
+  };
+
+  const double* X;
+  int M, N, NX, B;
+  int most = 0;          // active pixels of a solution at most
+  DevMem d_A, d_y;
+  std::vector<int> col;  // pixel -> column of the device's A
+  std::vector<std::unique_ptr<Lane>> lanes;
   int sms = 148;
 
-  Looe(const double* y, const double* A, int M_, int N_, int NX_) : M(M_), N(N_), NX(NX_) {
-    MF_CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+  Looe(const double* y, const double* A, int M_, int N_, int NX_, const double* X_, int B_)
+      : X(X_), M(M_), N(N_), NX(NX_), B(B_) {
     int dev = 0;
     MF_CK(cudaGetDevice(&dev));
     MF_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    d_A.upload(A, (size_t)M * N);
+    std::vector<char> used(N, 0);
+    for (int b = 0; b < B; ++b) {
+      int n = 0;
+      for (int j = 0; j < N; ++j)
+        if (fabs(X[(size_t)b * N + j]) > 0) {
+          used[j] = 1;
+          ++n;
+        }
+      most = std::max(most, n);
+    }
+    for (int j = 0, last = -1; j < N; ++j)
+      if (used[j]) {
+        if (last >= 0 && j - last <= kGap + 1) std::fill(used.begin() + last, used.begin() + j, 1);
+        last = j;
+      }
+    col.assign(N, 0);
+    int nc = 0;
+    for (int j = 0; j < N; ++j)
+      if (used[j]) col[j] = nc++;
+    d_A.alloc(sizeof(double) * (size_t)M * nc);
+    for (int j = 0; j < N;) {
+      int e = j;
+      while (e < N && used[e]) ++e;
+      if (e > j)
+        MF_CK(cudaMemcpy(d_A.as<double>() + (size_t)col[j] * M, A + (size_t)j * M, sizeof(double) * (size_t)(e - j) * M,
+                         cudaMemcpyHostToDevice));
+      j = e + 1;
+    }
     d_y.upload(y, (size_t)M);
-    d_S.alloc(sizeof(int) * N);
-    d_xs.alloc(sizeof(double) * N);
-    d_ax.alloc(sizeof(double) * kSplitR * (size_t)M);
-    d_lev.alloc(sizeof(double) * M);
-    d_part.alloc(sizeof(double) * 2 * (size_t)cdiv(M, 256));
-    d_info.alloc(sizeof(int));
-    d_out.alloc(sizeof(double) * 3);
+    MF_CK(cudaStreamSynchronize(nullptr));  // the lanes' streams do not wait for the copies' last part
     set_smem(k_looe_gram, dg::kSmem);
     set_smem(k_looe_panel, dg::kSmem);
     set_smem(k_looe_trail, dg::kSmem);
     set_smem(k_looe_rows, kRowsSmem);
-  }
-  ~Looe() {
-    if (s) cudaStreamDestroy(s);
-  }
-
-  static void grow(DevMem& d, size_t bytes) {
-    if (d.bytes < bytes) d.alloc(bytes);
+    const size_t bytes = sizeof(double) * layout(most).total;
+    for (int i = 0; i < std::min(kLanes, B); ++i) {
+      if (i > 0 && (i + 1) * bytes > kLaneBytes) break;
+      std::unique_ptr<Lane> l(new Lane);
+      if (i > 0) {
+        if (cudaMalloc(&l->mem.p, bytes) != cudaSuccess) {
+          cudaGetLastError();
+          break;
+        }
+        l->mem.bytes = bytes;
+      } else {
+        l->mem.alloc(bytes);
+      }
+      MF_CK(cudaStreamCreateWithFlags(&l->s, cudaStreamNonBlocking));
+      lanes.push_back(std::move(l));
+    }
   }
 
   // K splits of the lower tiles: the fewest (at most 4) whose CTAs spread over
@@ -407,41 +469,78 @@ struct Looe {
     }
     return best;
   }
+  static int tiles_of(int ns) {
+    const int np = cdiv(ns, kPanel);
+    return np * (np + 1) / 2;
+  }
 
-  // (looe_m, looe_std, positive) of one solution x [N]
-  void one(const double* x, double lam_tsv, double out[3]) {
-    std::vector<int> S;
-    std::vector<double> xs;
+  // room for every solution of at most ns active pixels
+  Layout layout(int ns) const {
+    Layout l;
+    size_t at = 0;
+    auto take = [&](size_t n) {
+      const size_t p = at;
+      at += (n + 31) & ~(size_t)31;  // 256 bytes
+      return p;
+    };
+    int splits = 1;
+    size_t hs = 0;
+    for (int n = 1, np = cdiv(ns, kPanel); n <= np; ++n) {  // a smaller solution may have more splits
+      const size_t m = std::min((size_t)n * kPanel, (size_t)ns);
+      splits = gram_splits(n * (n + 1) / 2);
+      hs = std::max(hs, splits * m * m);
+    }
+    l.xs = take(ns);
+    l.ax = take(kSplitR * (size_t)M);
+    l.Y = take((size_t)M * ns);
+    l.H = take((size_t)ns * ns);
+    l.Hs = take(hs);
+    l.W = take((size_t)cdiv(ns, kPanel) * kPanel * kPanel);
+    l.lev = take(M);
+    l.part = take(2 * (size_t)cdiv(M, 256));
+    l.out = take(3);
+    l.info = take(1);
+    l.idx = take(ns);  // 2 ns ints
+    l.total = at;
+    return l;
+  }
+
+  // the kernels of solution b on a lane; its results are in the lane's out
+  void launch(Lane& L, int b, double lam_tsv) {
+    const double* x = X + (size_t)b * N;
+    cudaStream_t s = L.s;
+    L.idx.clear();
+    L.xs.clear();
     for (int j = 0; j < N; ++j)
       if (fabs(x[j]) > 0) {
-        S.push_back(j);
-        xs.push_back(x[j]);
+        L.idx.push_back(j);
+        L.xs.push_back(x[j]);
       }
-    const int ns = (int)S.size();
-    const int np = cdiv(ns, kPanel), tiles = np * (np + 1) / 2;
-    const int* info = d_info.as<int>();
-    MF_CK(cudaMemsetAsync(d_info.p, 0, sizeof(int), s));
+    const int ns = (int)L.xs.size();
+    for (int q = 0; q < ns; ++q) L.idx.push_back(col[L.idx[q]]);
+    const int np = cdiv(ns, kPanel), tiles = tiles_of(ns);
+    const Layout l = layout(most);
+    double* m = L.mem.as<double>();
+    int* info = reinterpret_cast<int*>(m + l.info);
+    int *pix = reinterpret_cast<int*>(m + l.idx), *S = pix + ns;
+    MF_CK(cudaMemsetAsync(info, 0, sizeof(int), s));
     if (ns > 0) {
       const int nsplit = gram_splits(tiles);
       const int kchunk = cdiv(cdiv(M, nsplit), dg::kStep) * dg::kStep;
-      MF_CK(cudaMemcpyAsync(d_S.p, S.data(), sizeof(int) * ns, cudaMemcpyHostToDevice, s));
-      MF_CK(cudaMemcpyAsync(d_xs.p, xs.data(), sizeof(double) * ns, cudaMemcpyHostToDevice, s));
-      grow(d_Y, sizeof(double) * (size_t)M * ns);
-      grow(d_H, sizeof(double) * (size_t)ns * ns);
-      grow(d_Hs, sizeof(double) * (size_t)nsplit * ns * ns);
-      grow(d_W, sizeof(double) * (size_t)np * kPanel * kPanel);
-      double* H = d_H.as<double>();
+      MF_CK(cudaMemcpyAsync(pix, L.idx.data(), 2 * sizeof(int) * ns, cudaMemcpyHostToDevice, s));
+      MF_CK(cudaMemcpyAsync(m + l.xs, L.xs.data(), sizeof(double) * ns, cudaMemcpyHostToDevice, s));
+      double *H = m + l.H, *Hs = m + l.Hs;
       const double* A = d_A.as<double>();
-      k_looe_ax<<<dim3(cdiv(M, 256), kSplitR), 256, 0, s>>>(A, M, d_S.as<int>(), d_xs.as<double>(), ns, d_ax.as<double>());
+      k_looe_ax<<<dim3(cdiv(M, 256), kSplitR), 256, 0, s>>>(A, M, S, m + l.xs, ns, m + l.ax);
       MF_LAUNCH_CK();
-      k_looe_gram<<<dim3(tiles, nsplit), 128, dg::kSmem, s>>>(A, M, d_S.as<int>(), ns, kchunk, d_Hs.as<double>());
+      k_looe_gram<<<dim3(tiles, nsplit), 128, dg::kSmem, s>>>(A, M, S, ns, kchunk, Hs);
       MF_LAUNCH_CK();
-      k_looe_gram_sum<<<dim3(cdiv(ns, 256), ns), 256, 0, s>>>(d_Hs.as<double>(), nsplit, H, d_S.as<int>(), ns, NX, lam_tsv);
+      k_looe_gram_sum<<<dim3(cdiv(ns, 256), ns), 256, 0, s>>>(Hs, nsplit, H, pix, ns, NX, lam_tsv);
       MF_LAUNCH_CK();
       for (int k0 = 0; k0 < ns; k0 += kPanel) {
         const int nb = std::min(kPanel, ns - k0), nt = cdiv(ns - k0 - nb, kPanel);
-        double* W = d_W.as<double>() + (size_t)(k0 / kPanel) * kPanel * kPanel;
-        k_looe_chol_diag<<<1, 256, 0, s>>>(H, ns, k0, nb, W, d_info.as<int>());
+        double* W = m + l.W + (size_t)(k0 / kPanel) * kPanel * kPanel;
+        k_looe_chol_diag<<<1, 256, 0, s>>>(H, ns, k0, nb, W, info);
         MF_LAUNCH_CK();
         if (nt > 0) {
           k_looe_panel<<<nt, 128, dg::kSmem, s>>>(H, ns, k0, nb, W, info);
@@ -450,18 +549,32 @@ struct Looe {
           MF_LAUNCH_CK();
         }
       }
-      k_looe_rows<<<cdiv(M, kPanel), 256, kRowsSmem, s>>>(A, M, d_S.as<int>(), ns, H, d_W.as<double>(), d_Y.as<double>(),
-                                                         d_lev.as<double>(), info);
+      k_looe_rows<<<cdiv(M, kPanel), 256, kRowsSmem, s>>>(A, M, S, ns, H, m + l.W, m + l.Y, m + l.lev, info);
       MF_LAUNCH_CK();
     }
     const int nblk = cdiv(M, 256);
-    k_looe_terms<<<nblk, 256, 0, s>>>(d_y.as<double>(), d_ax.as<double>(), ns > 0 ? kSplitR : 0, d_lev.as<double>(), M,
-                                      d_part.as<double>(), info);
+    k_looe_terms<<<nblk, 256, 0, s>>>(d_y.as<double>(), m + l.ax, ns > 0 ? kSplitR : 0, m + l.lev, M, m + l.part, info);
     MF_LAUNCH_CK();
-    k_looe_final<<<1, 32, 0, s>>>(d_part.as<double>(), nblk, M, info, d_out.as<double>());
+    k_looe_final<<<1, 32, 0, s>>>(m + l.part, nblk, M, info, m + l.out);
     MF_LAUNCH_CK();
-    MF_CK(cudaMemcpyAsync(out, d_out.p, sizeof(double) * 3, cudaMemcpyDeviceToHost, s));
-    MF_CK(cudaStreamSynchronize(s));
+  }
+
+  // f(b, {looe_m, looe_std, positive}) for every solution in order
+  template <typename F> void all(const double* lambda_tsv, F f) {
+    const int nl = (int)lanes.size();
+    const Layout l = layout(most);
+    auto finish = [&](int b) {
+      Lane& L = *lanes[b % nl];
+      double out[3];
+      MF_CK(cudaMemcpyAsync(out, L.mem.as<double>() + l.out, sizeof(out), cudaMemcpyDeviceToHost, L.s));
+      MF_CK(cudaStreamSynchronize(L.s));
+      f(b, out);
+    };
+    for (int b = 0; b < B; ++b) {
+      if (b >= nl) finish(b - nl);  // the lane's solution before
+      launch(*lanes[b % nl], b, lambda_tsv ? lambda_tsv[b] : 0.0);
+    }
+    for (int b = std::max(0, B - nl); b < B; ++b) finish(b);
   }
 };
 

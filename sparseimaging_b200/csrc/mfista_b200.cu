@@ -1016,14 +1016,12 @@ extern "C" int mfista_dft_looe(const double* y, const double* A, int M, int N, i
     if (M < 2 || N < 1 || NX < 1 || B < 1) throw Error(MFISTA_ERR_ARG, "mfista_dft_looe: needs M >= 2, N, NX, B >= 1");
     if (!y || !A || !X || !looe_m || !looe_std || !hessian_positive)
       throw Error(MFISTA_ERR_ARG, "mfista_dft_looe: null pointer");
-    looe::Looe L(y, A, M, N, NX);
-    for (int b = 0; b < B; ++b) {
-      double out[3];
-      L.one(X + (size_t)b * N, lambda_tsv ? lambda_tsv[b] : 0.0, out);
+    looe::Looe L(y, A, M, N, NX, X, B);
+    L.all(lambda_tsv, [&](int b, const double* out) {
       looe_m[b] = out[0];
       looe_std[b] = out[1];
       hessian_positive[b] = out[2] > 0.5 ? 1 : 0;
-    }
+    });
     return MFISTA_OK;
   } catch (const Error& e) {
     return fail(e.status, e.what(), false);

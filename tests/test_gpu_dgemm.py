@@ -35,3 +35,33 @@ def test_looe_tile_edges_match_oracle(gpulib, m, ns):
     st, wm, ws = O.looe(y, A, x, nx, 0.3)
     assert st == 1 and pos[0]
     assert abs(mean[0] - wm) <= 1e-9 * abs(wm) and abs(std[0] - ws) <= 1e-9 * abs(ws)
+
+
+@pytest.mark.parametrize("b", [1, 2, 9])
+def test_looe_of_a_batch_is_that_of_its_solutions(gpulib, b):
+    """More solutions than streams, each with its own support (columns of A in
+    runs with gaps of 1 to 5, the first and the last one; one solution empty,
+    one not positive definite between good ones): same bits as alone."""
+    rng = np.random.default_rng(b)
+    nx, m = 16, 400
+    n = nx * nx
+    A = rng.normal(size=(m, n)) / np.sqrt(m)
+    A[:, 7] = 0.0  # a column of zeros: singular without lambda_tsv
+    X = np.zeros((b, n))
+    for k in range(b):
+        at = np.cumsum(rng.integers(1, 7, size=n // 4))
+        X[k, at[at < n]] = 1 + rng.random((at < n).sum())
+        X[k, 7] = 1.0 if k == 3 else 0.0
+    X[0, [0, n - 1]] = 2.0
+    if b > 4:
+        X[4] = 0.0
+    y = A @ X[0] + 0.01 * rng.normal(size=m)
+    lam = np.where(np.arange(b) == 3, 0.0, 0.1 * (1 + np.arange(b)))
+    mean, std, pos = gpulib.dft_looe(y, A, X, nx, lambda_tsv=lam)
+    for k in range(b):
+        one = gpulib.dft_looe(y, A, X[k:k + 1], nx, lambda_tsv=lam[k:k + 1])
+        assert (mean[k], std[k], pos[k]) == (one[0][0], one[1][0], one[2][0])
+        assert pos[k] == (k != 3)
+        if k not in (3, 4):
+            _, wm, ws = O.looe(y, A, X[k], nx, lam[k])
+            assert abs(mean[k] - wm) <= 1e-9 * abs(wm) and abs(std[k] - ws) <= 1e-9 * abs(ws)
