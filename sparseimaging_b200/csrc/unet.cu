@@ -68,6 +68,7 @@ struct ConvArgs {
   const float* b;
   int cb;
   const __nv_bfloat16* w;  // [cout][ca+cb][3][3]
+  const __nv_bfloat16* wtap;  // the same for the tensor cores: [chunk of 16 inputs][tap][cout][16], zeros beyond ca+cb
   const float* bias;       // [cout] or null
   float* out;
   int cout, H, W, relu;
@@ -195,14 +196,30 @@ __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], const uint32_t (&a
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+// a pair of values as BF16 planes: the packed high parts, and the low parts
+__device__ __forceinline__ uint32_t split_pair(float v0, float v1, uint32_t& lo) {
+  const __nv_bfloat16 h0 = __float2bfloat16_rn(v0), h1 = __float2bfloat16_rn(v1);
+  const __nv_bfloat16 l0 = __float2bfloat16_rn(v0 - __bfloat162float(h0));
+  const __nv_bfloat16 l1 = __float2bfloat16_rn(v1 - __bfloat162float(h1));
+  lo = (uint32_t)__bfloat16_as_ushort(l0) | ((uint32_t)__bfloat16_as_ushort(l1) << 16);
+  return (uint32_t)__bfloat16_as_ushort(h0) | ((uint32_t)__bfloat16_as_ushort(h1) << 16);
+}
+
+// Staging, not the products, is what a CTA spends its issue slots and its
+// waiting on (tensor pipe 8-17 % busy): a thread keeps three (halo pixel, half
+// chunk) items for all chunks, reads an item's 8 channels into registers, all
+// in flight at once, and stores them as two 16-byte words; the weights lie
+// tap-major and come by cp.async.  One element at a time, with its index
+// arithmetic and two 2-byte stores, a gradient at 256 x 256, batch 8 took 5.7
+// ms, 4.05 this way (the weight gradient's staging included).  A second buffer
+// for the next chunk cost more in occupancy than it hid (4.15 ms).
 template <int MT>
 __global__ void __launch_bounds__(256) k_conv3x3_tc(ConvArgs g) {
   constexpr int CO = 16 * MT;
+  constexpr int kItems = (2 * kTcHalo + 255) / 256;
   extern __shared__ __align__(16) uint32_t s_tc[];
-  uint32_t* s_x = s_tc;                                  // [2][324][kTcRow]
-  uint32_t* s_w = s_tc + 2 * kTcHalo * kTcRow;           // [9][CO][kTcRow]
-  __nv_bfloat16* s_x16 = reinterpret_cast<__nv_bfloat16*>(s_x);
-  __nv_bfloat16* s_w16 = reinterpret_cast<__nv_bfloat16*>(s_w);
+  uint32_t* s_x = s_tc;                          // [2][324][kTcRow]
+  uint32_t* s_w = s_tc + 2 * kTcHalo * kTcRow;   // [9][CO][kTcRow]
   const int tiles_x = cdiv(g.W, kCT);
   const int tx0 = (blockIdx.x % tiles_x) * kCT, ty0 = (blockIdx.x / tiles_x) * kCT;
   const int co0 = blockIdx.y * CO, n = blockIdx.z;
@@ -217,35 +234,84 @@ __global__ void __launch_bounds__(256) k_conv3x3_tc(ConvArgs g) {
 #pragma unroll
       for (int e = 0; e < 4; ++e) acc[m][j][e] = 0.f;
   const int ha = g.a_up ? g.H / 2 : g.H, wa = g.a_up ? g.W / 2 : g.W;
-  for (int c0 = 0; c0 < cin; c0 += kCI) {
-    __syncthreads();  // the previous chunk's fragments have been read
-    for (int t = threadIdx.x; t < kCI * kTcHalo; t += blockDim.x) {
-      const int ci = t / kTcHalo, pix = t - ci * kTcHalo;
-      const int yy = pix / (kCT + 2), xx = pix - yy * (kCT + 2);
-      const int y = ty0 + yy - 1, x = tx0 + xx - 1;
-      const int c = c0 + ci;
-      float v = 0.f;
-      if (c < cin && y >= 0 && y < g.H && x >= 0 && x < g.W) {
-        if (c < g.ca) {
-          const int sy = g.a_up ? y >> 1 : y, sx = g.a_up ? x >> 1 : x;
-          const size_t idx = (((size_t)n * g.ca + c) * ha + sy) * wa + sx;
-          v = g.a[idx];
-          if (g.amask && !(g.amask[idx] > 0.f)) v = 0.f;
-        } else {
-          v = g.b[(((size_t)n * g.cb + (c - g.ca)) * g.H + y) * g.W + x];
+  const size_t pa = (size_t)ha * wa, pb = (size_t)g.H * g.W;
+  const float* abase = g.a + (size_t)n * g.ca * pa;
+  const float* mbase = g.amask ? g.amask + (size_t)n * g.ca * pa : nullptr;
+  const float* bbase = g.b ? g.b + (size_t)n * g.cb * pb : nullptr;
+  int offa[kItems], offb[kItems];  // -1: outside the image
+#pragma unroll
+  for (int r = 0; r < kItems; ++r) {
+    const int t = threadIdx.x + 256 * r, pix = t < kTcHalo ? t : t - kTcHalo;
+    const int yy = pix / (kCT + 2), xx = pix - yy * (kCT + 2);
+    const int y = ty0 + yy - 1, x = tx0 + xx - 1;
+    offa[r] = offb[r] = -1;
+    if (t < 2 * kTcHalo && y >= 0 && y < g.H && x >= 0 && x < g.W) {
+      offa[r] = g.a_up ? (y >> 1) * wa + (x >> 1) : y * wa + x;
+      offb[r] = y * g.W + x;
+    }
+  }
+  float v[kItems][8];
+  auto fetch = [&](int c0) {
+#pragma unroll
+    for (int r = 0; r < kItems; ++r) {
+      const int c = c0 + ((int)threadIdx.x + 256 * r < kTcHalo ? 0 : 8);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) v[r][q] = 0.f;
+      if (offa[r] < 0) continue;
+      if (c + 8 <= g.ca) {
+        const size_t idx = (size_t)c * pa + offa[r];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[r][q] = abase[idx + q * pa];
+        if (mbase) {
+#pragma unroll
+          for (int q = 0; q < 8; ++q)
+            if (!(mbase[idx + q * pa] > 0.f)) v[r][q] = 0.f;
+        }
+      } else {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          if (c + q < g.ca) {
+            const size_t idx = (size_t)(c + q) * pa + offa[r];
+            v[r][q] = abase[idx];
+            if (mbase && !(mbase[idx] > 0.f)) v[r][q] = 0.f;
+          } else if (c + q < cin) {
+            v[r][q] = bbase[(size_t)(c + q - g.ca) * pb + offb[r]];
+          }
         }
       }
-      const __nv_bfloat16 hi = __float2bfloat16_rn(v);
-      const __nv_bfloat16 lo = __float2bfloat16_rn(v - __bfloat162float(hi));
-      s_x16[(size_t)pix * (2 * kTcRow) + ci] = hi;
-      s_x16[(size_t)(kTcHalo + pix) * (2 * kTcRow) + ci] = lo;
     }
-    for (int t = threadIdx.x; t < 9 * CO * kCI; t += blockDim.x) {
-      const int ci = t % kCI, r = t / kCI, co = r % CO, tap = r / CO;
-      __nv_bfloat16 w = __float2bfloat16_rn(0.f);
-      if (co0 + co < g.cout && c0 + ci < cin) w = g.w[((size_t)(co0 + co) * cin + c0 + ci) * 9 + tap];
-      s_w16[(size_t)(tap * CO + co) * (2 * kTcRow) + ci] = w;
+  };
+  auto put = [&]() {
+#pragma unroll
+    for (int r = 0; r < kItems; ++r) {
+      const int t = threadIdx.x + 256 * r;
+      if (t >= 2 * kTcHalo) continue;
+      uint4 hi, lo;
+      hi.x = split_pair(v[r][0], v[r][1], lo.x);
+      hi.y = split_pair(v[r][2], v[r][3], lo.y);
+      hi.z = split_pair(v[r][4], v[r][5], lo.z);
+      hi.w = split_pair(v[r][6], v[r][7], lo.w);
+      uint32_t* d = s_x + (size_t)(t < kTcHalo ? t : t - kTcHalo) * kTcRow + (t < kTcHalo ? 0 : 4);
+      *reinterpret_cast<uint4*>(d) = hi;
+      *reinterpret_cast<uint4*>(d + kTcHalo * kTcRow) = lo;
     }
+  };
+  auto weights = [&](int c0) {
+    const __nv_bfloat16* src = g.wtap + (size_t)(c0 / kCI) * 9 * g.cout * kCI;
+    for (int t = threadIdx.x; t < 18 * CO; t += 256) {
+      const int row = t >> 1, tap = row / CO, co = row - tap * CO;
+      const bool ok = co0 + co < g.cout;
+      const unsigned int d = (unsigned int)__cvta_generic_to_shared(s_w + (size_t)row * kTcRow + 4 * (t & 1));
+      const __nv_bfloat16* p = src + ((size_t)tap * g.cout + (ok ? co0 + co : 0)) * kCI + 8 * (t & 1);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(p), "r"(ok ? 16 : 0) : "memory");
+    }
+  };
+  for (int c0 = 0; c0 < cin; c0 += kCI) {
+    fetch(c0);
+    __syncthreads();  // the previous chunk's fragments have been read
+    weights(c0);
+    put();
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
 #pragma unroll 1
     for (int tap = 0; tap < 9; ++tap) {
@@ -294,6 +360,7 @@ __global__ void __launch_bounds__(256) k_conv3x3_tc(ConvArgs g) {
 template <int MT> constexpr size_t conv_tc_smem() { return sizeof(uint32_t) * (2 * kTcHalo + 9 * 16 * MT) * kTcRow; }
 
 // weights of the backward-data convolution: wt[ci][co][k] = w[co][ci][8 - k]
+// (the CUDA-core path; the tensor cores' copies come with the rounding)
 __global__ void k_flip_transpose(const __nv_bfloat16* __restrict__ w, int cout, int cin,
                                  __nv_bfloat16* __restrict__ wt) {
   int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -385,6 +452,10 @@ __global__ void __launch_bounds__(256) k_conv3x3_wgrad(WgradArgs g) {
 // accumulated in FP32 (lo*lo, ~2^-18 of the rest, is left out).  Nine warps,
 // one per tap; the partials go to the same layout as k_conv3x3_wgrad's and
 // are reduced over tiles in tile order by k_reduce_partials.
+// Bound by staging: pairs of pixels are read into registers, all loads in
+// flight, and stored as words of two BF16; a pair that starts at the odd
+// column of a tap comes from two words.  Element by element it took 1.9 ms of
+// a gradient at 256 x 256, batch 8, 1.3 ms this way.
 constexpr int kWgG = 132;  // 32-bit words per staged G row (256 pixels + pad)
 constexpr int kWgX = 164;  // 32-bit words per staged X channel (324 halo pixels + pad)
 
@@ -392,8 +463,6 @@ __global__ void __launch_bounds__(288) k_conv3x3_wgrad_tc(WgradArgs g) {
   extern __shared__ __align__(16) uint32_t s_wg[];
   uint32_t* s_g = s_wg;                   // [2][16][kWgG]
   uint32_t* s_x = s_wg + 2 * 16 * kWgG;   // [2][16][kWgX]
-  __nv_bfloat16* s_g16 = reinterpret_cast<__nv_bfloat16*>(s_g);
-  __nv_bfloat16* s_x16 = reinterpret_cast<__nv_bfloat16*>(s_x);
   const int tiles_x = cdiv(g.W, kCT), tiles_y = cdiv(g.H, kCT);
   const int tile = blockIdx.x;  // over n * tiles
   const int n = tile / (tiles_x * tiles_y), tr = tile - n * tiles_x * tiles_y;
@@ -401,36 +470,70 @@ __global__ void __launch_bounds__(288) k_conv3x3_wgrad_tc(WgradArgs g) {
   const int co0 = blockIdx.y * 16, ci0 = blockIdx.z * kCI;
   const int cin = g.ca + g.cb;
   const int ha = g.a_up ? g.H / 2 : g.H, wa = g.a_up ? g.W / 2 : g.W;
-  for (int t = threadIdx.x; t < 16 * kCT * kCT; t += blockDim.x) {
-    const int co = t / (kCT * kCT), p = t - co * kCT * kCT;
-    const int y = ty0 + p / kCT, x = tx0 + p % kCT;
-    float v = 0.f;
-    if (co0 + co < g.cout && y < g.H && x < g.W) {
-      const size_t idx = (((size_t)n * g.cout + co0 + co) * g.H + y) * g.W + x;
-      v = g.g[idx];
-      if (g.gmask && !(g.gmask[idx] > 0.f)) v = 0.f;
+  // G: a thread takes two adjacent pixels of 8 channels
+  if (threadIdx.x < 256) {
+    const int pp = threadIdx.x & 127, cg0 = (threadIdx.x >> 7) * 8;
+    const int y = ty0 + pp / (kCT / 2), x = tx0 + 2 * (pp % (kCT / 2));
+    const bool in = y < g.H && x < g.W, two = x + 1 < g.W, vec = (g.W & 1) == 0;  // odd widths: unaligned pairs
+    const size_t hw = (size_t)g.H * g.W, idx = ((size_t)n * g.cout + co0 + cg0) * hw + (size_t)y * g.W + x;
+    auto pair = [&](const float* p) {
+      return vec ? *reinterpret_cast<const float2*>(p) : make_float2(p[0], two ? p[1] : 0.f);
+    };
+    float2 v[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      v[q] = make_float2(0.f, 0.f);
+      if (in && co0 + cg0 + q < g.cout) v[q] = pair(g.g + idx + q * hw);
     }
-    const __nv_bfloat16 hi = __float2bfloat16_rn(v);
-    s_g16[(size_t)co * (2 * kWgG) + p] = hi;
-    s_g16[(size_t)(16 + co) * (2 * kWgG) + p] = __float2bfloat16_rn(v - __bfloat162float(hi));
-  }
-  for (int t = threadIdx.x; t < kCI * kTcHalo; t += blockDim.x) {
-    const int ci = t / kTcHalo, pix = t - ci * kTcHalo;
-    const int yy = pix / (kCT + 2), xx = pix - yy * (kCT + 2);
-    const int y = ty0 + yy - 1, x = tx0 + xx - 1;
-    const int c = ci0 + ci;
-    float v = 0.f;
-    if (c < cin && y >= 0 && y < g.H && x >= 0 && x < g.W) {
-      if (c < g.ca) {
-        const int sy = g.a_up ? y >> 1 : y, sx = g.a_up ? x >> 1 : x;
-        v = g.a[(((size_t)n * g.ca + c) * ha + sy) * wa + sx];
-      } else {
-        v = g.b[(((size_t)n * g.cb + (c - g.ca)) * g.H + y) * g.W + x];
+    if (g.gmask) {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        if (in && co0 + cg0 + q < g.cout) {
+          const float2 m = pair(g.gmask + idx + q * hw);
+          if (!(m.x > 0.f)) v[q].x = 0.f;
+          if (!(m.y > 0.f)) v[q].y = 0.f;
+        }
       }
     }
-    const __nv_bfloat16 hi = __float2bfloat16_rn(v);
-    s_x16[(size_t)ci * (2 * kWgX) + pix] = hi;
-    s_x16[(size_t)(16 + ci) * (2 * kWgX) + pix] = __float2bfloat16_rn(v - __bfloat162float(hi));
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      uint32_t lo;
+      s_g[(size_t)(cg0 + q) * kWgG + pp] = split_pair(v[q].x, v[q].y, lo);
+      s_g[(size_t)(16 + cg0 + q) * kWgG + pp] = lo;
+    }
+  }
+  // X: 162 pairs of halo pixels x 16 channels, nine a thread
+  constexpr int kPairs = kTcHalo / 2;
+  static_assert(kPairs * kCI == 9 * 288, "nine pairs a thread");
+  {
+    float2 v[9];
+#pragma unroll
+    for (int r = 0; r < 9; ++r) {
+      const int t = threadIdx.x + 288 * r, ci = t / kPairs, pr = t - ci * kPairs;
+      const int yy = pr / (kCT / 2 + 1), xx = 2 * (pr - yy * (kCT / 2 + 1));
+      const int y = ty0 + yy - 1, x = tx0 + xx - 1, c = ci0 + ci;
+      v[r] = make_float2(0.f, 0.f);
+      if (c < cin && y >= 0 && y < g.H) {
+        const float* row;
+        int x0 = x, x1 = x + 1;
+        if (c < g.ca) {
+          const int sy = g.a_up ? y >> 1 : y;
+          row = g.a + (((size_t)n * g.ca + c) * ha + sy) * wa;
+          if (g.a_up) x0 >>= 1, x1 >>= 1;
+        } else {
+          row = g.b + (((size_t)n * g.cb + (c - g.ca)) * g.H + y) * g.W;
+        }
+        if (x >= 0 && x < g.W) v[r].x = row[x0];
+        if (x + 1 < g.W) v[r].y = row[x1];
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < 9; ++r) {
+      const int t = threadIdx.x + 288 * r, ci = t / kPairs, pr = t - ci * kPairs;
+      uint32_t lo;
+      s_x[(size_t)ci * kWgX + pr] = split_pair(v[r].x, v[r].y, lo);
+      s_x[(size_t)(16 + ci) * kWgX + pr] = lo;
+    }
   }
   __syncthreads();
   const int lane = threadIdx.x & 31, tap = threadIdx.x >> 5;  // warp = tap
@@ -441,9 +544,6 @@ __global__ void __launch_bounds__(288) k_conv3x3_wgrad_tc(WgradArgs g) {
   for (int j = 0; j < 2; ++j)
 #pragma unroll
     for (int e = 0; e < 4; ++e) acc[j][e] = 0.f;
-  auto pack = [](__nv_bfloat16 lo16, __nv_bfloat16 hi16) -> uint32_t {
-    return (uint32_t)__bfloat16_as_ushort(lo16) | ((uint32_t)__bfloat16_as_ushort(hi16) << 16);
-  };
 #pragma unroll 1
   for (int py = 0; py < kCT; ++py) {  // k16 step: pixels (py, 0..15)
     uint32_t a[2][4];                   // G planes: rows co = gid (+8), k = pixel
@@ -462,9 +562,15 @@ __global__ void __launch_bounds__(288) k_conv3x3_wgrad_tc(WgradArgs g) {
       uint32_t b[2][2];
 #pragma unroll
       for (int pl = 0; pl < 2; ++pl) {
-        const __nv_bfloat16* xr = s_x16 + (size_t)(pl * 16 + 8 * j + gid) * (2 * kWgX) + hrow;
-        b[pl][0] = pack(xr[tig * 2], xr[tig * 2 + 1]);
-        b[pl][1] = pack(xr[tig * 2 + 8], xr[tig * 2 + 9]);
+        // pixels hrow + 2 tig, + 1 (and 8 further): a word, or the halves of
+        // two where the tap's column is the odd one
+        const uint32_t* xr = s_x + (size_t)(pl * 16 + 8 * j + gid) * kWgX + (hrow >> 1) + tig;
+        b[pl][0] = xr[0];
+        b[pl][1] = xr[4];
+        if (kx == 1) {
+          b[pl][0] = __funnelshift_r(b[pl][0], xr[1], 16);
+          b[pl][1] = __funnelshift_r(b[pl][1], xr[5], 16);
+        }
       }
       mma_bf16_16816(acc[j], a[0], b[0][0], b[0][1]);  // hi * hi
       mma_bf16_16816(acc[j], a[0], b[1][0], b[1][1]);  // hi * lo
@@ -604,9 +710,27 @@ __global__ void __launch_bounds__(256) k_head_sums(const float* __restrict__ h, 
 }
 
 // Adam on FP32 master parameters; refreshes the BF16 weight copies
+// master parameter -> its BF16 copies.  wmap [n][3]: the place in parameter
+// order, tap-major for the forward and tap-major, flipped and transposed, for
+// the backward convolutions, or -1
+__device__ __forceinline__ void round_weight(float p, long i, __nv_bfloat16* wbf, __nv_bfloat16* wtap, const int* wmap) {
+  const int m0 = wmap[3 * i], m1 = wmap[3 * i + 1], m2 = wmap[3 * i + 2];
+  const __nv_bfloat16 w = __float2bfloat16(p);
+  if (m0 >= 0) wbf[m0] = w;
+  if (m1 >= 0) wtap[m1] = w;
+  if (m2 >= 0) wtap[m2] = w;
+}
+
+__global__ void k_round_weights(const float* __restrict__ p, long n, __nv_bfloat16* __restrict__ wbf,
+                                __nv_bfloat16* __restrict__ wtap, const int* __restrict__ wmap) {
+  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) round_weight(p[i], i, wbf, wtap, wmap);
+}
+
 __global__ void k_adam(float* __restrict__ p, const float* __restrict__ gr, float* __restrict__ m,
                        float* __restrict__ v, long n, float lr, float b1, float b2, float eps, float c1, float c2,
-                       __nv_bfloat16* __restrict__ wbf, const int* __restrict__ wmap) {
+                       __nv_bfloat16* __restrict__ wbf, __nv_bfloat16* __restrict__ wtap,
+                       const int* __restrict__ wmap) {
   long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float gi = gr[i];
@@ -616,14 +740,7 @@ __global__ void k_adam(float* __restrict__ p, const float* __restrict__ gr, floa
   v[i] = vi;
   const float pi = p[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
   p[i] = pi;
-  if (wmap[i] >= 0) wbf[wmap[i]] = __float2bfloat16(pi);
-}
-
-// master parameters -> BF16 weight copies
-__global__ void k_round_weights(const float* __restrict__ p, long n, __nv_bfloat16* __restrict__ wbf,
-                                const int* __restrict__ wmap) {
-  long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n && wmap[i] >= 0) wbf[wmap[i]] = __float2bfloat16(p[i]);
+  round_weight(pi, i, wbf, wtap, wmap);
 }
 
 // ---------------------------------------------------------------------------
@@ -657,6 +774,7 @@ struct Conv {
   int level;          // resolution level (0 = full)
   long w_off, b_off;  // offsets into the FP32 parameter vector
   long wbf_off;       // offset into the BF16 weights
+  long tap_f, tap_b;  // and into the tap-major ones: forward, backward
 };
 
 // input a of conv i: -1 the network input, -2..-4 pool outputs 0..2,
@@ -672,7 +790,7 @@ struct Net {
   std::vector<Conv> convs;
   long nparam = 0, nweights = 0;
   long head_w = 0, head_b = 0, head_wbf = 0;
-  Mem p, g, m, v, wbf, wmap, wt, part;
+  Mem p, g, m, v, wbf, wtap, wmap, wt, part;
   std::vector<Mem> act, gact;  // act[0] input, act[i + 1] output of conv i (post-ReLU)
   Mem pool[3], gpool[3], gup, out, sq, gpre, hsum, tgt, red;
   cudaStream_t s = nullptr;
@@ -685,7 +803,7 @@ struct Net {
   Net(int H_, int W_, int nmax_) : H(H_), W(W_), nmax(nmax_) {
     if (H < 16 || W < 16 || H % 8 || W % 8 || nmax < 1)
       throw Error(MFISTA_ERR_ARG, "U-Net needs H, W multiples of 8 (>= 16) and a batch >= 1");
-    auto add = [&](int cout, int ca, int cb, int up, int lv) { convs.push_back(Conv{cout, ca, cb, up, lv, 0, 0, 0}); };
+    auto add = [&](int cout, int ca, int cb, int up, int lv) { convs.push_back(Conv{cout, ca, cb, up, lv, 0, 0, 0, 0, 0}); };
     add(16, 2, 0, 0, 0);     // 0  e1a
     add(16, 16, 0, 0, 0);    // 1  e1
     add(32, 16, 0, 0, 1);    // 2  e2a  (input pool(e1))
@@ -727,12 +845,29 @@ struct Net {
     v.alloc(sizeof(float) * nparam);
     UN_CK(cudaMemset(g.p, 0, g.bytes));
     wbf.alloc(sizeof(__nv_bfloat16) * nweights);
-    std::vector<int> map(nparam, -1);
-    for (const Conv& c : convs)
-      for (long i = 0; i < (long)c.cout * (c.ca + c.cb) * 9; ++i) map[c.w_off + i] = (int)(c.wbf_off + i);
-    for (int i = 0; i < 16; ++i) map[head_w + i] = (int)(head_wbf + i);
-    wmap.alloc(sizeof(int) * nparam);
-    UN_CK(cudaMemcpy(wmap.p, map.data(), sizeof(int) * nparam, cudaMemcpyHostToDevice));
+    std::vector<int> map(3 * nparam, -1);
+    long to = 0;
+    for (Conv& c : convs) {
+      const int cin = c.ca + c.cb;
+      c.tap_f = to;
+      to += (long)cdiv(cin, kCI) * kCI * 9 * c.cout;
+      c.tap_b = to;
+      if (c.w_off > 0) to += (long)cdiv(c.cout, kCI) * kCI * 9 * cin;  // the first has no data gradient
+      for (int co = 0; co < c.cout; ++co)
+        for (int ci = 0; ci < cin; ++ci)
+          for (int k = 0; k < 9; ++k) {
+            const long i = ((long)co * cin + ci) * 9 + k;
+            int* e = &map[3 * (c.w_off + i)];
+            e[0] = (int)(c.wbf_off + i);
+            e[1] = (int)(c.tap_f + ((long)(ci / kCI * 9 + k) * c.cout + co) * kCI + ci % kCI);
+            if (c.w_off > 0) e[2] = (int)(c.tap_b + ((long)(co / kCI * 9 + 8 - k) * cin + ci) * kCI + co % kCI);
+          }
+    }
+    for (int i = 0; i < 16; ++i) map[3 * (head_w + i)] = (int)(head_wbf + i);
+    wmap.alloc(sizeof(int) * map.size());
+    UN_CK(cudaMemcpy(wmap.p, map.data(), wmap.bytes, cudaMemcpyHostToDevice));
+    wtap.alloc(sizeof(__nv_bfloat16) * to);
+    UN_CK(cudaMemset(wtap.p, 0, wtap.bytes));
     long maxw = 0;
     size_t maxpart = 0, maxred = 0;
     for (const Conv& c : convs) {
@@ -802,7 +937,7 @@ struct Net {
   void set_params(const float* hp) {
     UN_CK(cudaMemcpyAsync(p.p, hp, sizeof(float) * nparam, cudaMemcpyHostToDevice, s));
     k_round_weights<<<cdiv(nparam, 256), 256, 0, s>>>(p.as<float>(), nparam, wbf.as<__nv_bfloat16>(),
-                                                      wmap.as<int>());
+                                                      wtap.as<__nv_bfloat16>(), wmap.as<int>());
     UN_LAUNCH();
     UN_CK(cudaMemsetAsync(m.p, 0, m.bytes, s));
     UN_CK(cudaMemsetAsync(v.p, 0, v.bytes, s));
@@ -825,6 +960,8 @@ struct Net {
   }
 
   const __nv_bfloat16* wb(const Conv& c) const { return wbf.as<__nv_bfloat16>() + c.wbf_off; }
+
+  const __nv_bfloat16* tap(long off) const { return wtap.as<__nv_bfloat16>() + off; }
 
   const float* src_a_ptr(int i) const {
     const int sa = kSrcA[i];
@@ -853,7 +990,7 @@ struct Net {
 
   void conv_forward(int i, int n) {
     const Conv& c = convs[i];
-    ConvArgs ga{src_a_ptr(i), nullptr, c.ca, c.a_up, src_b_ptr(i), c.cb, wb(c), p.as<float>() + c.b_off,
+    ConvArgs ga{src_a_ptr(i), nullptr, c.ca, c.a_up, src_b_ptr(i), c.cb, wb(c), tap(c.tap_f), p.as<float>() + c.b_off,
                 act[i + 1].as<float>(), c.cout, lvH(c.level), lvW(c.level), 1, nullptr, c.cout};
     conv(ga, n);
   }
@@ -912,11 +1049,13 @@ struct Net {
     // data: the transposed convolution of the masked gradient, straight into
     // the producers' gradients (it is the first, for all but e1..e3 the only
     // contribution to each; those get their pool's afterwards)
-    k_flip_transpose<<<cdiv(len, 256), 256, 0, s>>>(wb(c), c.cout, cin, wt.as<__nv_bfloat16>());
-    UN_LAUNCH();
+    if (cuda_cores) {
+      k_flip_transpose<<<cdiv(len, 256), 256, 0, s>>>(wb(c), c.cout, cin, wt.as<__nv_bfloat16>());
+      UN_LAUNCH();
+    }
     float* ga_dst = src_a_grad(i);
     float* gb_dst = c.cb ? gact[src_b(i)].as<float>() : nullptr;
-    ConvArgs gd{go, mask, c.cout, 0, nullptr, 0, wt.as<__nv_bfloat16>(), nullptr, c.a_up ? gup.as<float>() : ga_dst, cin,
+    ConvArgs gd{go, mask, c.cout, 0, nullptr, 0, wt.as<__nv_bfloat16>(), tap(c.tap_b), nullptr, c.a_up ? gup.as<float>() : ga_dst, cin,
                 Hl, Wl, 0, gb_dst, c.ca};
     conv(gd, n);
     if (c.a_up) {  // sum the 2x2 blocks into a's half-resolution gradient
@@ -1062,7 +1201,7 @@ int mfista_unet_train_step(void* net, const float* in, const float* target, int 
     const float c1 = 1.f - powf(b1, (float)N->step), c2 = 1.f - powf(b2, (float)N->step);
     unet::k_adam<<<unet::cdiv(N->nparam, 256), 256, 0, N->s>>>(
         N->p.as<float>(), N->g.as<float>(), N->m.as<float>(), N->v.as<float>(), N->nparam, lr, b1, b2, 1e-8f, c1,
-        c2, N->wbf.as<__nv_bfloat16>(), N->wmap.as<int>());
+        c2, N->wbf.as<__nv_bfloat16>(), N->wtap.as<__nv_bfloat16>(), N->wmap.as<int>());
     UN_LAUNCH();
     const float l = N->loss(n);
     if (loss) *loss = l;

@@ -31,3 +31,24 @@ def test_gradient_sums_match_oracle(gpulib, monkeypatch, h, n, cores):
         assert rel(g[w0:b0], g_ref[w0:b0]) < 1e-3
         assert rel(g[b0:b0 + 16], g_ref[b0:b0 + 16]) < 1e-3
     net.close()
+
+
+@pytest.mark.parametrize("h", [24, 72])  # widths 3 and 9 at the coarsest level
+def test_weight_copies_follow_training(gpulib, h):
+    """The convolutions' rounded weight copies after training steps are those of
+    the parameters: a fresh net with them gives the same output and gradient."""
+    from sparseimaging_b200 import warmstart
+    rng = np.random.default_rng(h)
+    x = rng.standard_normal((2, 2, h, h)).astype(np.float32)
+    t = np.abs(rng.standard_normal((2, h, h))).astype(np.float32)
+    net, fresh = warmstart.UNet(h, h, 2), warmstart.UNet(h, h, 2)
+    for _ in range(3):
+        net.train_step(x, t, 1e-3)
+    before = fresh.forward(x)
+    fresh.set_params(net.params())
+    y = net.forward(x)
+    assert not np.array_equal(y, before)
+    np.testing.assert_array_equal(y, fresh.forward(x))
+    np.testing.assert_array_equal(net.grad(x, t)[1], fresh.grad(x, t)[1])
+    net.close()
+    fresh.close()
