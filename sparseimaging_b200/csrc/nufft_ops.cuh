@@ -1037,6 +1037,11 @@ template <int N> __device__ __forceinline__ void cp_async_wait() {
 // relative per product, the accuracy of FP32 sums over the 576 taps).  The
 // epilogue is the one of k_nufft_interp_group: FP64 residual, chi^2, the
 // models of the corrected form.
+// With 20 points a CTA on average the staging weighs as much as the products
+// (which split each value about as often as it is staged).  At 128 x 128 with
+// 64 problems: 142 us with index arithmetic and eight loads a cell one cell
+// at a time, 119 us with the column's part found once and two cells' loads in
+// flight.
 // ---------------------------------------------------------------------------
 constexpr int kItcTile = 8;    // home tile (first-tap positions per axis)
 constexpr int kItcWin = 32;    // window cells per axis
@@ -1123,44 +1128,50 @@ static __global__ void __launch_bounds__(256, 3) k_nufft_interp_tc(
       fa[kk][q] = ((second ? vb : va) && jy >= 0 && jy < kTaps)
                       ? geo.wy[(size_t)(second ? kb : ka) * kTaps + jy] : 0.f;
     }
-  // the window: virtual cell -> stored cell, sign of the imaginary part
-  for (int v = threadIdx.x; v < kItcWin * kItcWin; v += blockDim.x) {
-    const int vr = tl.row0 + (v >> 5), vc = tl.col0 + (v & 31);
-    int cell = -1;
-    float sgn = -1.f;  // NU_SIGN on direct taps
-    int col = half_col(vc, ny);
-    if (col >= 0) {
-      const int row = wrap_row(vr, nx);
-      if (row >= 0) cell = row * (ny + 1) + col;
-    } else {
-      col = half_col(-vc, ny);
-      const int row = wrap_row(-vr, nx);
-      if (col >= 0 && row >= 0) {
-        cell = row * (ny + 1) + col;
-        sgn = 1.f;
-      }
-    }
-    float* dst = s_g + (size_t)v * (2 * kItcProb);
-    const int sw = itc_swz(v & 31);
+  // the window: virtual cell -> stored cell, sign of the imaginary part.  A
+  // thread's four cells lie in one column, so its column's fold and the order
+  // in which it takes the problem pairs are found once, and the loads of two
+  // cells are in flight together
+  {
+    const int vc = tl.col0 + lane;
+    const bool direct = half_col(vc, ny) >= 0;
+    const int col = direct ? half_col(vc, ny) : half_col(-vc, ny);
+    const float sgn = direct ? -1.f : 1.f;  // NU_SIGN on direct taps
+    const int sw = itc_swz(lane);
     // the four 16-byte stores of a cell in an order rotated by the cell, so
     // that the 32 lanes of a store instruction cover all banks
+    const int rot = (lane >> 1) & 3;
+    size_t base[kItcProb];  // problem of pair q4, member h
 #pragma unroll
-    for (int q4 = 0; q4 < 4; ++q4) {
-      const int s = 2 * ((q4 + (v >> 1)) & 3);
-      float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (cell >= 0) {
-        if (s < nact) {
-          const cplx<float> a = gall[(size_t)s_list[s] * gstride + cell];
-          q.x = a.x;
-          q.y = sgn * a.y;
-        }
-        if (s + 1 < nact) {
-          const cplx<float> a = gall[(size_t)s_list[s + 1] * gstride + cell];
-          q.z = a.x;
-          q.w = sgn * a.y;
+    for (int q = 0; q < kItcProb; ++q) {
+      const int sl = 2 * (((q >> 1) + rot) & 3) + (q & 1);
+      base[q] = sl < nact ? (size_t)s_list[sl] * gstride : (size_t)-1;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i += 2) {
+      cplx<float> a[2][kItcProb];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int vr = tl.row0 + warp + 8 * (i + e);
+        const int row = direct ? wrap_row(vr, nx) : wrap_row(-vr, nx);
+        const bool ok = col >= 0 && row >= 0;
+        const size_t cell = ok ? (size_t)row * (ny + 1) + col : 0;
+#pragma unroll
+        for (int q = 0; q < kItcProb; ++q) {
+          a[e][q] = mk<float>(0.f, 0.f);
+          if (ok && base[q] != (size_t)-1) a[e][q] = gall[base[q] + cell];
         }
       }
-      *reinterpret_cast<float4*>(dst + ((2 * s) ^ sw)) = q;
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        float* dst = s_g + (size_t)((warp + 8 * (i + e)) * kItcWin + lane) * (2 * kItcProb);
+#pragma unroll
+        for (int q4 = 0; q4 < 4; ++q4) {
+          const cplx<float> u = a[e][2 * q4], w = a[e][2 * q4 + 1];
+          *reinterpret_cast<float4*>(dst + ((4 * ((q4 + rot) & 3)) ^ sw)) =
+              make_float4(u.x, sgn * u.y, w.x, sgn * w.y);
+        }
+      }
     }
   }
   if (lane < kItcProb) s_chi[warp][lane] = 0.0;
@@ -1305,6 +1316,9 @@ static __global__ void __launch_bounds__(256, 3) k_nufft_interp_tc(
 // finish (a ticket per tile and problem chunk) adds the segments in segment
 // order and writes the tile, so the result does not depend on the order the
 // CTAs ran in.
+// The gather of the residuals is the part that is not matrix products: a value
+// at a time, list entry before residual, the launch took 125 us at 128 x 128
+// with 64 problems; an entry per thread, its problems' loads together, 105 us.
 // ---------------------------------------------------------------------------
 constexpr int kStcRows = 8, kStcCols = 16;
 constexpr int kStcProb = 8;   // problems per CTA (16 real columns)
@@ -1378,7 +1392,7 @@ static __global__ void __launch_bounds__(256) k_nufft_spread_tc(
     const float4* __restrict__ afrag, const float* __restrict__ bxg, const cplx<float>* __restrict__ y2,
     cplx<float>* __restrict__ gall, long gstride, int nx, int ny, int ntcol, const ProbState* __restrict__ st,
     int gate, int B, float* __restrict__ scratch, unsigned int* __restrict__ tickets) {
-  __shared__ float s_y[kStcSeg * 24];  // [entry][16 problem columns] (row stride 24: conflict-free B loads)
+  __shared__ __align__(16) float s_y[kStcSeg * 24];  // [entry][16 problem columns] (row stride 24: conflict-free B loads)
   __shared__ int s_list[kStcProb];
   __shared__ int s_cnt[8];
   __shared__ unsigned int s_ticket;
@@ -1392,15 +1406,21 @@ static __global__ void __launch_bounds__(256) k_nufft_spread_tc(
   const int nj = nact > 4 ? 2 : 1;
   // the chunk's half residuals of the segment's entries, imaginary sign of
   // direct / mirrored taps (the only data that changes between launches)
-  for (int e = threadIdx.x; e < it.count * 2 * kStcProb; e += blockDim.x) {
-    const int q = e >> 4, n = e & 15, sl = n >> 1;
-    float v = 0.f;
-    const int code = vlist[it.start + q];
-    if (code >= 0 && sl < nact) {
-      const cplx<float> r = y2[(size_t)s_list[sl] * geo.y2_bstride + (code & 0xffffff)];
-      v = (n & 1) ? (((code >> 24) & 1) ? 0.5f * r.y : -0.5f * r.y) : 0.5f * r.x;
+  // (an entry per thread, its problems' loads in flight together)
+  static_assert(kStcSeg <= 256, "an entry per thread");
+  if ((int)threadIdx.x < it.count) {
+    const int q = threadIdx.x, code = vlist[it.start + q];
+    cplx<float> r[kStcProb];
+#pragma unroll
+    for (int sl = 0; sl < kStcProb; ++sl) {
+      r[sl] = mk<float>(0.f, 0.f);
+      if (code >= 0 && sl < nact) r[sl] = y2[(size_t)s_list[sl] * geo.y2_bstride + (code & 0xffffff)];
     }
-    s_y[q * 24 + n] = v;
+    const float im = ((code >> 24) & 1) ? 0.5f : -0.5f;
+#pragma unroll
+    for (int sl = 0; sl < kStcProb; sl += 2)
+      *reinterpret_cast<float4*>(s_y + q * 24 + 2 * sl) =
+          make_float4(0.5f * r[sl].x, im * r[sl].y, 0.5f * r[sl + 1].x, im * r[sl + 1].y);
   }
   __syncthreads();
   float d[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
