@@ -1,4 +1,6 @@
 // Shared-memory mixed-radix Stockham FFT, executed cooperatively by a CTA.
+// The transforms of the FP32 operators; FP64 runs through registers
+// (fft_reg.cuh), which would round differently here.
 //
 // `count` independent transforms of length n live in shared memory at
 // data[t*ld + k]; every stage reads one buffer and writes the other

@@ -17,12 +17,13 @@
 //
 // Measured on B200, FP64, microseconds per launch, tap by tap -> here:
 //   grid, points, problems          interpolation    spreading
-//   64 x 64, 2016, 1                 40.1 -> 12.4     37.0 -> 10.6
-//   128 x 128, 8100, 1               39.7 -> 12.4     60.6 -> 14.5
-//   128 x 128, 8100, 64               489 -> 187       581 -> 199
-//   256 x 256, 19998, 64             1130 -> 486      1710 -> 508
-//   128 x 128, 102070 over 16 frames  163 -> 54        605 -> 123
-// The products alone would take 87 us and 80 us at 128 x 128 with 64 problems.
+//   64 x 64, 2016, 1                 40.1 -> 7.3      37.0 -> 10.4
+//   128 x 128, 8100, 1               39.7 -> 10.2     60.6 -> 14.5
+//   128 x 128, 8100, 64               489 -> 170       581 -> 142
+//   256 x 256, 19998, 64             1130 -> 471      1710 -> 361
+//   128 x 128, 102070 over 16 frames  163 -> 50        605 -> 117
+// The products alone would take 60 us and 80 us at 128 x 128 with 64 problems;
+// a copy of the interpolation without them takes 51 us.
 #pragma once
 #include "nufft_ops.cuh"
 

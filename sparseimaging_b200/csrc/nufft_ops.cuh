@@ -6,11 +6,14 @@
 //   * the centred zero padding and the E4 grid correction are fused into the
 //     first (row) pass of the r2c FFT and the last (row) pass of the c2r FFT,
 //     and both column passes skip the all-zero half of the padded image;
-//   * interpolation (NUFFT2d2) is one warp per uv point, 576 taps over the 32
-//     lanes, complex grid cells read as one 8/16-byte vector;
-//   * spreading (NUFFT2d1) is output-stationary: every CTA owns a tile of
-//     the half-plane grid and gathers the taps of the points binned to it, so
-//     there are no atomics and the result is deterministic.
+//   * interpolation (NUFFT2d2) and spreading (NUFFT2d1) are matrix products:
+//     TF32 pairs here for FP32 operators that share their points
+//     (k_nufft_interp_tc, k_nufft_spread_tc), FP64 in nufft_mma.cuh for the
+//     others; the tap-by-tap kernels (one warp per uv point, 576 taps over
+//     the lanes) are kept for comparison runs;
+//   * spreading is output-stationary: every CTA owns a tile of the half-plane
+//     grid and gathers the taps of the points binned to it, so there are no
+//     atomics and the result is deterministic.
 #pragma once
 #include <cooperative_groups.h>
 #include "common.cuh"
