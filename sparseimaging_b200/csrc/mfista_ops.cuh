@@ -119,7 +119,7 @@ __global__ void k_update_tsv(const double* __restrict__ zall, const double* __re
       v[4] = tsv_pairs_at(z, f, dm.NX, dm.NY);
     }
   }
-  block_sum<5>(v, sh);
+  block_sum5(v, sh);
   if (threadIdx.x == 0) {
     part.at(kQDq1, b)[blockIdx.x] = v[0];
     part.at(kQDq2, b)[blockIdx.x] = v[1];
@@ -160,7 +160,7 @@ __global__ void k_stats(const double* __restrict__ vall, const double* __restric
       acc[1] = df * df;
     }
   }
-  block_sum<5>(acc, sh);
+  block_sum5(acc, sh);
   if (threadIdx.x == 0) {
     if (want_q) {
       part.at(kQDq1, b)[blockIdx.x] = acc[0];
