@@ -73,10 +73,12 @@ __global__ void __launch_bounds__(128, 3) k_looe_gram(const double* __restrict__
 }
 
 // H = sum of the splits (in order), lower triangle, plus lambda_tsv d2(S_j) on
-// the diagonal (TSV form); H may be split 0 itself
+// the diagonal (TSV form); grid: ns columns of cdiv(ns, blockDim.x) CTAs each,
+// in x (y ends at 65535, and there may be more columns)
 __global__ void k_looe_gram_sum(const double* __restrict__ part, int nsplit, double* __restrict__ H,
                                 const int* __restrict__ S, int ns, int nx, double lam) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y;
+  const int nb = (ns + (int)blockDim.x - 1) / (int)blockDim.x;
+  const int j = blockIdx.x / nb, i = (blockIdx.x - j * nb) * blockDim.x + threadIdx.x;
   if (i >= ns || i < j) return;
   const size_t e = (size_t)i + (size_t)j * ns;
   double h = 0.0;
@@ -535,7 +537,7 @@ struct Looe {
       MF_LAUNCH_CK();
       k_looe_gram<<<dim3(tiles, nsplit), 128, dg::kSmem, s>>>(A, M, S, ns, kchunk, Hs);
       MF_LAUNCH_CK();
-      k_looe_gram_sum<<<dim3(cdiv(ns, 256), ns), 256, 0, s>>>(Hs, nsplit, H, pix, ns, NX, lam_tsv);
+      k_looe_gram_sum<<<(unsigned int)cdiv(ns, 256) * ns, 256, 0, s>>>(Hs, nsplit, H, pix, ns, NX, lam_tsv);
       MF_LAUNCH_CK();
       for (int k0 = 0; k0 < ns; k0 += kPanel) {
         const int nb = std::min(kPanel, ns - k0), nt = cdiv(ns - k0 - nb, kPanel);
