@@ -52,10 +52,10 @@ __device__ __forceinline__ void lower_tile(int e, int& ti, int& tj) {
   tj = e - ti * (ti + 1) / 2;
 }
 
-// lower tiles of A_S^T A_S over the K range of split blockIdx.y: part
-// [split][n_s x n_s]; grid (lower tiles, splits)
+// lower tiles of A_S^T A_S over the K range of split blockIdx.y: split 0 into H,
+// split q > 0 into part[q - 1], n_s x n_s each; grid (lower tiles, splits)
 __global__ void __launch_bounds__(128, 3) k_looe_gram(const double* __restrict__ A, int M, const int* __restrict__ S,
-                                                      int ns, int kchunk, double* __restrict__ part) {
+                                                      int ns, int kchunk, double* __restrict__ H0, double* __restrict__ part) {
   extern __shared__ __align__(16) double looe_smem[];
   int ti, tj;
   lower_tile(blockIdx.x, ti, tj);
@@ -65,15 +65,15 @@ __global__ void __launch_bounds__(128, 3) k_looe_gram(const double* __restrict__
   dg::clear(acc);
   const int k0 = blockIdx.y * kchunk;
   dg::tile_product_nb<8>(X, Y, k0, min(M, k0 + kchunk), looe_smem, acc);
-  double* H = part + (size_t)blockIdx.y * ns * ns;
+  double* H = blockIdx.y ? part + (size_t)(blockIdx.y - 1) * ns * ns : H0;
   dg::each(acc, [&](int r, int c, double v) {
     const int i = ti * kPanel + r, j = tj * kPanel + c;
     if (i < ns && j < ns) H[(size_t)i + (size_t)j * ns] = v;
   });
 }
 
-// H = sum of the splits (in order), lower triangle, plus lambda_tsv d2(S_j) on
-// the diagonal (TSV form); grid: ns columns of cdiv(ns, blockDim.x) CTAs each,
+// H += the splits behind the first (in order), lower triangle, plus lambda_tsv
+// d2(S_j) on the diagonal (TSV form); grid: ns columns of cdiv(ns, blockDim.x) CTAs each,
 // in x (y ends at 65535, and there may be more columns)
 __global__ void k_looe_gram_sum(const double* __restrict__ part, int nsplit, double* __restrict__ H,
                                 const int* __restrict__ S, int ns, int nx, double lam) {
@@ -81,8 +81,8 @@ __global__ void k_looe_gram_sum(const double* __restrict__ part, int nsplit, dou
   const int j = blockIdx.x / nb, i = (blockIdx.x - j * nb) * blockDim.x + threadIdx.x;
   if (i >= ns || i < j) return;
   const size_t e = (size_t)i + (size_t)j * ns;
-  double h = 0.0;
-  for (int q = 0; q < nsplit; ++q) h += part[(size_t)q * ns * ns + e];
+  double h = H[e];
+  for (int q = 0; q < nsplit - 1; ++q) h += part[(size_t)q * ns * ns + e];
   if (i == j && lam != 0.0) {
     const int pix = S[j], r = pix % nx, c = pix / nx;
     const bool ri = r > 0 && r < nx - 1, ci = c > 0 && c < nx - 1;
@@ -487,10 +487,13 @@ struct Looe {
     };
     int splits = 1;
     size_t hs = 0;
-    for (int n = 1, np = cdiv(ns, kPanel); n <= np; ++n) {  // a smaller solution may have more splits
+    // splits behind the first: none above 62 panels (3968 pixels) on 148 SMs, so
+    // they take at most 0.4 GB beside H, which is held once.  (A smaller
+    // solution may have more splits.)
+    for (int n = 1, np = cdiv(ns, kPanel); n <= np; ++n) {
       const size_t m = std::min((size_t)n * kPanel, (size_t)ns);
       splits = gram_splits(n * (n + 1) / 2);
-      hs = std::max(hs, splits * m * m);
+      hs = std::max(hs, (size_t)(splits - 1) * m * m);
     }
     l.xs = take(ns);
     l.ax = take(kSplitR * (size_t)M);
@@ -535,10 +538,12 @@ struct Looe {
       const double* A = d_A.as<double>();
       k_looe_ax<<<dim3(cdiv(M, 256), kSplitR), 256, 0, s>>>(A, M, S, m + l.xs, ns, m + l.ax);
       MF_LAUNCH_CK();
-      k_looe_gram<<<dim3(tiles, nsplit), 128, dg::kSmem, s>>>(A, M, S, ns, kchunk, Hs);
+      k_looe_gram<<<dim3(tiles, nsplit), 128, dg::kSmem, s>>>(A, M, S, ns, kchunk, H, Hs);
       MF_LAUNCH_CK();
-      k_looe_gram_sum<<<(unsigned int)cdiv(ns, 256) * ns, 256, 0, s>>>(Hs, nsplit, H, pix, ns, NX, lam_tsv);
-      MF_LAUNCH_CK();
+      if (nsplit > 1 || lam_tsv != 0.0) {
+        k_looe_gram_sum<<<(unsigned int)cdiv(ns, 256) * ns, 256, 0, s>>>(Hs, nsplit, H, pix, ns, NX, lam_tsv);
+        MF_LAUNCH_CK();
+      }
       for (int k0 = 0; k0 < ns; k0 += kPanel) {
         const int nb = std::min(kPanel, ns - k0), nt = cdiv(ns - k0 - nb, kPanel);
         double* W = m + l.W + (size_t)(k0 / kPanel) * kPanel * kPanel;

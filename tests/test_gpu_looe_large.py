@@ -5,6 +5,8 @@ With fewer visibilities than pixels, H = A^T A + lambda D (D the curvature of
 the TSV term) and the leverages follow from an M x M system alone
 (Woodbury): with G = A D^-1 A^T / lambda, A H^-1 A^T = (I + G)^-1 G."""
 
+import threading
+
 import numpy as np
 import pytest
 
@@ -39,3 +41,31 @@ def test_more_active_pixels_than_grid_rows(gpulib, nx, active):
     wm, ws = _expected(A, x, S, y, nx, 2.0)
     assert pos[0]
     assert abs(mean[0] - wm) <= 1e-9 * wm and abs(std[0] - ws) <= 1e-9 * ws
+
+
+def test_hessian_is_held_once(gpulib):
+    """8281 active pixels, 0.55 GB of Hessian (its product is not split at this
+    size): a call's largest device memory, read while it runs."""
+    import torch
+    nx = 91
+    A, x, S, y = _case(nx, nx * nx, 6, 2)
+    call = lambda: gpulib.dft_looe(y, A, x[None], nx, lambda_tsv=[2.0])
+    mean, std, pos = call()
+    wm, ws = _expected(A, x, S, y, nx, 2.0)
+    assert pos[0] and abs(mean[0] - wm) <= 1e-9 * wm and abs(std[0] - ws) <= 1e-9 * ws
+    torch.cuda.synchronize()
+    before, least, done = torch.cuda.mem_get_info()[0], [], threading.Event()
+
+    def watch():
+        while not done.is_set():
+            least.append(torch.cuda.mem_get_info()[0])
+
+    w = threading.Thread(target=watch)
+    w.start()
+    for _ in range(3):
+        call()
+    done.set()
+    w.join()
+    hessian = 8 * len(S) ** 2
+    used = before - min(least)
+    assert hessian <= used < 1.5 * hessian
