@@ -34,6 +34,7 @@
 // 19 x 7 us.  A call with three solutions: 32 ms -> 8.9 ms.
 #pragma once
 
+#include "column_runs.h"
 #include "dgemm_mma.cuh"
 #include "solver.cuh"
 
@@ -366,8 +367,8 @@ __global__ void k_looe_final(const double* __restrict__ part, int nblk, int M, c
 // column-major M x N); lambda_tsv per solution (null: 0).  Kernels per
 // solution: 6 + 3 ceil(n_s / 64).
 //
-// Only the columns of A that some solution uses go to the device, in runs (a
-// gap of at most kGap columns is copied along rather than splitting a copy).
+// Only the columns of A that some solution uses go to the device, in runs
+// (column_runs.h).
 // Solutions run on up to kLanes streams, each with its own scratch: one
 // solution's factorisation is a chain of small kernels (840 of 2190 us at 1261
 // active pixels) and its other kernels leave SMs idle, which the next one's
@@ -375,7 +376,7 @@ __global__ void k_looe_final(const double* __restrict__ part, int nblk, int M, c
 // kLaneBytes, and given up when their memory cannot be had; the results do
 // not depend on them.
 struct Looe {
-  static constexpr int kLanes = 4, kGap = 2;
+  static constexpr int kLanes = 4;
   static constexpr size_t kLaneBytes = (size_t)1 << 30;
 
   struct Lane {
@@ -415,24 +416,15 @@ struct Looe {
         }
       most = std::max(most, n);
     }
-    for (int j = 0, last = -1; j < N; ++j)
-      if (used[j]) {
-        if (last >= 0 && j - last <= kGap + 1) std::fill(used.begin() + last, used.begin() + j, 1);
-        last = j;
-      }
+    const std::vector<ColumnRun> runs = column_runs(used, sizeof(double) * M);
     col.assign(N, 0);
     int nc = 0;
-    for (int j = 0; j < N; ++j)
-      if (used[j]) col[j] = nc++;
+    for (const ColumnRun& r : runs)
+      for (int j = r.first; j < r.last; ++j) col[j] = nc++;
     d_A.alloc(sizeof(double) * (size_t)M * nc);
-    for (int j = 0; j < N;) {
-      int e = j;
-      while (e < N && used[e]) ++e;
-      if (e > j)
-        MF_CK(cudaMemcpy(d_A.as<double>() + (size_t)col[j] * M, A + (size_t)j * M, sizeof(double) * (size_t)(e - j) * M,
-                         cudaMemcpyHostToDevice));
-      j = e + 1;
-    }
+    for (const ColumnRun& r : runs)
+      MF_CK(cudaMemcpy(d_A.as<double>() + (size_t)col[r.first] * M, A + (size_t)r.first * M,
+                       sizeof(double) * (size_t)(r.last - r.first) * M, cudaMemcpyHostToDevice));
     d_y.upload(y, (size_t)M);
     MF_CK(cudaStreamSynchronize(nullptr));  // the lanes' streams do not wait for the copies' last part
     set_smem(k_looe_gram, dg::kSmem);
