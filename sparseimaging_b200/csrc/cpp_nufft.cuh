@@ -300,7 +300,7 @@ struct CppNufftOp : Op {
     Prep pr(u, v, M, nx, ny);
     std::vector<double> zero(M, 0.0), one(M, 1.0);
     NufftInput in{u, v, zero.data(), zero.data(), one.data(), nullptr, 1, M, nx, ny};
-    fft.reset(new NufftOp<double>(ctx, in));
+    fft.reset(new NufftOp<double>(ctx, in, false, true));
     d_e4.upload(pr.e4.data(), pr.e4.size());
     d_mx.upload(pr.mx.data(), M);
     d_my.upload(pr.my.data(), M);

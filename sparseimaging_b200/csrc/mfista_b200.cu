@@ -744,7 +744,7 @@ int nufft_apply(const double* u, const double* v, const double* wstd, int M, int
   S.init_common(1, Nx * Ny, Nx, Ny, kFormTSV, 100, nullptr);
   std::vector<double> zero(std::max(M, 1), 0.0), one(std::max(M, 1), 1.0);
   NufftInput in{u, v, zero.data(), zero.data(), wstd ? wstd : one.data(), nullptr, 1, M, Nx, Ny};
-  NufftOp<T>* op = new NufftOp<T>(S.ctx, in);
+  NufftOp<T>* op = new NufftOp<T>(S.ctx, in, false, x != nullptr);
   S.op.reset(op);
   int slots = std::max({op->chi_slots(), op->tsv_slots(), 1});
   S.d_part.alloc(sizeof(double) * (size_t)kNumQ * slots);

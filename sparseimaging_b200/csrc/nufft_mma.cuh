@@ -352,12 +352,16 @@ __global__ void __launch_bounds__(256, 2)
 // both parities to a warp and two CTAs.  Each block's sum is the even steps'
 // plus the odd steps' whatever the mapping, and longer lists are cut into
 // segments whose partial tiles the tile's last CTA adds in segment order, so
-// neither the batch nor the order of the CTAs changes a result.
+// neither the batch nor the order of the CTAs changes a result.  A segment is
+// kSmSeg entries, or as many times that (staged one after another) as leave
+// at most kSmSegMax partial tiles, 2 KB each, to a problem: the scratch stays
+// within 8 MB a problem, where it would be 75 bytes a point and problem.
 // The weights are read where they lie (48 values a point, shared by the tiles
 // around it): cached, with the taps outside [0, 24) as zeros.
 // ---------------------------------------------------------------------------
 constexpr int kSmRows = 8, kSmCols = 16;
-constexpr int kSmSeg = 256;  // list entries per CTA at most
+constexpr int kSmSeg = 256;  // list entries staged at once
+constexpr int kSmSegMax = 4096;  // partial tiles of a problem at most
 
 struct SmItem {
   int tile;          // tile of the stored half grid, row-major
@@ -430,7 +434,9 @@ __device__ __forceinline__ void spread_products(const SmPoint* s_pt, const doubl
   }
 }
 
-template <typename T, int PB>
+// kLong: there are segments of more than kSmSeg entries (an instance of its
+// own: with the loop the others take 2-5 % longer)
+template <typename T, int PB, bool kLong>
 __global__ void __launch_bounds__(256, PB > 1 ? 3 : 2)
     k_nufft_spread_mma(NufftGeom<T> geo, const double* __restrict__ wxd, const double* __restrict__ wyd,
                        const SmItem* __restrict__ items, const unsigned int* __restrict__ vlist,
@@ -458,29 +464,6 @@ __global__ void __launch_bounds__(256, PB > 1 ? 3 : 2)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int tr = it.tile / ntcol, tcl = it.tile - tr * ntcol;
   const int row_base = tr * kSmRows, col_base = tcl * kSmCols;
-  for (int e = threadIdx.x; e < it.count * nact; e += blockDim.x) {
-    const int i = e / it.count, q = e - i * it.count;
-    const unsigned int code = vlist[it.start + q];
-    double2 y = make_double2(0.0, 0.0);
-    if (code != 0xffffffffu) {
-      const int k = (int)(code >> 1);
-      const cplx<T> r = y2[(size_t)s_list[i] * geo.y2_bstride + k];
-      y = make_double2(0.5 * (double)r.x, (code & 1u) ? 0.5 * (double)r.y : -0.5 * (double)r.y);
-    }
-    s_y[(size_t)i * kSmSeg + q] = y;
-    if (i == 0) {
-      SmPoint p{0, 1 << 29, 1 << 29, 0};  // an empty entry: no tap anywhere
-      if (code != 0xffffffffu) {
-        const int k = (int)(code >> 1), fl = (int)(code & 1u);
-        p.k24 = (unsigned int)k * kTaps;
-        p.x0 = fl ? -geo.mx[k] - kMSP : geo.mx[k] - (kMSP - 1);
-        p.y0 = fl ? -geo.my[k] - kMSP : geo.my[k] - (kMSP - 1);
-        p.fl = fl;
-      }
-      s_pt[q] = p;
-    }
-  }
-  __syncthreads();
   // warps over (pair of problems, blocks of the tile, parity of the steps):
   // the fewer pairs, the fewer blocks a warp takes
   const int ch = warp & 1, groups = nact > 4 ? 1 : nact > 2 ? 2 : 4;
@@ -493,23 +476,50 @@ __global__ void __launch_bounds__(256, PB > 1 ? 3 : 2)
 #pragma unroll
     for (int m = 0; m < 4; ++m) acc[q][m][0] = acc[q][m][1] = 0.0;
   const double2* yp = s_y + (size_t)2 * pair * kSmSeg;
-  if (PB > 1 && groups == 1) {
-    if (np == 2)
-      spread_products<2, 2, 2>(s_pt, yp, it.count, 0, 0, ch, row_base, col_base, nx, ny, lane, wxd, wyd, acc);
-    else if (np == 1)
-      spread_products<2, 2, 1>(s_pt, yp, it.count, 0, 0, ch, row_base, col_base, nx, ny, lane, wxd, wyd, acc);
-  } else if (PB > 1 && groups == 2) {
-    if (np == 2)
-      spread_products<1, 2, 2>(s_pt, yp, it.count, sub, 0, ch, row_base, col_base, nx, ny, lane, wxd, wyd, acc);
-    else if (np == 1)
-      spread_products<1, 2, 1>(s_pt, yp, it.count, sub, 0, ch, row_base, col_base, nx, ny, lane, wxd, wyd, acc);
-  } else {
-    if (PB > 1 && np == 2)
-      spread_products<1, 1, 2>(s_pt, yp, it.count, sub >> 1, sub & 1, ch, row_base, col_base, nx, ny, lane, wxd, wyd,
-                               acc);
-    else if (np == 1)
-      spread_products<1, 1, 1>(s_pt, yp, it.count, sub >> 1, sub & 1, ch, row_base, col_base, nx, ny, lane, wxd, wyd,
-                               acc);
+  for (int base = 0; base < (kLong ? it.count : 1); base += kSmSeg) {
+    const int cnt = kLong ? min(kSmSeg, it.count - base) : it.count;
+    if (base) __syncthreads();  // the entries before have been read
+    for (int e = threadIdx.x; e < cnt * nact; e += blockDim.x) {
+      const int i = e / cnt, q = e - i * cnt;
+      const unsigned int code = vlist[it.start + base + q];
+      double2 y = make_double2(0.0, 0.0);
+      if (code != 0xffffffffu) {
+        const int k = (int)(code >> 1);
+        const cplx<T> r = y2[(size_t)s_list[i] * geo.y2_bstride + k];
+        y = make_double2(0.5 * (double)r.x, (code & 1u) ? 0.5 * (double)r.y : -0.5 * (double)r.y);
+      }
+      s_y[(size_t)i * kSmSeg + q] = y;
+      if (i == 0) {
+        SmPoint p{0, 1 << 29, 1 << 29, 0};  // an empty entry: no tap anywhere
+        if (code != 0xffffffffu) {
+          const int k = (int)(code >> 1), fl = (int)(code & 1u);
+          p.k24 = (unsigned int)k * kTaps;
+          p.x0 = fl ? -geo.mx[k] - kMSP : geo.mx[k] - (kMSP - 1);
+          p.y0 = fl ? -geo.my[k] - kMSP : geo.my[k] - (kMSP - 1);
+          p.fl = fl;
+        }
+        s_pt[q] = p;
+      }
+    }
+    __syncthreads();
+    if (PB > 1 && groups == 1) {
+      if (np == 2)
+        spread_products<2, 2, 2>(s_pt, yp, cnt, 0, 0, ch, row_base, col_base, nx, ny, lane, wxd, wyd, acc);
+      else if (np == 1)
+        spread_products<2, 2, 1>(s_pt, yp, cnt, 0, 0, ch, row_base, col_base, nx, ny, lane, wxd, wyd, acc);
+    } else if (PB > 1 && groups == 2) {
+      if (np == 2)
+        spread_products<1, 2, 2>(s_pt, yp, cnt, sub, 0, ch, row_base, col_base, nx, ny, lane, wxd, wyd, acc);
+      else if (np == 1)
+        spread_products<1, 2, 1>(s_pt, yp, cnt, sub, 0, ch, row_base, col_base, nx, ny, lane, wxd, wyd, acc);
+    } else {
+      if (PB > 1 && np == 2)
+        spread_products<1, 1, 2>(s_pt, yp, cnt, sub >> 1, sub & 1, ch, row_base, col_base, nx, ny, lane, wxd, wyd,
+                                 acc);
+      else if (np == 1)
+        spread_products<1, 1, 1>(s_pt, yp, cnt, sub >> 1, sub & 1, ch, row_base, col_base, nx, ny, lane, wxd, wyd,
+                                 acc);
+    }
   }
   // even plus odd steps: warp c of the two parities keeps the pair's problem c
   // and hands over the other

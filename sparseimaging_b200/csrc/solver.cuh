@@ -325,6 +325,7 @@ template <typename T> struct NufftOp : Op {
   DevMem d_im, d_imperm, d_smitems, d_smlist, d_smscratch, d_smtickets;
   DevMem d_wxd, d_wyd;  // FP64 weights of an FP32 operator (wxd(), wyd())
   int nim = 0, im_chunks = 1, nsm = 0, sm_cols = 0;
+  bool sm_long = false;  // some problem's lists are cut at more than kSmSeg entries
   // chi^2 partial slots every interpolation kernel of this operator writes
   // (at least its own CTA count; the extra CTAs write zeros), so that the
   // CUDA-core, tensor-core and FP64 kernels fill the same slots
@@ -637,7 +638,8 @@ template <typename T> struct NufftOp : Op {
 
   // k_nufft_spread_mma's tiles and lists: per stored tile the virtual points
   // (point << 1 | mirrored) with a tap on it, in (point, mirrored) order,
-  // padded with empty entries to a multiple of 8 and cut into segments.
+  // padded with empty entries to a multiple of 8 and cut into segments, whose
+  // length follows from the problem's own points.
   void build_sm_items(const std::vector<int>& mx, const std::vector<int>& my, const std::vector<int>& lo,
                       const std::vector<int>& hi) {
     const int ntr = cdiv(2 * nx, kSmRows);
@@ -692,13 +694,22 @@ template <typename T> struct NufftOp : Op {
       };
       std::fill(cnt.begin(), cnt.end(), 0);
       each([&](int t, unsigned int) { ++cnt[t]; });
+      auto partials = [&](int len) {  // of lists cut at len entries
+        long n = 0;
+        for (int t = 0; t < nt; ++t)
+          if (cnt[t] > len) n += cdiv(cnt[t], len);
+        return n;
+      };
+      int len = kSmSeg;
+      while (partials(len) > kSmSegMax) len += kSmSeg;
+      sm_long = sm_long || len > kSmSeg;
       size_t pos = flat.size();
       for (int t = 0; t < nt; ++t) {
         at[t] = pos;
         const int c8 = (cnt[t] + 7) & ~7;
-        const int nseg = std::max(1, cdiv(c8, kSmSeg));
+        const int nseg = std::max(1, cdiv(c8, len));
         for (int sg = 0; sg < nseg; ++sg)
-          items.push_back(SmItem{t, (int)(pos + (size_t)sg * kSmSeg), std::min(kSmSeg, c8 - sg * kSmSeg), sg, nseg, nscr,
+          items.push_back(SmItem{t, (int)(pos + (size_t)sg * len), std::min(len, c8 - sg * len), sg, nseg, nscr,
                                  g * nt + t, shared ? -1 : g});
         if (nseg > 1) nscr += nseg;
         pos += c8;
@@ -716,8 +727,10 @@ template <typename T> struct NufftOp : Op {
     d_smscratch.alloc(sizeof(double) * (size_t)std::max(nscr, 1) * chunks * pb * 256);
     d_smtickets.alloc(sizeof(unsigned int) * (size_t)ngeo * nt * chunks);
     MF_CK(cudaMemset(d_smtickets.p, 0, d_smtickets.bytes));
-    set_smem(k_nufft_spread_mma<T, 1>, sm_smem<T, 1>());
-    set_smem(k_nufft_spread_mma<T, kMmaProb>, sm_smem<T, kMmaProb>());
+    set_smem(k_nufft_spread_mma<T, 1, false>, sm_smem<T, 1>());
+    set_smem(k_nufft_spread_mma<T, 1, true>, sm_smem<T, 1>());
+    set_smem(k_nufft_spread_mma<T, kMmaProb, false>, sm_smem<T, kMmaProb>());
+    set_smem(k_nufft_spread_mma<T, kMmaProb, true>, sm_smem<T, kMmaProb>());
   }
   // problems per CTA of the two: one where each problem has its own points
   // or the batch is a single problem, else chunks of 8
@@ -963,14 +976,12 @@ template <typename T> struct NufftOp : Op {
     const NufftGeom<T> geo = geo_now();
     if (spread_mma) {
       const dim3 grid(nsm, mma_chunks());
-      if (mma_prob() == 1)
-        k_nufft_spread_mma<T, 1><<<grid, 256, sm_smem<T, 1>(), s>>>(
-            geo, wxd(), wyd(), d_smitems.as<SmItem>(), d_smlist.as<unsigned int>(), d_y2.as<cplx<T>>(), g, gstride, nx, ny,
-            sm_cols, c.st, gate, B, d_smscratch.as<double>(), d_smtickets.as<unsigned int>());
-      else
-        k_nufft_spread_mma<T, kMmaProb><<<grid, 256, sm_smem<T, kMmaProb>(), s>>>(
-            geo, wxd(), wyd(), d_smitems.as<SmItem>(), d_smlist.as<unsigned int>(), d_y2.as<cplx<T>>(), g, gstride, nx, ny,
-            sm_cols, c.st, gate, B, d_smscratch.as<double>(), d_smtickets.as<unsigned int>());
+      const bool one = mma_prob() == 1;
+      const auto kern = one ? (sm_long ? k_nufft_spread_mma<T, 1, true> : k_nufft_spread_mma<T, 1, false>)
+                            : (sm_long ? k_nufft_spread_mma<T, kMmaProb, true> : k_nufft_spread_mma<T, kMmaProb, false>);
+      kern<<<grid, 256, one ? sm_smem<T, 1>() : sm_smem<T, kMmaProb>(), s>>>(
+          geo, wxd(), wyd(), d_smitems.as<SmItem>(), d_smlist.as<unsigned int>(), d_y2.as<cplx<T>>(), g, gstride, nx, ny,
+          sm_cols, c.st, gate, B, d_smscratch.as<double>(), d_smtickets.as<unsigned int>());
       MF_LAUNCH_CK();
       return;
     }
