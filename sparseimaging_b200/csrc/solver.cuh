@@ -208,6 +208,8 @@ struct Op {
   virtual int max_chi_slots() const { return chi_slots(); }
   virtual int tsv_slots() const = 0;
   virtual LaunchShapes shapes() const { return LaunchShapes(); }
+  // shapes() with 0 also for what its present kernels do not depend on
+  virtual LaunchShapes tunable() const { return shapes(); }
   // throws Error(MFISTA_ERR_ARG) for a shape the operator cannot run
   virtual void set_shapes(const LaunchShapes& sh) { (void)sh; }
   virtual double fscale() const = 0;
@@ -1054,6 +1056,14 @@ template <typename T> struct NufftOp : Op {
     sh.spread_cluster = shared ? spread_cs : 0;
     sh.rows_per_cta = rpc;
     sh.cols_per_cta = cpc;
+    return sh;
+  }
+
+  // the matrix-product kernels divide points and tiles by their own rules
+  LaunchShapes tunable() const override {
+    LaunchShapes sh = shapes();
+    if (interp_tc || interp_mma) sh.interp_ppw = 0;
+    if (spread_tc || spread_mma) sh.spread_cluster = 0;
     return sh;
   }
 
@@ -2087,9 +2097,12 @@ struct Solver {
   // t_all / min t_all + 2 t_one / min t_one: a lambda grid's iteration
   // counts spread over decades, so many loop steps run with a handful of
   // problems left (the 128x128 64-problem grid: 2234 of 4553 steps with 8
-  // or fewer).  ms_out[k]: t_all (ms per launch) of knob k's choice.
+  // or fewer).  ms_out[k]: t_all (ms per launch) of knob k's choice.  A knob
+  // that the kernels do not depend on keeps its value: its candidates would
+  // differ by noise alone.
   LaunchShapes tune(int reps, double ms_out[4]) {
     LaunchShapes cur = op->shapes();
+    const LaunchShapes live = op->tunable();
     // knob -> kernels timed (profile_kernel ids) and candidates
     struct Knob { int LaunchShapes::*field; std::vector<int> kernels; std::vector<int> cand; };
     std::vector<Knob> knobs = {
@@ -2102,6 +2115,7 @@ struct Solver {
       ms_out[k] = 0;
       Knob& kb = knobs[k];
       if (cur.*(kb.field) == 0) continue;  // not used by this operator
+      if (live.*(kb.field) == 0) kb.cand = {cur.*(kb.field)};
       std::vector<int> vals;
       std::vector<double> t_all, t_one;
       for (int v : kb.cand) {
