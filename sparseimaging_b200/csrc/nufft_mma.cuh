@@ -73,10 +73,23 @@ __device__ __forceinline__ void cp_async_cell(cplx<T>* dst, const cplx<T>* src, 
 // the sum, when all columns of the unit are) and the sum is negated once.
 // A problem's sums depend neither on its CTA's points nor on the other
 // problems: groups and chi^2 slots (32 points) are the same for every cut.
+//
+// Problems with points of their own can make thousands of tiles of a few
+// points, which stage a window each and leave most of eight warps idle.  Where
+// there are many (NufftOp::build_im_tiles) a CTA has kImFew threads and at most
+// kImFewPts points, twice as many are resident, and only the cells that the
+// points reach are read (the others are zeros, as their weights are): the same
+// bits.  Microseconds per launch with eight warps -> four (tap by tap before):
+// 10 frames of 3000 random points at 256 x 256 125 -> 88 (49), along tracks
+// 49 -> 37 (48); 16 of 1000 at 128 x 128 53 -> 39 (30) and 28 -> 23 (30); 16 of
+// 12000 98 -> 82 (283) and 80 -> 74 (280).  Two warps and 32 points: 83, 37,
+// 37, 23, 102 and 90.
 // ---------------------------------------------------------------------------
 constexpr int kImTile = 16;
 constexpr int kImWin = kImTile + kTaps;  // 40: 39 used, a multiple of 4
 constexpr int kImPts = 128;              // points per CTA at most: 8 warps x 16
+constexpr int kImFew = 128;              // threads per CTA where there are many tiles
+constexpr int kImFewPts = kImFew / 2;    // and their points at most
 constexpr int kImSteps = kImWin / 4;     // column steps of 4
 
 struct ImTileItem {
@@ -85,6 +98,7 @@ struct ImTileItem {
   int prob;          // its problem (points of its own), or -1 (shared points)
   int slot, nslot;   // first chi^2 slot (one per 32 points), slots of the problem
   int item, nitem;   // CTA of the problem, CTAs of the problem
+  int box;           // cells of the window that its points reach: rows [r0, r1), columns [c0, c1), 8 bits each
 };
 
 // row stride of the staged window: the four rows of a B fragment hit all banks
@@ -159,8 +173,8 @@ __device__ __forceinline__ void interp_unit(const ImUnit& u, int nk, const T* w,
   }
 }
 
-template <typename T, int PB>
-__global__ void __launch_bounds__(256, 2)
+template <typename T, int PB, int NT>
+__global__ void __launch_bounds__(NT, 512 / NT)
     k_nufft_interp_mma(NufftGeom<T> geo, const double* __restrict__ wxd, const double* __restrict__ wyd,
                        const ImTileItem* __restrict__ tiles, const int2* __restrict__ perm,
                        const cplx<T>* __restrict__ gall, long gstride, int nx, int ny, double inv_mm,
@@ -168,7 +182,7 @@ __global__ void __launch_bounds__(256, 2)
                        cplx<T>* __restrict__ y2, int B, const double2* __restrict__ ax_base,
                        double2* __restrict__ ax_out) {
   constexpr int LD = ImWindow<T>::kLd;
-  constexpr int kCells = (kImWin * kImWin + 255) / 256;
+  constexpr int kCells = (kImWin * kImWin + NT - 1) / NT, NW = NT / 32;
   extern __shared__ __align__(16) unsigned char im_smem_raw[];
   cplx<T>* win = reinterpret_cast<cplx<T>*>(im_smem_raw);
   double* s_red = reinterpret_cast<double*>(im_smem_raw + (PB > 1 ? kImBuf : 1) * ImWindow<T>::kBytes);
@@ -191,10 +205,12 @@ __global__ void __launch_bounds__(256, 2)
   int cell[kCells];
 #pragma unroll
   for (int i = 0; i < kCells; ++i) {
-    const int v = threadIdx.x + 256 * i;
+    const int v = threadIdx.x + NT * i;
     cell[i] = -1;
-    if (v < kImWin * kImWin) {
-      const int vr = tl.row0 + v / kImWin, vc = tl.col0 + v % kImWin;
+    const int r = v / kImWin, c = v % kImWin;
+    if (v < kImWin * kImWin &&
+        (NT == 256 || (r >= (tl.box & 255) && r < ((tl.box >> 8) & 255) && c >= ((tl.box >> 16) & 255) && c < tl.box >> 24))) {
+      const int vr = tl.row0 + r, vc = tl.col0 + c;
       int col = half_col(vc, ny), row = -1;
       if (col >= 0) {
         row = wrap_row(vr, nx);
@@ -210,7 +226,7 @@ __global__ void __launch_bounds__(256, 2)
     cplx<T>* w = win + (size_t)buf * kImWin * LD;
 #pragma unroll
     for (int i = 0; i < kCells; ++i) {
-      const int v = threadIdx.x + 256 * i;
+      const int v = threadIdx.x + NT * i;
       if (v < kImWin * kImWin)
         cp_async_cell<T>(w + (v / kImWin) * LD + v % kImWin, gr + max(cell[i], 0), cell[i] >= 0);
     }
@@ -224,7 +240,7 @@ __global__ void __launch_bounds__(256, 2)
     for (int sl = tl.nslot + tl.item; sl < nslots; sl += tl.nitem) part.at(qchi, s_list[threadIdx.x])[sl] = 0.0;
 
   // warps over (unit of 16 points, row groups): nu units, ng warps a unit
-  const int nu = max(1, (tl.count + 15) >> 4), ng = nu > 4 ? 1 : nu > 2 ? 2 : 4;
+  const int nu = max(1, (tl.count + 15) >> 4), ng = 2 * nu > NW ? 1 : 4 * nu > NW ? 2 : 4;
   const int unit = warp % nu, grp = warp / nu;
   const bool on = grp < ng;
   const int p0 = tl.start + unit * 16;
@@ -305,7 +321,7 @@ __global__ void __launch_bounds__(256, 2)
   __syncthreads();
   // residual, chi^2 and models: a warp per (problem, 32 points)
   const int nq = (nu + 1) >> 1;
-  for (int e0 = warp; e0 < nact * nq; e0 += 8) {
+  for (int e0 = warp; e0 < nact * nq; e0 += NW) {
     const int i = e0 / nq, j0 = 32 * (e0 - i * nq);
     const int b = s_list[i];
     const int j = j0 + lane;

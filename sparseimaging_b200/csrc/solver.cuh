@@ -327,6 +327,7 @@ template <typename T> struct NufftOp : Op {
   DevMem d_im, d_imperm, d_smitems, d_smlist, d_smscratch, d_smtickets;
   DevMem d_wxd, d_wyd;  // FP64 weights of an FP32 operator (wxd(), wyd())
   int nim = 0, im_chunks = 1, nsm = 0, sm_cols = 0;
+  bool im_few = false;   // interpolation CTAs of four warps
   bool sm_long = false;  // some problem's lists are cut at more than kSmSeg entries
   // chi^2 partial slots every interpolation kernel of this operator writes
   // (at least its own CTA count; the extra CTAs write zeros), so that the
@@ -534,6 +535,7 @@ template <typename T> struct NufftOp : Op {
     std::vector<int2> perm;
     std::vector<Key> keys;
     const int ngeo = shared ? 1 : B;
+    std::vector<int> nslots(ngeo, 0);
     int most = 1, im_pts = kImPts;
     auto first = [](int m) { return (long long)std::max(-(1 << 28), std::min(1 << 28, m)) - (kMSP - 1); };
     auto fdiv = [](long long a) { return a >= 0 ? a / kImTile : -((-a + kImTile - 1) / kImTile); };
@@ -596,7 +598,7 @@ template <typename T> struct NufftOp : Op {
         for (size_t a = i; a < j; a += im_pts) {
           const int cnt = (int)std::min<size_t>(im_pts, j - a);
           tiles.push_back(ImTileItem{(int)(tx * kImTile), (int)(ty * kImTile), (int)(perm.size() + (a - i)), cnt,
-                                     shared ? -1 : g, slots, 0, 0, 0});
+                                     shared ? -1 : g, slots, 0, 0, 0, 0});
           slots += cdiv(cnt, 32);
         }
         for (size_t a = i; a < j; ++a) {
@@ -606,17 +608,39 @@ template <typename T> struct NufftOp : Op {
         i = j;
       }
       if (tiles.size() == t0) {
-        tiles.push_back(ImTileItem{0, 0, 0, 0, shared ? -1 : g, 0, 0, 0, 0});
+        tiles.push_back(ImTileItem{0, 0, 0, 0, shared ? -1 : g, 0, 0, 0, 0, 0});
         slots = 1;
       }
-      const int nt = (int)(tiles.size() - t0);
-      for (int q = 0; q < nt; ++q) {
-        tiles[t0 + q].nslot = slots;
-        tiles[t0 + q].item = q;
-        tiles[t0 + q].nitem = nt;
-      }
+      nslots[g] = slots;
       most = std::max(most, slots);
     }
+    // many tiles of points of their own: smaller CTAs (with few, one CTA's
+    // chain is what counts: 3 frames of 800 points on tracks 8.4 us, 10.4)
+    im_few = !shared && tiles.size() > kImFewTiles;
+    if (im_few)
+      for (size_t q = 0; q < tiles.size(); ++q)
+        if (tiles[q].count > kImFewPts) {
+          ImTileItem rest = tiles[q];
+          rest.start += kImFewPts;
+          rest.count -= kImFewPts;
+          rest.slot += kImFewPts / 32;
+          tiles[q].count = kImFewPts;
+          tiles.push_back(rest);
+        }
+    std::vector<int> nitems(ngeo, 0);
+    for (ImTileItem& t : tiles) {
+      const int g = std::max(t.prob, 0);
+      t.nslot = nslots[g];
+      t.item = nitems[g]++;
+      int r0 = kImWin, r1 = 0, c0 = kImWin, c1 = 0;
+      for (int a = t.start; a < t.start + t.count; ++a) {
+        const int r = perm[a].y & 0xff, c = perm[a].y >> 8;
+        r0 = std::min(r0, r), r1 = std::max(r1, r + kTaps);
+        c0 = std::min(c0, c), c1 = std::max(c1, c + kTaps);
+      }
+      t.box = r0 | r1 << 8 | c0 << 16 | c1 << 24;
+    }
+    for (ImTileItem& t : tiles) t.nitem = nitems[std::max(t.prob, 0)];
     // launch order: fullest CTAs first, so that the last wave holds short ones
     std::stable_sort(tiles.begin(), tiles.end(),
                      [](const ImTileItem& a, const ImTileItem& b) { return a.count > b.count; });
@@ -634,8 +658,9 @@ template <typename T> struct NufftOp : Op {
     if (perm.empty()) perm.push_back(make_int2(0, 0));
     d_im.upload(tiles.data(), tiles.size());
     d_imperm.upload(perm.data(), perm.size());
-    set_smem(k_nufft_interp_mma<T, 1>, im_smem<T, 1>());
-    set_smem(k_nufft_interp_mma<T, kImProb>, im_smem<T, kImProb>());
+    set_smem(k_nufft_interp_mma<T, 1, 256>, im_smem<T, 1>());
+    set_smem(k_nufft_interp_mma<T, 1, kImFew>, im_smem<T, 1>());
+    set_smem(k_nufft_interp_mma<T, kImProb, 256>, im_smem<T, kImProb>());
   }
 
   // k_nufft_spread_mma's tiles and lists: per stored tile the virtual points
@@ -737,6 +762,7 @@ template <typename T> struct NufftOp : Op {
   // problems per CTA of the two: one where each problem has its own points
   // or the batch is a single problem, else chunks of 8
   static constexpr int kMmaProb = 8, kImProb = 6;
+  static constexpr size_t kImFewTiles = 600;  // two rounds of 148 SMs with two CTAs each
   int mma_prob() const { return shared && B > 1 ? kMmaProb : 1; }
   int mma_chunks() const { return shared ? cdiv(B, mma_prob()) : 1; }
 
@@ -875,15 +901,12 @@ template <typename T> struct NufftOp : Op {
                      double2* out = nullptr) {
     const NufftGeom<T> geo = geo_now();
     if (interp_mma) {
-      const dim3 grid(nim, im_chunks);
-      if (mma_prob() == 1)
-        k_nufft_interp_mma<T, 1><<<grid, 256, im_smem<T, 1>(), s>>>(
-            geo, wxd(), wyd(), d_im.as<ImTileItem>(), d_imperm.as<int2>(), g, gstride, nx, ny, inv_mm, c.st, gate, c.part,
-            qchi, chi_slots(), y2, B, base, out);
-      else
-        k_nufft_interp_mma<T, kImProb><<<grid, 256, im_smem<T, kImProb>(), s>>>(
-            geo, wxd(), wyd(), d_im.as<ImTileItem>(), d_imperm.as<int2>(), g, gstride, nx, ny, inv_mm, c.st, gate, c.part,
-            qchi, chi_slots(), y2, B, base, out);
+      const bool one = mma_prob() == 1;
+      const auto kern = !one ? k_nufft_interp_mma<T, kImProb, 256>
+                             : im_few ? k_nufft_interp_mma<T, 1, kImFew> : k_nufft_interp_mma<T, 1, 256>;
+      kern<<<dim3(nim, im_chunks), im_few ? kImFew : 256, one ? im_smem<T, 1>() : im_smem<T, kImProb>(), s>>>(
+          geo, wxd(), wyd(), d_im.as<ImTileItem>(), d_imperm.as<int2>(), g, gstride, nx, ny, inv_mm, c.st, gate, c.part,
+          qchi, chi_slots(), y2, B, base, out);
       MF_LAUNCH_CK();
       return;
     }
