@@ -374,11 +374,22 @@ __global__ void __launch_bounds__(NT, 512 / NT)
 // within 8 MB a problem, where it would be 75 bytes a point and problem.
 // The weights are read where they lie (48 values a point, shared by the tiles
 // around it): cached, with the taps outside [0, 24) as zeros.
+// Thinly spread points leave most tiles with a few entries, a CTA's chain of
+// loads and barriers each.  Where one problem, or problems with points of their
+// own, make many tiles (NufftOp::build_sm_items), those of at most kSmLight
+// entries go eight to a CTA, one to a warp, entries in the lanes: the same sums
+// without barriers.  Microseconds per launch with a CTA to every tile -> here
+// (tap by tap before): 10 frames of 3000 random points at 256 x 256 86 -> 33
+// (92), of 300 66 -> 12 (23), 16 of 12000 at 128 x 128 273 -> 195 (585); one
+// problem of 3000 points at 512 x 512 31 -> 8 (220).  With at most 16 entries
+// a light tile: 58, 12, 195 and 8.
 // ---------------------------------------------------------------------------
 constexpr int kSmRows = 8, kSmCols = 16;
 constexpr int kSmSeg = 256;  // list entries staged at once
 constexpr int kSmSegMax = 4096;  // partial tiles of a problem at most
+constexpr int kSmLight = 32;     // entries of a tile that one warp takes at most
 
+// nseg = 0: `count` light tiles, items[start] and following
 struct SmItem {
   int tile;          // tile of the stored half grid, row-major
   int start, count;  // list entries; count a multiple of 8
@@ -394,12 +405,39 @@ struct SmPoint {
   int fl;      // mirrored
 };
 
+// a list entry's geometry; an empty one has no tap anywhere
+template <typename T>
+__device__ __forceinline__ SmPoint sm_point(const NufftGeom<T>& geo, unsigned int code) {
+  SmPoint p{0, 1 << 29, 1 << 29, 0};
+  if (code != 0xffffffffu) {
+    const int k = (int)(code >> 1), fl = (int)(code & 1u);
+    p.k24 = (unsigned int)k * kTaps;
+    p.x0 = fl ? -geo.mx[k] - kMSP : geo.mx[k] - (kMSP - 1);
+    p.y0 = fl ? -geo.my[k] - kMSP : geo.my[k] - (kMSP - 1);
+    p.fl = fl;
+  }
+  return p;
+}
+
+// and its half residual, the imaginary part negated for a direct point
+template <typename T>
+__device__ __forceinline__ double2 sm_residual(const cplx<T>* __restrict__ y2, unsigned int code) {
+  if (code == 0xffffffffu) return make_double2(0.0, 0.0);
+  const cplx<T> r = y2[code >> 1];
+  return make_double2(0.5 * (double)r.x, (code & 1u) ? 0.5 * (double)r.y : -0.5 * (double)r.y);
+}
+
 // (the exchange of the parities' sums reuses the residuals' space)
 constexpr size_t sm_exchange(int pb) { return sizeof(double) * 64 * (pb > 1 ? 8 * 4 : 8); }
 template <typename T, int PB> constexpr size_t sm_smem() {
   const size_t y = sizeof(double2) * (size_t)PB * kSmSeg;
   return (size_t)kSmSeg * sizeof(SmPoint) + (y > sm_exchange(PB) ? y : sm_exchange(PB));
 }
+
+constexpr int kSmOut = 1 << 28;  // no tap reaches it
+// virtual row and column of a stored one
+__device__ __forceinline__ int sm_row(int row, int nx) { return row < nx ? row : row < 2 * nx ? row - 2 * nx : kSmOut; }
+__device__ __forceinline__ int sm_col(int col, int ny) { return col < ny ? col : col == ny ? -ny : kSmOut; }
 
 // the products of NP problems' MB x NB blocks (from mb0, nb0) over the steps
 // of parity ch0; problem p's residuals at s_yp + p kSmSeg
@@ -409,18 +447,11 @@ __device__ __forceinline__ void spread_products(const SmPoint* s_pt, const doubl
                                                 const double* __restrict__ wxd, const double* __restrict__ wyd,
                                                 double (&d)[2][4][2]) {
   const int g = lane >> 2, t = lane & 3;
-  constexpr int kOut = 1 << 28;  // no tap reaches it
   int mr[MB], mc[NB];
 #pragma unroll
-  for (int m = 0; m < MB; ++m) {
-    const int row = row_base + 4 * (mb0 + m) + (g >> 1);
-    mr[m] = row < nx ? row : row < 2 * nx ? row - 2 * nx : kOut;
-  }
+  for (int m = 0; m < MB; ++m) mr[m] = sm_row(row_base + 4 * (mb0 + m) + (g >> 1), nx);
 #pragma unroll
-  for (int n = 0; n < NB; ++n) {
-    const int col = col_base + 8 * (nb0 + n) + g;
-    mc[n] = col < ny ? col : col == ny ? -ny : kOut;
-  }
+  for (int n = 0; n < NB; ++n) mc[n] = sm_col(col_base + 8 * (nb0 + n) + g, ny);
   const SmPoint* pt = s_pt + 4 * ch0 + t;
   const double* yp = reinterpret_cast<const double*>(s_yp + 4 * ch0 + t) + (g & 1);
 #pragma unroll 4
@@ -450,10 +481,71 @@ __device__ __forceinline__ void spread_products(const SmPoint* s_pt, const doubl
   }
 }
 
+// block blk of a tile into the grid.  Lane (g, t): row g >> 1, re or im (g & 1),
+// columns 2t, 2t + 1; lanes g and g ^ 1 exchange so that each writes one
+// complex cell
+template <typename T>
+__device__ __forceinline__ void sm_store(cplx<T>* __restrict__ gr, int blk, double d0, double d1, int row_base,
+                                         int col_base, int nx, int ny, int lane) {
+  const int g = lane >> 2, t = lane & 3;
+  const double other = __shfl_xor_sync(0xffffffffu, (g & 1) ? d0 : d1, 4);
+  const double re = (g & 1) ? other : d0, im = (g & 1) ? d1 : other;
+  const int row = row_base + 4 * (blk >> 1) + (g >> 1), col = col_base + 8 * (blk & 1) + 2 * t + (g & 1);
+  if (row < 2 * nx && col <= ny) gr[(size_t)row * (ny + 1) + col] = mk<T>((T)re, (T)im);
+}
+
+// a light tile, by a warp
+template <typename T>
+__device__ __forceinline__ void spread_light(const NufftGeom<T>& geo, const double* __restrict__ wxd,
+                                             const double* __restrict__ wyd, const unsigned int* __restrict__ list,
+                                             int count, const cplx<T>* __restrict__ y2, cplx<T>* __restrict__ gr,
+                                             int row_base, int col_base, int nx, int ny, int lane) {
+  const unsigned int all = 0xffffffffu;
+  const int g = lane >> 2, t = lane & 3;
+  const unsigned int code = lane < count ? list[lane] : all;
+  const SmPoint p = sm_point<T>(geo, code);
+  const double2 y = sm_residual<T>(y2, code);
+  int mr[2], mc[2];
+#pragma unroll
+  for (int m = 0; m < 2; ++m) {
+    mr[m] = sm_row(row_base + 4 * m + (g >> 1), nx);
+    mc[m] = sm_col(col_base + 8 * m + g, ny);
+  }
+  double acc[2][4][2];  // even and odd steps
+#pragma unroll
+  for (int q = 0; q < 2; ++q)
+#pragma unroll
+    for (int m = 0; m < 4; ++m) acc[q][m][0] = acc[q][m][1] = 0.0;
+  for (int e = 0; e < count; e += 8)
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int src = e + 4 * q + t;
+      const unsigned int k24 = __shfl_sync(all, p.k24, src);
+      const int x0 = __shfl_sync(all, p.x0, src), y0 = __shfl_sync(all, p.y0, src), fl = __shfl_sync(all, p.fl, src);
+      const double re = __shfl_sync(all, y.x, src), im = __shfl_sync(all, y.y, src);
+      double a[2], b[2];
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        const int j = mr[m] - x0, i = mc[m] - y0;
+        a[m] = (unsigned)j < (unsigned)kTaps ? __ldg(wxd + k24 + (fl ? kTaps - 1 - j : j)) : 0.0;
+        b[m] = (unsigned)i < (unsigned)kTaps ? __ldg(wyd + k24 + (fl ? kTaps - 1 - i : i)) : 0.0;
+      }
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        const double ay = a[m] * ((g & 1) ? im : re);
+#pragma unroll
+        for (int n = 0; n < 2; ++n) dmma_884(acc[q][2 * m + n], ay, b[n]);
+      }
+    }
+#pragma unroll
+  for (int m = 0; m < 4; ++m)
+    sm_store<T>(gr, m, acc[0][m][0] + acc[1][m][0], acc[0][m][1] + acc[1][m][1], row_base, col_base, nx, ny, lane);
+}
+
 // kLong: there are segments of more than kSmSeg entries (an instance of its
 // own: with the loop the others take 2-5 % longer)
 template <typename T, int PB, bool kLong>
-__global__ void __launch_bounds__(256, PB > 1 ? 3 : 2)
+__global__ void __launch_bounds__(256, 3)
     k_nufft_spread_mma(NufftGeom<T> geo, const double* __restrict__ wxd, const double* __restrict__ wyd,
                        const SmItem* __restrict__ items, const unsigned int* __restrict__ vlist,
                        const cplx<T>* __restrict__ y2, cplx<T>* __restrict__ gall, long gstride, int nx, int ny,
@@ -467,17 +559,26 @@ __global__ void __launch_bounds__(256, PB > 1 ? 3 : 2)
   __shared__ int s_cnt[8];
   __shared__ unsigned int s_ticket;
   const SmItem it = items[blockIdx.x];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int nact;
   if (PB > 1) {
     nact = active_share<PB>(st, gate, B, s_list, s_cnt, geo.act_lists);
   } else {
+    if (it.nseg == 0) {
+      if (warp >= it.count) return;
+      const SmItem l = items[it.start + warp];
+      const int b = l.prob >= 0 ? l.prob : (int)blockIdx.y, tr = l.tile / ntcol;
+      if (!gate_ok(st[b], gate)) return;
+      spread_light<T>(geo, wxd, wyd, vlist + l.start, l.count, y2 + (size_t)b * geo.y2_bstride,
+                      gall + (size_t)b * gstride, tr * kSmRows, (l.tile - tr * ntcol) * kSmCols, nx, ny, lane);
+      return;
+    }
     const int b = it.prob >= 0 ? it.prob : (int)blockIdx.y;
     nact = gate_ok(st[b], gate) ? 1 : 0;
     if (threadIdx.x == 0) s_list[0] = b;
     __syncthreads();
   }
   if (nact == 0) return;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int tr = it.tile / ntcol, tcl = it.tile - tr * ntcol;
   const int row_base = tr * kSmRows, col_base = tcl * kSmCols;
   // warps over (pair of problems, blocks of the tile, parity of the steps):
@@ -498,24 +599,8 @@ __global__ void __launch_bounds__(256, PB > 1 ? 3 : 2)
     for (int e = threadIdx.x; e < cnt * nact; e += blockDim.x) {
       const int i = e / cnt, q = e - i * cnt;
       const unsigned int code = vlist[it.start + base + q];
-      double2 y = make_double2(0.0, 0.0);
-      if (code != 0xffffffffu) {
-        const int k = (int)(code >> 1);
-        const cplx<T> r = y2[(size_t)s_list[i] * geo.y2_bstride + k];
-        y = make_double2(0.5 * (double)r.x, (code & 1u) ? 0.5 * (double)r.y : -0.5 * (double)r.y);
-      }
-      s_y[(size_t)i * kSmSeg + q] = y;
-      if (i == 0) {
-        SmPoint p{0, 1 << 29, 1 << 29, 0};  // an empty entry: no tap anywhere
-        if (code != 0xffffffffu) {
-          const int k = (int)(code >> 1), fl = (int)(code & 1u);
-          p.k24 = (unsigned int)k * kTaps;
-          p.x0 = fl ? -geo.mx[k] - kMSP : geo.mx[k] - (kMSP - 1);
-          p.y0 = fl ? -geo.my[k] - kMSP : geo.my[k] - (kMSP - 1);
-          p.fl = fl;
-        }
-        s_pt[q] = p;
-      }
+      s_y[(size_t)i * kSmSeg + q] = sm_residual<T>(y2 + (size_t)s_list[i] * geo.y2_bstride, code);
+      if (i == 0) s_pt[q] = sm_point<T>(geo, code);
     }
     __syncthreads();
     if (PB > 1 && groups == 1) {
@@ -585,19 +670,10 @@ __global__ void __launch_bounds__(256, PB > 1 ? 3 : 2)
     if (threadIdx.x == 0) tickets[(size_t)it.ticket * gridDim.y + blockIdx.y] = 0u;  // for the next launch
   }
   if (nblk == 0) return;
-  // lane (g, t): row g >> 1, re or im (g & 1), columns 2t, 2t + 1; lanes g and
-  // g ^ 1 exchange so that each writes one complex cell
-  const int g = lane >> 2, t = lane & 3;
   cplx<T>* gr = gall + (size_t)s_list[prob] * gstride;
 #pragma unroll
   for (int q = 0; q < kBlkW; ++q)
-    if (q < nblk) {
-      const double other = __shfl_xor_sync(0xffffffffu, (g & 1) ? d[q][0] : d[q][1], 4);
-      const double re = (g & 1) ? other : d[q][0], im = (g & 1) ? d[q][1] : other;
-      const int blk = blk0 + q;
-      const int row = row_base + 4 * (blk >> 1) + (g >> 1), col = col_base + 8 * (blk & 1) + 2 * t + (g & 1);
-      if (row < 2 * nx && col <= ny) gr[(size_t)row * (ny + 1) + col] = mk<T>((T)re, (T)im);
-    }
+    if (q < nblk) sm_store<T>(gr, blk0 + q, d[q][0], d[q][1], row_base, col_base, nx, ny, lane);
 }
 
 }  // namespace mf

@@ -747,6 +747,17 @@ template <typename T> struct NufftOp : Op {
     // launch order: longest segments first
     std::stable_sort(items.begin(), items.end(), [](const SmItem& a, const SmItem& b) { return a.count > b.count; });
     nsm = (int)items.size();
+    // many tiles: the light ones eight to a CTA (few: a CTA each is quicker)
+    if (mma_prob() == 1 && items.size() > kSmLightTiles) {
+      const auto light = std::stable_partition(
+          items.begin(), items.end(), [](const SmItem& t) { return t.nseg > 1 || t.count > kSmLight; });
+      const std::vector<SmItem> tail(light, items.end());
+      items.erase(light, items.end());
+      nsm = (int)items.size() + cdiv((long)tail.size(), 8);
+      for (size_t q = 0; q < tail.size(); q += 8)
+        items.push_back(SmItem{0, nsm + (int)q, (int)std::min<size_t>(8, tail.size() - q), 0, 0, 0, 0, 0});
+      items.insert(items.end(), tail.begin(), tail.end());
+    }
     if (flat.empty()) flat.push_back(0xffffffffu);
     d_smitems.upload(items.data(), items.size());
     d_smlist.upload(flat.data(), flat.size());
@@ -762,6 +773,7 @@ template <typename T> struct NufftOp : Op {
   // problems per CTA of the two: one where each problem has its own points
   // or the batch is a single problem, else chunks of 8
   static constexpr int kMmaProb = 8, kImProb = 6;
+  static constexpr size_t kSmLightTiles = 600;  // more than 148 SMs hold at once
   static constexpr size_t kImFewTiles = 600;  // two rounds of 148 SMs with two CTAs each
   int mma_prob() const { return shared && B > 1 ? kMmaProb : 1; }
   int mma_chunks() const { return shared ? cdiv(B, mma_prob()) : 1; }
