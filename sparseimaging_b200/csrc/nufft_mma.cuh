@@ -76,20 +76,18 @@ __device__ __forceinline__ void cp_async_cell(cplx<T>* dst, const cplx<T>* src, 
 //
 // Problems with points of their own can make thousands of tiles of a few
 // points, which stage a window each and leave most of eight warps idle.  Where
-// there are many (NufftOp::build_im_tiles) a CTA has kImFew threads and at most
-// kImFewPts points, twice as many are resident, and only the cells that the
-// points reach are read (the others are zeros, as their weights are): the same
-// bits.  Microseconds per launch with eight warps -> four (tap by tap before):
-// 10 frames of 3000 random points at 256 x 256 125 -> 88 (49), along tracks
-// 49 -> 37 (48); 16 of 1000 at 128 x 128 53 -> 39 (30) and 28 -> 23 (30); 16 of
-// 12000 98 -> 82 (283) and 80 -> 74 (280).  Two warps and 32 points: 83, 37,
-// 37, 23, 102 and 90.
+// there are many (NufftOp::build_im_tiles) a CTA has four warps, or two, and at
+// most half as many points as threads, two to four times as many are resident,
+// and only the cells that the points reach are read (the others are zeros, as
+// their weights are): the same bits.  Microseconds per launch with eight, four
+// and two warps (tap by tap before): 10 frames of 3000 random points at 256 x
+// 256 125, 88, 83 (49; FP32 125, 88, 76 (45)), along tracks 49, 37, 37 (48); 16
+// of 1000 at 128 x 128 53, 39, 37 (30) and 28, 23, 23 (30); 16 of 12000 98, 82,
+// 102 (283) and 80, 74, 90 (280).
 // ---------------------------------------------------------------------------
 constexpr int kImTile = 16;
 constexpr int kImWin = kImTile + kTaps;  // 40: 39 used, a multiple of 4
 constexpr int kImPts = 128;              // points per CTA at most: 8 warps x 16
-constexpr int kImFew = 128;              // threads per CTA where there are many tiles
-constexpr int kImFewPts = kImFew / 2;    // and their points at most
 constexpr int kImSteps = kImWin / 4;     // column steps of 4
 
 struct ImTileItem {

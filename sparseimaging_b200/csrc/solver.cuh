@@ -327,7 +327,7 @@ template <typename T> struct NufftOp : Op {
   DevMem d_im, d_imperm, d_smitems, d_smlist, d_smscratch, d_smtickets;
   DevMem d_wxd, d_wyd;  // FP64 weights of an FP32 operator (wxd(), wyd())
   int nim = 0, im_chunks = 1, nsm = 0, sm_cols = 0;
-  bool im_few = false;   // interpolation CTAs of four warps
+  int im_threads = 256;  // of an interpolation CTA
   bool sm_long = false;  // some problem's lists are cut at more than kSmSeg entries
   // chi^2 partial slots every interpolation kernel of this operator writes
   // (at least its own CTA count; the extra CTAs write zeros), so that the
@@ -615,16 +615,18 @@ template <typename T> struct NufftOp : Op {
       most = std::max(most, slots);
     }
     // many tiles of points of their own: smaller CTAs (with few, one CTA's
-    // chain is what counts: 3 frames of 800 points on tracks 8.4 us, 10.4)
-    im_few = !shared && tiles.size() > kImFewTiles;
-    if (im_few)
+    // chain is what counts: 3 frames of 800 points on tracks 8.4 us, 10.4 with
+    // four warps); two warps where a tile has less than half a unit's points
+    im_threads = shared || tiles.size() <= kImManyTiles ? 256 : perm.size() < 8 * tiles.size() ? 64 : 128;
+    const int cut = im_threads / 2;
+    if (im_threads < 256)
       for (size_t q = 0; q < tiles.size(); ++q)
-        if (tiles[q].count > kImFewPts) {
+        if (tiles[q].count > cut) {
           ImTileItem rest = tiles[q];
-          rest.start += kImFewPts;
-          rest.count -= kImFewPts;
-          rest.slot += kImFewPts / 32;
-          tiles[q].count = kImFewPts;
+          rest.start += cut;
+          rest.count -= cut;
+          rest.slot += cut / 32;
+          tiles[q].count = cut;
           tiles.push_back(rest);
         }
     std::vector<int> nitems(ngeo, 0);
@@ -659,7 +661,8 @@ template <typename T> struct NufftOp : Op {
     d_im.upload(tiles.data(), tiles.size());
     d_imperm.upload(perm.data(), perm.size());
     set_smem(k_nufft_interp_mma<T, 1, 256>, im_smem<T, 1>());
-    set_smem(k_nufft_interp_mma<T, 1, kImFew>, im_smem<T, 1>());
+    set_smem(k_nufft_interp_mma<T, 1, 128>, im_smem<T, 1>());
+    set_smem(k_nufft_interp_mma<T, 1, 64>, im_smem<T, 1>());
     set_smem(k_nufft_interp_mma<T, kImProb, 256>, im_smem<T, kImProb>());
   }
 
@@ -774,7 +777,7 @@ template <typename T> struct NufftOp : Op {
   // or the batch is a single problem, else chunks of 8
   static constexpr int kMmaProb = 8, kImProb = 6;
   static constexpr size_t kSmLightTiles = 600;  // more than 148 SMs hold at once
-  static constexpr size_t kImFewTiles = 600;  // two rounds of 148 SMs with two CTAs each
+  static constexpr size_t kImManyTiles = 600;  // two rounds of 148 SMs with two CTAs each
   int mma_prob() const { return shared && B > 1 ? kMmaProb : 1; }
   int mma_chunks() const { return shared ? cdiv(B, mma_prob()) : 1; }
 
@@ -915,8 +918,10 @@ template <typename T> struct NufftOp : Op {
     if (interp_mma) {
       const bool one = mma_prob() == 1;
       const auto kern = !one ? k_nufft_interp_mma<T, kImProb, 256>
-                             : im_few ? k_nufft_interp_mma<T, 1, kImFew> : k_nufft_interp_mma<T, 1, 256>;
-      kern<<<dim3(nim, im_chunks), im_few ? kImFew : 256, one ? im_smem<T, 1>() : im_smem<T, kImProb>(), s>>>(
+                        : im_threads == 64  ? k_nufft_interp_mma<T, 1, 64>
+                        : im_threads == 128 ? k_nufft_interp_mma<T, 1, 128>
+                                            : k_nufft_interp_mma<T, 1, 256>;
+      kern<<<dim3(nim, im_chunks), im_threads, one ? im_smem<T, 1>() : im_smem<T, kImProb>(), s>>>(
           geo, wxd(), wyd(), d_im.as<ImTileItem>(), d_imperm.as<int2>(), g, gstride, nx, ny, inv_mm, c.st, gate, c.part,
           qchi, chi_slots(), y2, B, base, out);
       MF_LAUNCH_CK();

@@ -1,10 +1,10 @@
 """Problems with points of their own and few of them to a tile, against the
 tap-by-tap kernels.  Spots of 1 to 150 points, points at the edges of the grid
 (dropped and mirrored taps), frames of one point; few frames, and enough of
-them that interpolation takes the smaller CTAs of many tiles (and cuts a frame
-of 2000 points in one place into more).  Operators agree to 1e-12, so four
-steps agree to 1e-10; the FP32 form to its 2e-5.  A frame has the same bits
-alone and among others."""
+them that interpolation takes the smaller CTAs of many tiles, of two and of
+four warps (and cuts a frame of 2000 points in one place into more).  Operators
+agree to 1e-12, so four steps agree to 1e-10; the FP32 form to its 2e-5.  A
+frame has the same bits alone and among others."""
 import numpy as np
 import pytest
 
@@ -27,7 +27,7 @@ def _frames(nx, more):
     return (at[:, 0].copy(), at[:, 1].copy(), vis[0], vis[1], np.full(len(at), 2.0)), off
 
 
-@pytest.mark.parametrize("nx, more", [(16, 0), (54, 0), (128, 0), (54, 40), (128, 30)])
+@pytest.mark.parametrize("nx, more", [(16, 0), (54, 0), (128, 0), (54, 40), (128, 30), (20, 170)])
 @pytest.mark.parametrize("precision", ["fp64", "fp32"])
 def test_sparse_frames(gpulib, monkeypatch, nx, more, precision):
     prec = gpulib.FP64 if precision == "fp64" else gpulib.FP32
