@@ -24,6 +24,7 @@
 #include "fft_smem.cuh"
 #include "fftvar_ops.cuh"
 #include "fgp.cuh"
+#include "fgp_rule.h"
 #include "mfista_ops.cuh"
 #include "nufft_mma.cuh"
 #include "nufft_ops.cuh"
@@ -1850,81 +1851,51 @@ struct Solver {
   }
 
   struct FgpShape {
-    int cs = 0, rpc = 0, nr = 0, threads = 256;
+    int cs = 0, nr = 0, rpc = 0, threads = 256;
     size_t bytes = 0;
     double cost = 1e300;
   };
 
-  // Time of an FGP launch in units of one problem with k_fgp_reg<1> and 16
-  // CTAs, from the clusters that are resident at once: whole rounds and a rest.
-  // `one`: a round with a CTA per SM; share[k]: what a round costs when k + 1
-  // CTAs share an SM (their pipes and barriers overlap in part).
-  double fgp_cost(int resident, int cs, double one, const double (&share)[4], int sms) const {
-    if (resident < 1) return 1e300;
-    auto round = [&](int n) { return n ? one * share[std::min(3, cdiv((long)n * cs, sms) - 1)] : 0.0; };
-    return (ctx.B / resident) * round(resident) + round(ctx.B % resident);
+  // kern with nr rows a thread (0: k_fgp) and cs CTAs a problem, if it fits and
+  // is expected to be faster than `best`
+  template <typename K> void try_fgp(K kern, int nr, int cs, int threads, size_t bytes, int sms, FgpShape& best) {
+    if (threads > kFgpThreads || bytes > 200 * 1024) return;
+    prep_fgp_kernel(kern, cs, bytes);
+    const FgpCandidate c{nr, cs, max_clusters(kern, cs, bytes, threads)};
+    const double cost = fgp_cost(c, precision != MFISTA_FP32, ctx.tsvNX, ctx.tsvNY, ctx.B, sms);
+    if (cost < best.cost) best = FgpShape{cs, nr, cdiv(ctx.tsvNY, cs), threads, bytes, cost};
   }
 
-  // k_fgp_reg with NR rows a thread and cs CTAs a problem, if it fits and is
-  // expected to be faster than `best`
-  template <typename T, int NR> void try_fgp_reg(int cs, double one, int sms, FgpShape& best) {
-    const int NX = ctx.tsvNX, rows = cdiv(ctx.tsvNY, cs), groups = cdiv(rows, NR);
-    const size_t bytes = fgp_reg_smem<T>(rows, NX);
-    if ((long)groups * NX > kFgpThreads || bytes > 200 * 1024) return;
-    prep_fgp_kernel(k_fgp_reg<T, NR>, cs, bytes);
-    const double share[4] = {1.0, 1.25, 1.5, 1.75};
-    const double cost = fgp_cost(max_clusters(k_fgp_reg<T, NR>, cs, bytes, groups * NX), cs, one, share, sms);
-    if (cost < best.cost) best = FgpShape{cs, rows, NR, groups * NX, bytes, cost};
-  }
-
-  // Picks the FGP cluster shape: slabs in shared memory with 8 or 16 CTAs
-  // when they fit and such a cluster can be resident, else global slabs.
+  // Picks the FGP kernel and cluster by their expected time (fgp_rule.h): the
+  // duals in registers with one or two rows a thread, or slabs in shared memory,
+  // each with 8 and 16 CTAs a problem; else global slabs.  All give the same
+  // bits.
   template <typename T> void pick_fgp_shape() {
-    int NX = ctx.tsvNX, NY = ctx.tsvNY;
-    const size_t limit = 200 * 1024;
-    // few problems: 16 CTAs per problem (more SMs busy, half the rows per CTA);
-    // otherwise 8 (the GPU is full either way, fewer cluster-wide barriers)
-    const bool few = ctx.B * 8 < 148;
+    const int NX = ctx.tsvNX, NY = ctx.tsvNY;
     int dev = 0, sms = 148;
     MF_CK(cudaGetDevice(&dev));
     MF_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    // duals in registers: with one and two rows a thread and 16 and 8 CTAs a
-    // problem (measured at 64, 96 and 128 pixels a side: a round of one problem
-    // takes 1, 1.55, 1.08 and 2 times the first)
     FgpShape best;
-    try_fgp_reg<T, 1>(16, 1.0, sms, best);
-    try_fgp_reg<T, 1>(8, 1.08, sms, best);
-    try_fgp_reg<T, 2>(16, 1.55, sms, best);
-    try_fgp_reg<T, 2>(8, 2.0, sms, best);
+    for (int cs : {16, 8}) {
+      const int rows = cdiv(NY, cs);
+      const size_t reg = fgp_reg_smem<T>(rows, NX), slabs = (size_t)6 * rows * NX * sizeof(T);
+      const auto threads = [&](int nr) { return (int)std::min((long)kFgpThreads + 1, (long)cdiv(rows, nr) * NX); };
+      try_fgp(k_fgp_reg<T, 1>, 1, cs, threads(1), reg, sms, best);
+      try_fgp(k_fgp_reg<T, 2>, 2, cs, threads(2), reg, sms, best);
+      try_fgp(k_fgp<T, true>, 0, cs, 256, slabs, sms, best);
+    }
     d_betas.alloc(sizeof(double) * 2 * (size_t)std::max(fgp_iter, 1));
     k_fgp_betas<<<1, 32, 0, stream>>>(d_betas.as<double>(), fgp_iter);
     MF_LAUNCH_CK();
-    auto use_reg = [&]() {
+    if (best.cs) {
       fgp_cs = best.cs;
       fgp_rpc = best.rpc;
       fgp_nr = best.nr;
       fgp_threads = best.threads;
+      fgp_smem = true;
       fgp_smem_bytes = best.bytes;
-    };
-    for (int cs : {few ? 16 : 8, few ? 8 : 16}) {
-      int rpc = cdiv(NY, cs);
-      size_t bytes = (size_t)6 * rpc * NX * sizeof(T);
-      if (bytes > limit) continue;
-      prep_fgp_kernel(k_fgp<T, true>, cs, bytes);
-      const int resident = max_clusters(k_fgp<T, true>, cs, bytes);
-      if (resident > 0) {
-        // many small problems: its CTAs hide each other's barriers better (64 of
-        // 96 x 96 in FP64: 374 us, k_fgp_reg 475)
-        const double share[4] = {1.0, 1.8, 2.0, 2.2};
-        if (best.cost < fgp_cost(resident, cs, 2.8, share, sms)) return use_reg();
-        fgp_cs = cs;
-        fgp_rpc = rpc;
-        fgp_smem = true;
-        fgp_smem_bytes = bytes;
-        return;
-      }
+      return;
     }
-    if (best.nr) return use_reg();
     fgp_cs = 8;
     fgp_rpc = cdiv(NY, fgp_cs);
     fgp_smem = false;
