@@ -7,12 +7,12 @@
 // the auto-sorting order (no bit reversal).  The first stage reads its points
 // with the caller's `load` (global memory, with the padding, grid correction
 // or half-spectrum folding of the pass) and the last hands its results to the
-// caller's `store`, so a transform of two stages (up to 256 points) crosses
-// shared memory once.  Stages read one shared buffer and write the other, one
-// barrier each.
+// caller's `store`, so a transform of s stages crosses shared memory s - 1
+// times.  Stages read one shared buffer and write the other, one barrier each.
 //
-// Radices 16, 8, 4 and 2 for powers of two (fewest stages), 3 and 5 in closed
-// form, 7, 11 and 13 as symmetric direct sums.  The twiddles of a stage lie
+// Powers of two in radices of at most 4 in the row passes and 8 in the column
+// passes (fft_radices), 3 and 5 in closed form, 7, 11 and 13 as symmetric
+// direct sums.  The twiddles of a stage lie
 // together, [r - 1][k], so that a warp reads consecutive values (by index over
 // the whole table, a warp's reads were scattered and L1 was 64 % busy).
 // Forward sign is -1 (exp(-2 pi i jk/n)), unnormalised, matching FFTW's
@@ -74,37 +74,6 @@ template <typename T> struct Bfly<T, 8> {
     for (int k = 0; k < 4; ++k) {
       v[k] = cadd<T>(e[k], o[k]);
       v[k + 4] = csub<T>(e[k], o[k]);
-    }
-  }
-};
-
-// four columns of four, turned, then four rows of four
-template <typename T> struct Bfly<T, 16> {
-  static __device__ __forceinline__ void run(cplx<T>* v, int sign) {
-    const T h = T(0.7071067811865475244008), c = T(0.9238795325112867561282), s = T(0.3826834323650897717285);
-    cplx<T> a[4][4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {  // points q, q + 4, q + 8, q + 12
-#pragma unroll
-      for (int r = 0; r < 4; ++r) a[q][r] = v[q + 4 * r];
-      Bfly<T, 4>::run(a[q], sign);
-    }
-    // a[q][p] *= exp(sign 2 pi i q p / 16)
-    a[1][1] = crot<T>(a[1][1], c, s, sign);
-    a[1][2] = crot<T>(a[1][2], h, h, sign);
-    a[1][3] = crot<T>(a[1][3], s, c, sign);
-    a[2][1] = crot<T>(a[2][1], h, h, sign);
-    a[2][2] = cmul_si<T>(a[2][2], sign);
-    a[2][3] = crot<T>(a[2][3], -h, h, sign);
-    a[3][1] = crot<T>(a[3][1], s, c, sign);
-    a[3][2] = crot<T>(a[3][2], -h, h, sign);
-    a[3][3] = crot<T>(a[3][3], -c, -s, sign);
-#pragma unroll
-    for (int p = 0; p < 4; ++p) {
-      cplx<T> b[4] = {a[0][p], a[1][p], a[2][p], a[3][p]};
-      Bfly<T, 4>::run(b, sign);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) v[p + 4 * q] = b[q];
     }
   }
 };
@@ -254,7 +223,7 @@ struct FftLay {
 };
 
 // radices whose first or last stage exchanges with global memory
-__host__ __device__ __forceinline__ bool fft_fused(int r) { return r == 16 || r == 8 || r == 5 || r == 4; }
+__host__ __device__ __forceinline__ bool fft_fused(int r) { return r == 8 || r == 5 || r == 4; }
 
 // All stages.  With kToSmem the result stays in the returned buffer (after a
 // barrier); else every element goes to `store`, and the returned pointer is
@@ -285,8 +254,10 @@ __device__ __forceinline__ cplx<T>* fft_run(const FftDev<T>& p, int count, int s
   int s = 0, Ns = 1, last = p.nst;
   // first stage from global memory, if its radix has a fused instance
   switch (p.nst > 1 ? p.radix[0] : 0) {
-    case 16: fft_stage<T, 16, kCols>(n, count, 1, tw, sign, load, to); s = 1; break;
-    case 8: fft_stage<T, 8, kCols>(n, count, 1, tw, sign, load, to); s = 1; break;
+    case 8:
+      if constexpr (kCols) fft_stage<T, 8, kCols>(n, count, 1, tw, sign, load, to);  // rows have none
+      s = 1;
+      break;
     case 5: fft_stage<T, 5, kCols>(n, count, 1, tw, sign, load, to); s = 1; break;
     case 4: fft_stage<T, 4, kCols>(n, count, 1, tw, sign, load, to); s = 1; break;
     default: move([&](int tr, int i) { to(tr, i, load(tr, i)); });
@@ -300,8 +271,9 @@ __device__ __forceinline__ cplx<T>* fft_run(const FftDev<T>& p, int count, int s
   for (; s < last; ++s) {
     const int R = p.radix[s];
     switch (R) {
-      case 16: fft_stage<T, 16, kCols>(n, count, Ns, tw, sign, from, to); break;
-      case 8: fft_stage<T, 8, kCols>(n, count, Ns, tw, sign, from, to); break;
+      case 8:
+        if constexpr (kCols) fft_stage<T, 8, kCols>(n, count, Ns, tw, sign, from, to);
+        break;
       case 4: fft_stage<T, 4, kCols>(n, count, Ns, tw, sign, from, to); break;
       case 2: fft_stage<T, 2, kCols>(n, count, Ns, tw, sign, from, to); break;
       case 3: fft_stage<T, 3, kCols>(n, count, Ns, tw, sign, from, to); break;
@@ -320,23 +292,24 @@ __device__ __forceinline__ cplx<T>* fft_run(const FftDev<T>& p, int count, int s
     return nullptr;
   }
   switch (p.radix[last]) {
-    case 16: fft_stage<T, 16, kCols>(n, count, Ns, tw, sign, from, store); break;
-    case 8: fft_stage<T, 8, kCols>(n, count, Ns, tw, sign, from, store); break;
+    case 8:
+      if constexpr (kCols) fft_stage<T, 8, kCols>(n, count, Ns, tw, sign, from, store);
+      break;
     case 5: fft_stage<T, 5, kCols>(n, count, Ns, tw, sign, from, store); break;
     default: fft_stage<T, 4, kCols>(n, count, Ns, tw, sign, from, store); break;
   }
   return nullptr;
 }
 
-// The radices of length n in stage order (0: a prime factor above 13): powers
-// of two in as few radices up to 2^log2max (<= 4) as possible and as even as
-// possible; the two largest with an instance that exchanges with global memory
+// The radices of length n in stage order (0: a prime factor above 13; no int
+// has more than kMaxStages of them): powers of two in as few radices up to
+// 2^log2max as possible and as even as possible; the two largest with an instance that exchanges with global memory
 // (fft_fused) go first and last.
 // Columns take radices up to 8 and rows up to 4.  Larger ones make fewer trips
 // through shared memory but leave a CTA's few transforms to fewer threads, each
-// with a longer chain: an iteration of one problem takes 115 / 119 us at 64 /
+// with a longer chain: an iteration of one problem took 115 / 119 us at 64 /
 // 128 pixels a side with 16 and 8, 107 / 111 with 8 and 4; 32 problems at 256
-// take 312 either way.  (The lengths decide alone: a problem's values may not
+// took 312 either way.  (The lengths decide alone: a problem's values may not
 // depend on its batch.)
 constexpr int kColsLog2Max = 3, kRowsLog2Max = 2;
 
@@ -355,7 +328,7 @@ inline int fft_radices(int n, int (&radix)[kMaxStages], int log2max) {
       list[m++] = f;
       n /= f;
     }
-  if (n > 1 || m > kMaxStages) return 0;
+  if (n > 1) return 0;
   auto key = [](int r) { return (fft_fused(r) ? 100 : 0) + r; };
   for (int i = 1; i < m; ++i)  // fused first, by falling radix
     for (int j = i; j > 0 && key(list[j]) > key(list[j - 1]); --j) {
@@ -378,13 +351,13 @@ constexpr size_t kRowsPadMax = 96 * 1024;  // larger row buffers go without padd
 // buffers then take at most kRowsPadMax (a single row: half of it, so that no
 // length loses its place in the default shared memory), the host sizing them
 // alike.
-template <typename T> __host__ __device__ __forceinline__ int rows_psh() { return sizeof(T) == 8 ? 3 : 4; }
+constexpr int kRowsPsh = 3;  // an element in eight of 16 bytes
 template <typename T> __host__ __device__ __forceinline__ size_t rows_bytes(int h, int rows, int psh) {
   return 2 * sizeof(cplx<T>) * (size_t)rows * (h + 1 + (h >> psh));
 }
 template <typename T> __host__ __device__ __forceinline__ FftLay rows_lay(int h, int rows) {
   const size_t most = rows == 1 ? kRowsPadMax / 2 : kRowsPadMax;
-  const int psh = rows_bytes<T>(h, rows, rows_psh<T>()) <= most ? rows_psh<T>() : 31;
+  const int psh = rows_bytes<T>(h, rows, kRowsPsh) <= most ? kRowsPsh : 31;
   return FftLay{h + 1 + (h >> psh), psh};
 }
 template <typename T> __host__ __device__ __forceinline__ size_t rows_smem_bytes(int h, int rows) {
