@@ -19,7 +19,8 @@ CPP_LIB = os.path.join(PKG, "libmfista_b200_cpp.so")
 INCLUDE = os.path.abspath(os.path.join(PKG, "..", "include"))
 SOURCES = ["mfista_b200.cu", "nufft_noalloc.cu", "unet.cu"]
 HEADERS = ["common.cuh", "fft_smem.cuh", "fft_reg.cuh", "nufft_ops.cuh", "nufft_mma.cuh", "dgemm_mma.cuh", "fftvar_ops.cuh", "dft_ops.cuh",
-           "mfista_ops.cuh", "fgp.cuh", "solver.cuh", "looe.cuh", "dft_tc.cuh", "cpp_nufft.cuh", "column_runs.h", "fgp_rule.h"]
+           "mfista_ops.cuh", "fgp.cuh", "solver.cuh", "looe.cuh", "dft_tc.cuh", "cpp_nufft.cuh", "column_runs.h", "fgp_rule.h",
+           "looe_rule.h"]
 
 NVCC_FLAGS = ["-O3", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",
               "-Xcompiler", "-fPIC", "-shared", "-cudart", "static"]

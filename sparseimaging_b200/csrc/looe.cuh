@@ -36,6 +36,7 @@
 
 #include "column_runs.h"
 #include "dgemm_mma.cuh"
+#include "looe_rule.h"
 #include "solver.cuh"
 
 namespace mf {
@@ -369,7 +370,7 @@ __global__ void k_looe_final(const double* __restrict__ part, int nblk, int M, c
 //
 // Only the columns of A that some solution uses go to the device, in runs
 // (column_runs.h).
-// Solutions run on up to kLanes streams, each with its own scratch: one
+// Solutions run on up to kLanes streams (looe_rule.h), each with its own scratch: one
 // solution's factorisation is a chain of small kernels (840 of 2190 us at 1261
 // active pixels) and its other kernels leave SMs idle, which the next one's
 // fill.  Lanes beyond the first are taken only while all scratch stays within
@@ -381,7 +382,7 @@ struct Looe {
 
   struct Lane {
     cudaStream_t s = nullptr;
-    DevMem mem;
+    double* mem = nullptr;   // its part of d_lanes
     std::vector<int> idx;    // of the solution in flight: pixels, then columns of the device's A
     std::vector<double> xs;  // its active values
     ~Lane() {
@@ -396,7 +397,7 @@ struct Looe {
   const double* X;
   int M, N, NX, B;
   int most = 0;          // active pixels of a solution at most
-  DevMem d_A, d_y;
+  DevMem d_A, d_y, d_lanes;
   std::vector<int> col;  // pixel -> column of the device's A
   std::vector<std::unique_ptr<Lane>> lanes;
   int sms = 148;
@@ -431,19 +432,19 @@ struct Looe {
     set_smem(k_looe_panel, dg::kSmem);
     set_smem(k_looe_trail, dg::kSmem);
     set_smem(k_looe_rows, kRowsSmem);
-    const size_t bytes = sizeof(double) * layout(most).total;
-    for (int i = 0; i < std::min(kLanes, B); ++i) {
-      if (i > 0 && (i + 1) * bytes > kLaneBytes) break;
+    // one allocation for all lanes: each of its own cost 0.1 ms, and 0.7 ms from a few MB on
+    const size_t each = layout(most).total, bytes = sizeof(double) * each;
+    int n = looe_lanes(B, cdiv(most, kPanel), M, kLanes);
+    while (n > 1 && n * bytes > kLaneBytes) --n;
+    for (; n > 1; --n) {
+      if (cudaMalloc(&d_lanes.p, n * bytes) == cudaSuccess) break;
+      cudaGetLastError();
+    }
+    if (n > 1) d_lanes.bytes = n * bytes;
+    else d_lanes.alloc(bytes);
+    for (int i = 0; i < n; ++i) {
       std::unique_ptr<Lane> l(new Lane);
-      if (i > 0) {
-        if (cudaMalloc(&l->mem.p, bytes) != cudaSuccess) {
-          cudaGetLastError();
-          break;
-        }
-        l->mem.bytes = bytes;
-      } else {
-        l->mem.alloc(bytes);
-      }
+      l->mem = d_lanes.as<double>() + i * each;
       MF_CK(cudaStreamCreateWithFlags(&l->s, cudaStreamNonBlocking));
       lanes.push_back(std::move(l));
     }
@@ -517,7 +518,7 @@ struct Looe {
     for (int q = 0; q < ns; ++q) L.idx.push_back(col[L.idx[q]]);
     const int np = cdiv(ns, kPanel), tiles = tiles_of(ns);
     const Layout l = layout(most);
-    double* m = L.mem.as<double>();
+    double* m = L.mem;
     int* info = reinterpret_cast<int*>(m + l.info);
     int *pix = reinterpret_cast<int*>(m + l.idx), *S = pix + ns;
     MF_CK(cudaMemsetAsync(info, 0, sizeof(int), s));
@@ -565,7 +566,7 @@ struct Looe {
     auto finish = [&](int b) {
       Lane& L = *lanes[b % nl];
       double out[3];
-      MF_CK(cudaMemcpyAsync(out, L.mem.as<double>() + l.out, sizeof(out), cudaMemcpyDeviceToHost, L.s));
+      MF_CK(cudaMemcpyAsync(out, L.mem + l.out, sizeof(out), cudaMemcpyDeviceToHost, L.s));
       MF_CK(cudaStreamSynchronize(L.s));
       f(b, out);
     };
