@@ -303,8 +303,8 @@ __device__ __forceinline__ cplx<T>* fft_run(const FftDev<T>& p, int count, int s
 
 // The radices of length n in stage order (0: a prime factor above 13; no int
 // has more than kMaxStages of them): powers of two in as few radices up to
-// 2^log2max as possible and as even as possible; the two largest with an instance that exchanges with global memory
-// (fft_fused) go first and last.
+// 2^log2max as possible and as even as possible; the two largest with an
+// instance that exchanges with global memory (fft_fused) go first and last.
 // Columns take radices up to 8 and rows up to 4.  Larger ones make fewer trips
 // through shared memory but leave a CTA's few transforms to fewer threads, each
 // with a longer chain: an iteration of one problem took 115 / 119 us at 64 /

@@ -144,10 +144,14 @@ template <typename T> size_t fft_cols_smem(int n, int cols) {
   else return (size_t)2 * cols * (n + 1) * sizeof(cplx<T>);
 }
 
-// Threads of a CTA of the row passes, FP64: 128 where they do the first
-// stage's items (rows x length / radix) in one or two full rounds (64 x 128
-// rows of 128, two rounds: 44 us forward and back, 51 with 256 threads), else
-// 256 (11 x 100 rows of 100, 160 items: 19 us, 25 with 128 threads)
+// Threads of a CTA of the row passes, FP64: 128 where that many, or half of
+// them in two full rounds, take the first stage's items (rows x length / radix);
+// more would idle and keep other CTAs from the SM (us forward and back with 128
+// / 256 threads, 64 problems: 64 x 64 in rows of 8, 128 items, 14.4 / 20.6; 50
+// x 50 in rows of 8, 80 items, 16.5 / 25.6, and of 1 55 / 98; 128 x 128 in rows
+// of 8, 256 items, 37 / 45).  Else 256 (11 x 100 rows of 100, 160 items: 19 us,
+// 25 with 128 threads).  Two rounds cost where the chip is not full: 128 x 128
+// in rows of 8, 16 problems 20.6 / 16.5, one problem 16.5 / 14.6.
 template <typename T> int rows_threads(const FftDev<T>& f, int rows) {
   const int items = rows * (f.n / (f.nst ? f.radix[0] : 1));
   return kRegFft<T> && (items <= 128 || items == 256) ? 128 : 256;
