@@ -1,5 +1,6 @@
-// How long an FGP launch takes by the kernel and cluster that run it: the rule
-// that picks them (Solver::pick_fgp_shape).  Host arithmetic only.
+// How long an FGP launch, and the launches of a solve, take by the kernel and
+// cluster that run them: the rule that picks them (Solver::pick_fgp_shape).
+// Host arithmetic only.
 #pragma once
 #include <algorithm>
 
@@ -19,10 +20,8 @@ struct FgpCandidate {
 // over its rows (k_fgp: each a chain of shared-memory accesses); share: what
 // the CTAs of an SM cost each other.  Fitted to 3000 launches on B200 (both
 // precisions, 32 to 160 pixels a side, 1 to 128 problems, every candidate):
-// mean error 4 %; the candidate it picks takes 0.6 % more than the fastest on
-// average and 13 % at most, and 6 % less than a rule with one time per
-// candidate, which took up to 1.5 times as long as k_fgp (FP32, 128 problems of
-// 72 x 72: 580 us, now 381).
+// mean error 4 %; the fastest candidate by it takes 0.6 % more than the fastest
+// on average and 13 % at most.
 inline double fgp_cost(const FgpCandidate& c, bool fp64, int NX, int NY, int B, int sms) {
   struct Fit {
     double base, per, share, alone;
@@ -43,6 +42,19 @@ inline double fgp_cost(const FgpCandidate& c, bool fp64, int NX, int NY, int B, 
     return n ? (f.base + f.per * work) * (1 + f.share * std::max(0.0, (double)n * c.cs / sms - f.alone)) : 0.0;
   };
   return (B / c.resident) * round(c.resident) + round(B % c.resident);
+}
+
+// What the candidates are compared by: a launch with every problem active and
+// one with a single problem left.  Solves of a batch end one by one, so many of
+// their launches run few problems, and the kernel that is fastest with all of
+// them can be the slowest then (FP32, 16 of 128 x 128: k_fgp 220 us, 195 with one
+// left; k_fgp_reg 246 and 107; 100 iterations of the solve 74 and 53 ms).  The
+// weight fits 48 batches of 8 to 64 problems, 64 to 160 pixels a side, both
+// precisions, for 100 iterations and to convergence: the pick's solve takes 1.2
+// % more than the fastest on average and 10 % at most; by the full launch alone
+// 12 % and 72 %, by one fixed time per candidate 30 % and 168 %.
+inline double fgp_solve_cost(const FgpCandidate& c, bool fp64, int NX, int NY, int B, int sms) {
+  return fgp_cost(c, fp64, NX, NY, B, sms) + 1.25 * fgp_cost(c, fp64, NX, NY, 1, sms);
 }
 
 }  // namespace mf

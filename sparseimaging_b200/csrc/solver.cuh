@@ -1866,7 +1866,7 @@ struct Solver {
     if (threads > kFgpThreads || bytes > 200 * 1024) return;
     prep_fgp_kernel(kern, cs, bytes);
     const FgpCandidate c{nr, cs, max_clusters(kern, cs, bytes, threads)};
-    const double cost = fgp_cost(c, precision != MFISTA_FP32, ctx.tsvNX, ctx.tsvNY, ctx.B, sms);
+    const double cost = fgp_solve_cost(c, precision != MFISTA_FP32, ctx.tsvNX, ctx.tsvNY, ctx.B, sms);
     if (cost < best.cost) best = FgpShape{cs, nr, cdiv(ctx.tsvNY, cs), threads, bytes, cost};
   }
 
