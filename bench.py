@@ -295,8 +295,9 @@ def fft_config1(si, hbm_gbs):
             fgp[f"{name}_b{B}"] = {"ms": round(ms, 5), "GB/s": round(by / ms / 1e6, 1),
                                    "frac_of_hbm": round(by / ms / 1e6 / hbm_gbs, 4) if hbm_gbs else None}
     out["fgp_kernel"] = fgp
-    out["fgp_kernel_note"] = ("k_fgp: 50 FGP iterations of one prox per problem inside one launch (slabs in shared "
-                              "memory, DSMEM halos); compulsory bytes 24 B/pixel per prox (z, dfdx in, xnew out)")
+    out["fgp_kernel_note"] = ("k_fgp_reg or k_fgp: 50 FGP iterations of one prox per problem inside one launch (duals "
+                              "in registers or shared memory, DSMEM halos); compulsory bytes 24 B/pixel per prox "
+                              "(z, dfdx in, xnew out)")
     return out
 
 
